@@ -44,21 +44,22 @@ cudaError_t raise_smem_limit(F* func, size_t bytes) {
 
 // ---- filterbank kernels (kernels_fb.cu) ------------------------------------
 struct DedispArgs {
-  const uint8_t* in;      // FT rows, channel c at in + c*in_pitch
-  size_t in_pitch;
+  const uint32_t* in;     // four-sample words: channel c at in + c*in_pitch
+  size_t in_pitch;        // words
+  int split;              // word t holds samples t + q*split, q = 0..3
   const int* delays;      // [dm_count][nchans] delay in samples
-  const int* blk_min;     // [n_dm_blocks][nchans] min delay over the block's DMs
+  const int2* blk_range;  // [n_dm_blocks][nchans] least and largest delay of the block's DMs
   const int* chans;       // active (not killed) channel indices
   int nact;
   int nchans;
   int dm_count;
-  size_t nout;            // output samples per DM
+  int nout;               // output samples per DM
   float* out;
-  size_t out_pitch;       // floats between DM rows (multiple of 4)
-  int rowb;               // shared-memory row bytes (multiple of 16)
+  size_t out_pitch;       // floats between DM rows
+  int cap;                // bytes of a stage buffer (multiple of 16)
   unsigned* err;          // device error word (bit 0: staging wait timed out)
   int units;              // independent filterbanks dedispersed by one launch
-  size_t in_unit;         // bytes between units' FT inputs
+  size_t in_unit;         // words between units' inputs
   size_t out_unit;        // floats between units' outputs
   unsigned wait_limit;    // polls of each bounded mbarrier wait
   // test of the error path: the producer issues no copy for the last stage,
@@ -66,28 +67,37 @@ struct DedispArgs {
   int withhold_last;
   // always 1: the multiplier of the kernel's multiply-add accumulations.  A
   // runtime value keeps them multiply-adds, which issue to the FMA pipe and
-  // leave the ALU pipe (shifts, byte permutes, adds) to the rest of the work
+  // leave the ALU pipe (byte permutes, adds) to the rest of the work
   unsigned one;
 };
 
-// Dedispersion tile: DMs and output samples per CTA, channel rows staged per
-// pipeline stage.  Every tile gives the same (exact integer) sums.
+// Dedispersion tile: DMs and output samples per CTA (a quarter of them words
+// apart by `split`), and the bytes of a stage buffer of channel rows.  Every
+// tile gives the same (exact integer) sums.
 struct DedispTile {
-  int dm_block, time_block, rows;
+  int dm_block, time_block, stage;
 };
-constexpr int kDedispDmBlocks[3] = {8, 16, 32};
 // polls of a dedispersion mbarrier wait before it gives up and reports
 constexpr unsigned kDedispWaitLimit = 1u << 22;
-// candidate {dm_block, time_block} pairs: time_block = 128 K G with K output
-// words per lane (1, 3 or 5) in G groups; the launcher maps each pair to its
-// kernel instance
+// candidate {dm_block, time_block} pairs: time_block = 128 W with W words per
+// lane; the launcher maps each pair to its kernel instance
 constexpr int kDedispTiles[11][2] = {{8, 1024}, {8, 640},  {8, 768},  {8, 1152},
                                      {8, 1280}, {16, 512}, {16, 384}, {16, 640},
                                      {16, 768}, {32, 256}, {32, 384}};
-// rows per stage that fit shared memory for staged rows of rowb bytes (0: none)
-int dedisp_rows_per_stage(int dm_block, int rowb);
-size_t dedisp_smem_bytes(int dm_block, int rows, int rowb);
+// Tiles of few trials, for trials so far apart in delay that no block of eight
+// fits shared memory: two trials, and one (whose span is 0)
+constexpr int kDedispLongTiles[2][2] = {{2, 5120}, {1, 8192}};
+constexpr int kDedispRows = 32;  // channel rows per stage at most
+// bytes of a stage buffer for rows of these lengths (0: a row does not fit)
+int dedisp_stage_bytes(int dm_block, int time_block, int mean_row, int longest_row);
+size_t dedisp_smem_bytes(int dm_block, int time_block, int cap);
 cudaError_t launch_dedisp(const DedispArgs& a, const DedispTile& t, cudaStream_t s);
+// Four-sample words of the channel-major byte rows of `units` inputs: word t
+// (t < nwords) of a row = samples t + q*split, q = 0..3.  Pitches and units in
+// bytes (in, multiples of 16) and words (out, multiples of 16 and 4).
+cudaError_t launch_split_words(const uint8_t* in, size_t in_pitch, size_t in_unit, int nchans,
+                               size_t units, int split, size_t nwords, uint32_t* out,
+                               size_t out_pitch, size_t out_unit, cudaStream_t s);
 // TF -> channel-major copy of `units` filterbanks (nsamps x nchans bytes each,
 // consecutive in `in`); unit u's copy starts at out + u * out_unit.
 cudaError_t launch_transpose_tf_ft(const uint8_t* in, size_t nsamps, int nchans, uint8_t* out,

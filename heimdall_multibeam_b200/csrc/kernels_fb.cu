@@ -465,83 +465,88 @@ __global__ void k_nb_zap(uint32_t* __restrict__ data, size_t nsamps, int units, 
 //
 //   out[d][t] = (float) sum_{c active} in[c][t + delay[d][c]],  t < nout
 //
-// CTA = DB = 2*NW DMs x TB = 128*K*G samples, NW consumer warps + 1 producer
-// warp.  The producer walks the active channels in stages of CH: for each
-// stage it tabulates the byte offset of every (DM, channel) pair in shared
-// memory and issues one 1-D bulk async copy (TMA, cp.async.bulk) per channel
-// row segment [t0 + min_d delay - align, +rowb) into a ring of NST stage
-// buffers, signalling a `full` mbarrier; consumer warps release a buffer
-// through an `empty` mbarrier (one arrival per warp).  There is no block-wide
-// barrier in the main loop, so warps drift freely within the ring.
+// Input: four-sample words.  With S = split (a quarter of nout, rounded up to
+// 16), word t of channel c holds the bytes of samples t, t + S, t + 2S and
+// t + 3S (k_split_words).  A delay then moves whole words: word t + delay has
+// the four samples that outputs t + q S need, so a (DM, channel) term is one
+// shared-memory load at any delay, without realignment, and the 32 lanes'
+// loads (consecutive words) are one conflict-free wavefront.
 //
-// Warp w owns DMs 2w and 2w+1.  In each of G groups of 32*K words, lane l
-// owns the K consecutive output words (4K samples) starting at word K*l.  A
-// (DM, channel) term reads the K+1 row words that cover the lane's window
-// shifted by the delay, and realigns each output word with a funnel shift.
-// Because K is odd, the 32 lanes' j-th loads (word K*l + j) fall in 32
-// distinct banks: every shared load is one wavefront, and a term costs
-// 4 (K+1) / (4 K) bytes of shared-memory bandwidth per sample (2 at K = 1,
-// 1.33 at K = 3, 1.2 at K = 5).  Each realigned word is split into two
-// 16-bit lane pairs (even/odd samples); two channels are summed per 3-input
-// add, so one add accumulates four sample-channel terms.  The 16-bit lanes
-// are drained into 32-bit sums after at most 257 channels (255 * 257 =
-// 65535), so the sums are exact.  Every mbarrier wait is bounded; a wait that
-// gives up sets bit 0 of a.err and the warp leaves its loop.
+// CTA = DB = DPW*NWD DMs x TBW = 32*W*NWT words (4 TBW samples), NWD*NWT
+// consumer warps + 1 producer warp.  The producer walks the active channels in
+// stages: as many channel row segments [t0 + min_d delay - align, t0 + max_d
+// delay + TBW) as fit a stage buffer, each at the length its own DM block and
+// channel need, come by one 1-D bulk async copy (TMA, cp.async.bulk) each,
+// with the shared-memory byte offset of every (DM, channel) window in a table.
+// It loads the next stage's tables before it waits for a free buffer.  A
+// `full` mbarrier announces a stage, consumer warps release it through an
+// `empty` mbarrier (one arrival per warp).  There is no block-wide barrier in
+// the main loop.  Every mbarrier wait is bounded; a wait that gives up sets
+// bit 0 of a.err and the warp leaves its loop.
 //
-// Pipe balance: the shifts, byte permutes and 3-input adds all issue to the
-// ALU pipe, which bounds the kernel, while the FMA pipe idles.  The odd-byte
-// sums are therefore accumulated with integer multiply-adds by a.one (= 1,
-// unknown to the compiler), which issue to the FMA pipe; and the producer
-// tabulates, per (DM, channel), the shared-memory word index of the row
-// segment and the realignment shift, so the consumers spend no ALU work on
-// addressing.
+// A consumer lane owns words lane + 32 w of DPW DMs and keeps two 32-bit
+// accumulators per word for its four sums (dd_dot).  After each run of at most
+// 256 channels the sums of a word go to the output row: a single run is
+// converted and stored; with more channels the row holds 32-bit integer
+// partial sums (stored, then added to in L2) until the last run adds its own
+// and stores the float.  The sums are exact integers in any order.
+//
+// What bounds it: one shared load per word, DM and channel (128 sample terms a
+// wavefront), so the shared-memory pipe (75 % busy in ncu) and instruction
+// issue (70 %).  Measured sample-channel adds per second, the tile from the
+// autotuner, against the byte-row kernel before it (8 x 1280 samples, funnel
+// shifts to realign): 4096 channels, DM 0-500: 28.2 T/s (19.2); 1024 channels,
+// DM 0-2000: 26.7 (16.8); 256 channels, DM 0-1000: 20.4 (15.0); 36 x 320
+// channels at 655 us: 24 (19.6).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t d;
-  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
+// Two forms of a word's four sums, each two accumulators (raw, odd):
+//   permute: the words modulo 2^32, and the odd bytes in 16-bit lanes;
+//   dot:     S0 + 65535 S1 and S2 + 65535 S3 by 2-way dot products (every sum
+//            <= 256 * 255 < 65535, so a remainder and a quotient give both
+//            back).
+// The permutes and 3-input adds issue to the ALU pipe and the dot products to
+// the FMA pipe, so two words of three take the dot form.
+constexpr uint32_t kDot = 0xFFFF0001u;
+__host__ __device__ constexpr bool dd_dot(int w) { return w % 3 != 0; }
+
+constexpr int DD_NST = 2;      // stages of the row ring
+constexpr int DD_ROWS = kDedispRows;
+constexpr int DD_RUN = 256;    // channels between two flushes at most
+
+// CTAs per SM the register budget allows: two registers per owned word and DM
+// plus about 48 others, and a quarter of the SM's registers per scheduler.
+constexpr int dd_min_blocks(int warps, int words) {
+  const int per_sched = 16384 / (32 * ((2 * words + 48 + 7) / 8 * 8));
+  const int n = 4 * per_sched / (warps + 1);
+  return n < 1 ? 1 : n > 5 ? 5 : n;
 }
 
-// CTAs per SM the register budget allows: per lane about 12 registers per
-// owned output word (two DMs x {2 packed, 4 drained} sums; 8 with the
-// compact drain) plus ~48 others.
-constexpr int dd_regs(int k, int g, bool a16) { return (a16 ? 8 : 12) * k * g + 48; }
-constexpr int dd_min_blocks(int nw, int k, int g, bool a16) {
-  return (65536 / ((nw + 1) * 32 * dd_regs(k, g, a16))) < 1
-             ? 1
-             : (65536 / ((nw + 1) * 32 * dd_regs(k, g, a16))) > 3
-                   ? 3
-                   : (65536 / ((nw + 1) * 32 * dd_regs(k, g, a16)));
-}
-
-// A16 (at most 511 active channels): the sums drained after the first 256 or
-// 257 channels stay packed as two 16-bit lane pairs (each <= 257 * 255 =
-// 65535), and the remaining < 257 channels are added to them in 32 bits when
-// the output is written; 8 rather than 12 registers per output word, so
-// more CTAs fit an SM.
-template <int NW, int K, int G, int CH, int NST, bool A16>
-__global__ void __launch_bounds__((NW + 1) * 32, dd_min_blocks(NW, K, G, A16))
+template <int NWD, int NWT, int DPW, int W, int UC>
+__global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT, DPW * W))
     k_dedisp(DedispArgs a) {
-  static_assert(K % 2 == 1, "odd K keeps the strided shared loads conflict-free");
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr int DB = 2 * NW;
-  constexpr int TB = 128 * K * G;
+  constexpr int NW = NWD * NWT;
+  constexpr int DB = DPW * NWD;
+  constexpr int TBW = 32 * W * NWT;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* empty = full + NST;
-  // [NST][DB*CH] {word index of the (DM, channel) row segment in `rows`,
-  // realignment shift in bits}
-  int2* s_off = reinterpret_cast<int2*>(smem + 128);
-  uint8_t* rows = smem + 128 + NST * DB * CH * sizeof(int2);  // [NST][CH][rowb]
+  uint64_t* empty = full + DD_NST;
+  int* nrows = reinterpret_cast<int*>(empty + DD_NST);  // channels of each stage buffer
+  // [TBW] zero words (the window of a channel past the last one), then
+  // [NST][DB][CH] byte offsets from smem of the (DM, channel) windows, then
+  // [NST] stage buffers of a.cap bytes
+  constexpr int CH = DD_ROWS;
+  constexpr int ZERO = 128;
+  constexpr int OFFS = ZERO + TBW * 4;
+  constexpr int ROWS0 = OFFS + DD_NST * DB * CH * 4;
   const int dblk = blockIdx.x;
-  const size_t t0 = (size_t)blockIdx.y * TB;
+  const int t0 = blockIdx.y * TBW;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d_lo = dblk * DB;
-  const int* __restrict__ bmin = a.blk_min + (size_t)dblk * a.nchans;
-  const int nstage = (a.nact + CH - 1) / CH;
-  const size_t C = (size_t)a.nchans;
 
+  for (int i = threadIdx.x; i < TBW; i += (NW + 1) * 32)
+    reinterpret_cast<uint32_t*>(smem + ZERO)[i] = 0u;
   if (threadIdx.x == 0) {
-    for (int b = 0; b < NST; b++) {
+    for (int b = 0; b < DD_NST; b++) {
       mbar_init(&full[b], 1);
       mbar_init(&empty[b], NW);
     }
@@ -552,196 +557,221 @@ __global__ void __launch_bounds__((NW + 1) * 32, dd_min_blocks(NW, K, G, A16))
   if (warp == NW) {
     // ---------------- producer ----------------
     // blockIdx.z selects the unit (an independent filterbank of the batch)
-    const uint8_t* __restrict__ in = a.in + (size_t)blockIdx.z * a.in_unit;
-    int issued = 0;
-    for (int st = 0; st < nstage; st++) {
-      const int buf = st % NST;
-      if (st >= NST) {
-        if (!mbar_wait(&empty[buf], (uint32_t)(((st / NST) - 1) & 1), a.wait_limit)) {
+    const uint32_t* __restrict__ in = a.in + (size_t)blockIdx.z * a.in_unit;
+    const int2* __restrict__ brange = a.blk_range + (size_t)dblk * a.nchans;
+    // lane k < CH of a stage: its k-th channel and that channel's delay range
+    int c = 0;
+    int2 r = make_int2(0, 0);
+    auto channel = [&](int k0) {
+      const bool have = lane < CH && k0 + lane < a.nact;
+      c = have ? a.chans[k0 + lane] : 0;
+      r = have ? brange[c] : make_int2(0, 0);
+    };
+    channel(0);
+    int st = 0;
+    for (int k0 = 0; k0 < a.nact; st++) {
+      const int buf = st % DD_NST;
+      const bool have = lane < CH && k0 + lane < a.nact;
+      const int lo = (t0 + r.x) & ~3;
+      const int bytes = have ? (4 * (t0 + r.y - lo + TBW) + 15) & ~15 : 0;
+      int end = bytes;  // inclusive scan: the rows lie back to back
+#pragma unroll
+      for (int o = 1; o < CH; o *= 2) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+      }
+      // as many rows as fit the buffer, whole groups of UC where there are any
+      int nk = __popc(__ballot_sync(0xffffffffu, have && end <= a.cap));
+      if (nk > UC && k0 + nk < a.nact) nk -= nk % UC;
+      const int total = __shfl_sync(0xffffffffu, end, nk - 1);
+      const int at = ROWS0 + buf * a.cap + end - bytes;  // byte offset of the row
+      // the stage's delays (channel lane % CH, DR DMs a round), all loads in
+      // flight at once, and the next stage's channels, before the buffer is
+      // waited for
+      constexpr int DR = 32 / CH;  // DMs per round
+      constexpr int NR = (DB + DR - 1) / DR;
+      const int kl = lane % CH;
+      const int ck = __shfl_sync(0xffffffffu, c, kl);
+      const int row0 = __shfl_sync(0xffffffffu, at + 4 * (t0 - lo), kl);
+      int dl[NR];
+#pragma unroll
+      for (int i = 0; i < NR; i++) {
+        const int d = min(d_lo + DR * i + lane / CH, a.dm_count - 1);
+        dl[i] = a.delays[(size_t)d * a.nchans + ck];
+      }
+      const int c_now = c;
+      channel(k0 + nk);
+      if (st >= DD_NST) {
+        if (!mbar_wait(&empty[buf], (uint32_t)(((st / DD_NST) - 1) & 1), a.wait_limit)) {
           if (lane == 0) atomicOr(a.err, 1u);
           break;
         }
       }
       // error-path test: the last stage is never copied (nor announced), so
       // its `full` phase never completes and the consumers' wait gives up
-      if (a.withhold_last && st == nstage - 1) break;
-      const int k0 = st * CH;
-      const int nk = min(CH, a.nact - k0);
-      int2* off = s_off + buf * DB * CH;
-      for (int e = lane; e < DB * CH; e += 32) {
-        const int k = e % CH;
-        if (k < nk) {
-          const int c = a.chans[k0 + k];
-          const int d = min(d_lo + e / CH, a.dm_count - 1);
-          const size_t lo = (t0 + (size_t)bmin[c]) & ~(size_t)15;
-          const int o = (int)(t0 + (size_t)a.delays[(size_t)d * C + c] - lo);
-          off[e] = make_int2(((buf * CH + k) * a.rowb + o) >> 2, (o & 3) * 8);
-        }
-      }
+      if (a.withhold_last && k0 + nk == a.nact) break;
+      int* off = reinterpret_cast<int*>(smem + OFFS) + buf * DB * CH;
+#pragma unroll
+      for (int i = 0; i < NR; i++)
+        if (DR * i + lane / CH < DB)
+          off[32 * i + lane] = kl < nk ? row0 + 4 * dl[i] : ZERO;
+      if (lane == 0) nrows[buf] = nk;
       __syncwarp();
-      if (lane == 0) mbar_expect_tx(&full[buf], (uint32_t)(nk * a.rowb));
+      if (lane == 0) mbar_expect_tx(&full[buf], (uint32_t)total);
       __syncwarp();
-      if (lane < nk) {
-        const int c = a.chans[k0 + lane];
-        const size_t lo = (t0 + (size_t)bmin[c]) & ~(size_t)15;
-        bulk_g2s(rows + (size_t)(buf * CH + lane) * a.rowb, in + (size_t)c * a.in_pitch + lo,
-                 (uint32_t)a.rowb, &full[buf]);
-      }
-      issued = st + 1;
+      if (lane < nk)
+        bulk_g2s(smem + at, in + (size_t)c_now * a.in_pitch + lo, (uint32_t)bytes, &full[buf]);
+      k0 += nk;
     }
+    const int issued = st;
     // let every copy this CTA issued land before the warp exits
-    for (int st = (issued > NST ? issued - NST : 0); st < issued; st++)
-      mbar_wait(&full[st % NST], (uint32_t)((st / NST) & 1), a.wait_limit);
+    for (int j = (issued > DD_NST ? issued - DD_NST : 0); j < issued; j++)
+      mbar_wait(&full[j % DD_NST], (uint32_t)((j / DD_NST) & 1), a.wait_limit);
     return;
   }
 
   // ---------------- consumers ----------------
-  // pk[..][0] sums the raw words (bytes b0..b3 of 4 samples) modulo 2^32 and
-  // pk[..][1] the odd bytes (b1, b3) in two 16-bit lanes.  With at most 257
-  // channels between drains every byte-lane sum is <= 65535, so
-  // raw - (odd << 8) = E0 + 2^16 E2 exactly: the even-byte sums.
-  constexpr int W = K * G;  // output words per lane and DM
-  constexpr int NA = A16 ? 2 : 4;
-  uint32_t pk[2][W][2];
-  // drained sums: samples 0..3 in 32 bits, or (A16) {even, odd} lane pairs
-  uint32_t acc[2][W][NA];
+  const int wd = warp % NWD, wt = warp / NWD;
+  const int word0 = wt * 32 * W + lane;  // this lane's first word of the tile
+  const uint8_t* lane_base = smem + 4 * word0;
+  uint32_t raw[DPW][W], odd[DPW][W];
 #pragma unroll
-  for (int d = 0; d < 2; d++)
+  for (int d = 0; d < DPW; d++)
 #pragma unroll
-    for (int w = 0; w < W; w++) {
-      pk[d][w][0] = pk[d][w][1] = 0;
+    for (int w = 0; w < W; w++) raw[d][w] = odd[d][w] = 0;
+
+  float* __restrict__ out = a.out + (size_t)blockIdx.z * a.out_unit;
+  // the run's sums to the output rows; first / last: of this tile's runs
+  auto flush = [&](bool first, bool last) {
 #pragma unroll
-      for (int q = 0; q < NA; q++) acc[d][w][q] = 0;
-    }
-  auto drain = [&]() {
+    for (int d = 0; d < DPW; d++) {
+      const int dd = d_lo + DPW * wd + d;
+      if (dd < a.dm_count) {
+        float* o = out + (size_t)dd * a.out_pitch;
 #pragma unroll
-    for (int d = 0; d < 2; d++)
+        for (int w = 0; w < W; w++) {
+          const int t = t0 + word0 + 32 * w;
+          uint32_t v[4];
+          if (dd_dot(w)) {
+            v[0] = raw[d][w] % 65535u;
+            v[1] = raw[d][w] / 65535u;
+            v[2] = odd[d][w] % 65535u;
+            v[3] = odd[d][w] / 65535u;
+          } else {
+            const uint32_t even = raw[d][w] - (odd[d][w] << 8);
+            v[0] = even & 0xFFFFu;
+            v[1] = odd[d][w] & 0xFFFFu;
+            v[2] = even >> 16;
+            v[3] = odd[d][w] >> 16;
+          }
+          if (t < a.split) {
 #pragma unroll
-      for (int w = 0; w < W; w++) {
-        const uint32_t odd = pk[d][w][1];
-        const uint32_t even = pk[d][w][0] - (odd << 8);
-        if constexpr (A16) {
-          // only drain before the last: the accumulators are still zero
-          acc[d][w][0] = even;
-          acc[d][w][1] = odd;
-        } else {
-          acc[d][w][0] += even & 0xFFFFu;
-          acc[d][w][2] += even >> 16;
-          acc[d][w][1] += odd & 0xFFFFu;
-          acc[d][w][3] += odd >> 16;
+            for (int q = 0; q < 4; q++) {
+              const int at = t + q * a.split;
+              if (at < a.nout) {
+                if (last) {
+                  uint32_t sum = v[q];
+                  if (!first) sum += __ldcg(reinterpret_cast<const unsigned*>(o) + at);
+                  o[at] = __uint2float_rn(sum);
+                } else if (first) {
+                  __stcg(reinterpret_cast<unsigned*>(o) + at, v[q]);
+                } else {
+                  atomicAdd(reinterpret_cast<unsigned*>(o) + at, v[q]);
+                }
+              }
+            }
+          }
         }
-        pk[d][w][0] = pk[d][w][1] = 0;
       }
+#pragma unroll
+      for (int w = 0; w < W; w++) raw[d][w] = odd[d][w] = 0;
+    }
   };
-  // first word of this lane in group 0; group g adds 32*K*g words
-  const int lw = K * lane;
 
   int nsum = 0;
-  bool failed = false;
-  for (int st = 0; st < nstage; st++) {
-    const int buf = st % NST;
-    if (!mbar_wait(&full[buf], (uint32_t)((st / NST) & 1), a.wait_limit)) {
+  bool first = true;
+  for (int st = 0, k0 = 0; k0 < a.nact; st++) {
+    const int buf = st % DD_NST;
+    if (!mbar_wait(&full[buf], (uint32_t)((st / DD_NST) & 1), a.wait_limit)) {
       if (lane == 0) atomicOr(a.err, 1u);
-      failed = true;
-      break;
+      return;
     }
-    const int k0 = st * CH;
-    const int nk = min(CH, a.nact - k0);
-    const int2* off = s_off + buf * DB * CH + (2 * warp) * CH;
-    const uint32_t* rows32 = reinterpret_cast<const uint32_t*>(rows);
-    const uint32_t one = a.one;
-    int k = 0;
-    for (; k + 1 < nk; k += 2) {
+    const int nk = nrows[buf];
+    k0 += nk;
+    if (nsum + nk > DD_RUN) {
+      flush(first, false);
+      first = false;
+      nsum = 0;
+    }
+    const int* off = reinterpret_cast<const int*>(smem + OFFS) + (buf * DB + DPW * wd) * CH;
+    for (int k = 0; k < nk; k += UC) {
 #pragma unroll
-      for (int d = 0; d < 2; d++) {
-        const int2 oa = off[d * CH + k];
-        const int2 ob = off[d * CH + k + 1];
-        const uint32_t* pa = rows32 + (oa.x + lw);
-        const uint32_t* pb = rows32 + (ob.x + lw);
+      for (int d = 0; d < DPW; d++) {
+        int o[UC];
+        if constexpr (UC == 4) {
+          const int4 v = *reinterpret_cast<const int4*>(off + d * CH + k);
+          o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+        } else {
+          const int2 v = *reinterpret_cast<const int2*>(off + d * CH + k);
+          o[0] = v.x; o[1] = v.y;
+        }
+        const uint32_t* p[UC];
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-          uint32_t wa[K + 1], wb[K + 1];
+        for (int u = 0; u < UC; u++) p[u] = reinterpret_cast<const uint32_t*>(lane_base + o[u]);
 #pragma unroll
-          for (int j = 0; j <= K; j++) {
-            wa[j] = pa[32 * K * g + j];
-            wb[j] = pb[32 * K * g + j];
-          }
+        for (int w = 0; w < W; w++) {
+          uint32_t x[UC];
 #pragma unroll
-          for (int j = 0; j < K; j++) {
-            const uint32_t xa = __funnelshift_r(wa[j], wa[j + 1], oa.y);
-            const uint32_t xb = __funnelshift_r(wb[j], wb[j + 1], ob.y);
-            pk[d][K * g + j][0] += xa + xb;
-            pk[d][K * g + j][1] = mad_u32(__byte_perm(xb, 0u, 0x4341), one,
-                                          mad_u32(__byte_perm(xa, 0u, 0x4341), one,
-                                                  pk[d][K * g + j][1]));
+          for (int u = 0; u < UC; u++) x[u] = p[u][32 * w];
+#pragma unroll
+          for (int u = 0; u < UC; u += 2) {
+            if (dd_dot(w)) {
+              raw[d][w] = __dp2a_lo(kDot, x[u + 1], __dp2a_lo(kDot, x[u], raw[d][w]));
+              odd[d][w] = __dp2a_hi(kDot, x[u + 1], __dp2a_hi(kDot, x[u], odd[d][w]));
+            } else {
+              raw[d][w] += x[u] + x[u + 1];
+              odd[d][w] += __byte_perm(x[u], 0u, 0x4341) + __byte_perm(x[u + 1], 0u, 0x4341);
+            }
           }
         }
       }
-      nsum += 2;
-      if (nsum >= 256) { drain(); nsum = 0; }
     }
-    if (k < nk) {
-#pragma unroll
-      for (int d = 0; d < 2; d++) {
-        const int2 oa = off[d * CH + k];
-        const uint32_t* pa = rows32 + (oa.x + lw);
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-          uint32_t wa[K + 1];
-#pragma unroll
-          for (int j = 0; j <= K; j++) wa[j] = pa[32 * K * g + j];
-#pragma unroll
-          for (int j = 0; j < K; j++) {
-            const uint32_t xa = __funnelshift_r(wa[j], wa[j + 1], oa.y);
-            pk[d][K * g + j][0] += xa;
-            pk[d][K * g + j][1] = mad_u32(__byte_perm(xa, 0u, 0x4341), one, pk[d][K * g + j][1]);
-          }
-        }
-      }
-      nsum += 1;
-      if (nsum >= 256) { drain(); nsum = 0; }
-    }
+    nsum += nk;
     __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
-                                :: "r"(smem_addr(&empty[buf])) : "memory");
+    if (lane == 0) mbar_arrive(&empty[buf]);
   }
-  if (failed) return;
-  if constexpr (!A16) drain();
-  float* __restrict__ out = a.out + (size_t)blockIdx.z * a.out_unit;
+  flush(first, true);
+}
+
+// Channel-major byte rows -> four-sample words: word t of channel c holds
+// samples t, t + S, t + 2S, t + 3S of the row, for t < nwords (bytes past the
+// row's pitch read as 0; they reach no output).  Thread: 16 words, four
+// 16-byte loads and four 16-byte stores (S, the pitches and the bases are
+// multiples of 16).
+__global__ void __launch_bounds__(256) k_split_words(const uint8_t* __restrict__ in,
+                                                     size_t in_pitch, size_t in_unit, int split,
+                                                     int nwords, uint32_t* __restrict__ out,
+                                                     size_t out_pitch, size_t out_unit) {
+  const int t = 16 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= nwords) return;
+  const uint8_t* row = in + (size_t)blockIdx.z * in_unit + (size_t)blockIdx.y * in_pitch;
+  uint4 v[4];
 #pragma unroll
-  for (int d = 0; d < 2; d++) {
-    int dd = d_lo + 2 * warp + d;
-    if (dd >= a.dm_count) continue;
-    float* o = out + (size_t)dd * a.out_pitch;
+  for (int q = 0; q < 4; q++) {
+    const size_t at = (size_t)t + (size_t)q * split;
+    v[q] = at + 16 <= in_pitch ? __ldg(reinterpret_cast<const uint4*>(row + at))
+                               : make_uint4(0u, 0u, 0u, 0u);
+  }
+  uint4* o = reinterpret_cast<uint4*>(out + (size_t)blockIdx.z * out_unit +
+                                      (size_t)blockIdx.y * out_pitch + t);
+  const uint32_t* x = reinterpret_cast<const uint32_t*>(v);
 #pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-      for (int j = 0; j < K; j++) {
-        const int w = K * g + j;
-        size_t t = t0 + 4 * (32 * K * g + lw + j);
-        uint32_t s0, s1, s2, s3;
-        if constexpr (A16) {
-          const uint32_t odd = pk[d][w][1];
-          const uint32_t even = pk[d][w][0] - (odd << 8);
-          s0 = (even & 0xFFFFu) + (acc[d][w][0] & 0xFFFFu);
-          s2 = (even >> 16) + (acc[d][w][0] >> 16);
-          s1 = (odd & 0xFFFFu) + (acc[d][w][1] & 0xFFFFu);
-          s3 = (odd >> 16) + (acc[d][w][1] >> 16);
-        } else {
-          s0 = acc[d][w][0];
-          s1 = acc[d][w][1];
-          s2 = acc[d][w][2];
-          s3 = acc[d][w][3];
-        }
-        float4 v = make_float4((float)s0, (float)s1, (float)s2, (float)s3);
-        if (t + 3 < a.nout) {
-          *reinterpret_cast<float4*>(o + t) = v;
-        } else {
-          if (t < a.nout) o[t] = v.x;
-          if (t + 1 < a.nout) o[t + 1] = v.y;
-          if (t + 2 < a.nout) o[t + 2] = v.z;
-        }
-      }
+  for (int j = 0; j < 4; j++) {
+    const uint32_t a0 = x[j], a1 = x[4 + j], a2 = x[8 + j], a3 = x[12 + j];
+    const uint32_t lo01 = __byte_perm(a0, a1, 0x5140), lo23 = __byte_perm(a2, a3, 0x5140);
+    const uint32_t hi01 = __byte_perm(a0, a1, 0x7362), hi23 = __byte_perm(a2, a3, 0x7362);
+    o[j] = make_uint4(__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                      __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632));
   }
 }
 
@@ -933,74 +963,86 @@ cudaError_t narrow_band(uint8_t* tf, size_t units, size_t nsamps, int nchans, fl
   return cudaGetLastError();
 }
 
-namespace {
-constexpr int DD_NST = 3;
-// Shared memory of a variant: DB = dm_block DMs, `ch` channel rows per stage.
-size_t dd_smem(int dm_block, int ch, int rowb) {
-  return 128 + (size_t)DD_NST * dm_block * ch * sizeof(int2) + (size_t)DD_NST * ch * rowb;
+// Shared memory of a tile with stage buffers of cap bytes.
+size_t dedisp_smem_bytes(int dm_block, int time_block, int cap) {
+  return 128 + (size_t)time_block + (size_t)DD_NST * dm_block * DD_ROWS * 4 +
+         (size_t)DD_NST * cap;
 }
-template <int NW, int K, int G, int CH>
-cudaError_t launch_dd(const DedispArgs& a, cudaStream_t s) {
-  // the compact drain holds two 257-channel chunks at most
-  auto kern = a.nact <= 511 ? k_dedisp<NW, K, G, CH, DD_NST, true>
-                            : k_dedisp<NW, K, G, CH, DD_NST, false>;
-  const size_t smem = dd_smem(2 * NW, CH, a.rowb);
-  cudaError_t e = raise_smem_limit(kern, smem);
-  if (e != cudaSuccess) return e;
-  const int DB = 2 * NW, TB = 128 * K * G;
-  dim3 grid((unsigned)((a.dm_count + DB - 1) / DB), (unsigned)((a.nout + TB - 1) / TB),
-            (unsigned)a.units);
-  kern<<<grid, (NW + 1) * 32, smem, s>>>(a); note_launch();
-  return cudaGetLastError();
-}
-template <int NW, int K, int G>
-cudaError_t launch_rows(const DedispArgs& a, int rows, cudaStream_t s) {
-  switch (rows) {
-    case 16: return launch_dd<NW, K, G, 16>(a, s);
-    case 8: return launch_dd<NW, K, G, 8>(a, s);
-    case 4: return launch_dd<NW, K, G, 4>(a, s);
-    case 2: return launch_dd<NW, K, G, 2>(a, s);
-    case 1: return launch_dd<NW, K, G, 1>(a, s);
-    default: return cudaErrorInvalidValue;
-  }
-}
-}  // namespace
 
-// Channel rows per stage (16, 8, 4, 2 or 1): the most that keep three CTAs on
-// an SM (72 KB each), else two (110 KB), else one (200 KB).  More rows per
-// stage spread the per-stage waits and hand-offs over more channels.  Rows are long when few
-// channels cover a wide DM range (a DM block's delay span is long).  The
-// sums are exact integers, so the choice does not change the result.
-int dedisp_rows_per_stage(int dm_block, int rowb) {
-  for (size_t cap : {(size_t)72 * 1024, (size_t)110 * 1024, (size_t)200 * 1024})
-    for (int ch = 16; ch >= 1; ch /= 2)
-      if (dd_smem(dm_block, ch, rowb) <= cap) return ch;
+// Bytes of a stage buffer: kDedispRows rows of the mean length, or what four
+// CTAs on an SM leave for one (54 KB each, two buffers) if that is less, but
+// the longest row at least, with fewer CTAs where that takes more (0: it fits
+// nowhere).  Two long stages beat three short ones: each stage costs every
+// warp a wait and a hand-over (survey gulp, 1024 channels x 2^18, 8 x 1280:
+// 12.2 ms with two stages of 15 rows on average, 13.3 with three of 10, 14.5
+// with four of 7).  The sums are exact integers, so the choice does not change
+// the result.
+int dedisp_stage_bytes(int dm_block, int time_block, int mean_row, int longest_row) {
+  const size_t fixed = dedisp_smem_bytes(dm_block, time_block, 0);
+  for (size_t room : {(size_t)54 * 1024, (size_t)72 * 1024, (size_t)110 * 1024,
+                      (size_t)200 * 1024}) {
+    const size_t cap = (room - fixed) / DD_NST & ~(size_t)15;
+    if (cap >= (size_t)longest_row)
+      return (int)std::min(cap, std::max<size_t>((size_t)kDedispRows * mean_row + 1024, longest_row) &
+                                    ~(size_t)15);
+  }
   return 0;
 }
 
-size_t dedisp_smem_bytes(int dm_block, int rows, int rowb) {
-  return dd_smem(dm_block, rows, rowb);
+namespace {
+template <int NWD, int NWT, int DPW, int W, int UC>
+cudaError_t launch_dd(const DedispArgs& a, size_t smem, cudaStream_t s) {
+  auto kern = k_dedisp<NWD, NWT, DPW, W, UC>;
+  cudaError_t e = raise_smem_limit(kern, smem);
+  if (e != cudaSuccess) return e;
+  const int DB = DPW * NWD, TBW = 32 * W * NWT;
+  dim3 grid((unsigned)((a.dm_count + DB - 1) / DB), (unsigned)((a.split + TBW - 1) / TBW),
+            (unsigned)a.units);
+  kern<<<grid, (NWD * NWT + 1) * 32, smem, s>>>(a); note_launch();
+  return cudaGetLastError();
 }
+}  // namespace
 
-cudaError_t launch_dedisp(const DedispArgs& a, const DedispTile& t, cudaStream_t s) {
-  if (a.units < 1 || a.units > 65535) return cudaErrorInvalidValue;
-  // {dm_block, time_block} -> consumer warps NW = dm_block / 2, words per
-  // lane K, groups G with time_block = 128 K G (kDedispTiles)
-#define HDB_DD_TILE(DBk, NWk, Kk, Gk) \
-  if (t.dm_block == DBk && t.time_block == 128 * Kk * Gk) return launch_rows<NWk, Kk, Gk>(a, t.rows, s);
-  HDB_DD_TILE(8, 4, 1, 8)
-  HDB_DD_TILE(8, 4, 5, 1)
-  HDB_DD_TILE(8, 4, 3, 2)
-  HDB_DD_TILE(8, 4, 3, 3)
-  HDB_DD_TILE(8, 4, 5, 2)
-  HDB_DD_TILE(16, 8, 1, 4)
-  HDB_DD_TILE(16, 8, 3, 1)
-  HDB_DD_TILE(16, 8, 5, 1)
-  HDB_DD_TILE(16, 8, 3, 2)
-  HDB_DD_TILE(32, 16, 1, 2)
-  HDB_DD_TILE(32, 16, 3, 1)
+cudaError_t launch_dedisp(const DedispArgs& a0, const DedispTile& t, cudaStream_t s) {
+  if (a0.units < 1 || a0.units > 65535) return cudaErrorInvalidValue;
+  DedispArgs a = a0;
+  a.cap = t.stage;
+  const size_t smem = dedisp_smem_bytes(t.dm_block, t.time_block, t.stage);
+  // {dm_block, time_block} -> consumer warps over the DMs (NWD, DPW trials
+  // each) and over the words (NWT), W words per lane: time_block = 128 W NWT
+#define HDB_DD_TILE(DBk, NWDk, NWTk, DPWk, Wk)                                       \
+  if (t.dm_block == DBk && t.time_block == 128 * Wk * NWTk)                          \
+    return launch_dd<NWDk, NWTk, DPWk, Wk, 4>(a, smem, s);
+  HDB_DD_TILE(8, 4, 1, 2, 8)
+  HDB_DD_TILE(8, 4, 1, 2, 5)
+  HDB_DD_TILE(8, 4, 1, 2, 6)
+  HDB_DD_TILE(8, 4, 1, 2, 9)
+  HDB_DD_TILE(8, 4, 1, 2, 10)
+  HDB_DD_TILE(16, 8, 1, 2, 4)
+  HDB_DD_TILE(16, 8, 1, 2, 3)
+  HDB_DD_TILE(16, 8, 1, 2, 5)
+  HDB_DD_TILE(16, 8, 1, 2, 6)
+  HDB_DD_TILE(32, 16, 1, 2, 2)
+  HDB_DD_TILE(32, 16, 1, 2, 3)
+  HDB_DD_TILE(2, 1, 4, 2, 10)
+  HDB_DD_TILE(1, 1, 4, 1, 16)
 #undef HDB_DD_TILE
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_split_words(const uint8_t* in, size_t in_pitch, size_t in_unit, int nchans,
+                               size_t units, int split, size_t nwords, uint32_t* out,
+                               size_t out_pitch, size_t out_unit, cudaStream_t s) {
+  if (units < 1 || units > 65535 || nchans < 1 || nchans > 65535 || in_pitch % 16 ||
+      in_unit % 16 || split % 16 || out_pitch % 16 || out_unit % 4 || nwords > out_pitch ||
+      nwords > 0x7FFFFFF0ull)
+    return cudaErrorInvalidValue;
+  const unsigned nthr = (unsigned)((nwords + 15) / 16);
+  dim3 grid((nthr + 255) / 256, (unsigned)nchans, (unsigned)units);
+  k_split_words<<<grid, 256, 0, s>>>(in, in_pitch, in_unit, split, (int)nwords, out, out_pitch,
+                                     out_unit);
+  note_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace hdb

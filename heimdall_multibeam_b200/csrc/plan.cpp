@@ -96,12 +96,50 @@ static void free_dev(void* p) {
 static void free_groups(dedisp_plan p) {
   for (auto& g : p->groups) {
     free_dev(g.d_delays);
-    for (int* b : g.d_blk_min) free_dev(b);
+    for (int2* b : g.d_blk_range) free_dev(b);
   }
   p->groups.clear();
 }
 
-// Trials of one scrunch factor: delays at that factor, per DM-block minima
+// Per DM-block size: the least and the largest delay of every (block, channel),
+// and over those the largest and the mean span.
+static void block_ranges(const std::vector<int>& delays, size_t D, size_t C,
+                         std::vector<int2>* range, size_t* max_span, size_t* mean_span) {
+  for (int k = 0; k < kDedispDmBlockSizes; k++) {
+    const size_t DB = (size_t)kDedispDmBlocks[k];
+    const size_t nblk = (D + DB - 1) / DB;
+    range[k].resize(nblk * C);
+    max_span[k] = 0;
+    size_t sum = 0;
+    for (size_t b = 0; b < nblk; b++) {
+      int2* r = range[k].data() + b * C;
+      const size_t d1 = std::min(D, (b + 1) * DB);
+      for (size_t d = b * DB; d < d1; d++) {
+        const int* dl = delays.data() + d * C;
+        for (size_t c = 0; c < C; c++)
+          r[c] = d == b * DB ? int2{dl[c], dl[c]}
+                             : int2{std::min(r[c].x, dl[c]), std::max(r[c].y, dl[c])};
+      }
+      for (size_t c = 0; c < C; c++) {
+        max_span[k] = std::max(max_span[k], (size_t)(r[c].y - r[c].x));
+        sum += (size_t)(r[c].y - r[c].x);
+      }
+    }
+    mean_span[k] = range[k].empty() ? 0 : sum / range[k].size();
+  }
+}
+
+static dedisp_error upload_ranges(const std::vector<int2>* range, int2** d_range) {
+  for (int k = 0; k < kDedispDmBlockSizes; k++) {
+    const size_t bytes = range[k].size() * sizeof(int2);
+    if (dev_malloc(&d_range[k], bytes) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
+    if (cudaMemcpy(d_range[k], range[k].data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+      return DEDISP_MEM_COPY_FAILED;
+  }
+  return DEDISP_NO_ERROR;
+}
+
+// Trials of one scrunch factor: delays at that factor, per DM-block ranges
 // and spans, uploaded.
 static dedisp_error build_groups(dedisp_plan p) {
   free_groups(p);
@@ -122,21 +160,7 @@ static dedisp_error build_groups(dedisp_plan p) {
         g.delays[i * C + c] = v;
         g.max_delay = std::max(g.max_delay, (size_t)v);
       }
-    for (int k = 0; k < 3; k++) {
-      const size_t DB = (size_t)kDedispDmBlocks[k];
-      const size_t nblk = (Dg + DB - 1) / DB;
-      g.blk_min[k].assign(nblk * C, 0);
-      for (size_t b = 0; b < nblk; b++)
-        for (size_t c = 0; c < C; c++) {
-          int lo = 0x7FFFFFFF, hi = 0;
-          for (size_t i = b * DB; i < std::min(Dg, (b + 1) * DB); i++) {
-            lo = std::min(lo, g.delays[i * C + c]);
-            hi = std::max(hi, g.delays[i * C + c]);
-          }
-          g.blk_min[k][b * C + c] = lo;
-          g.max_span[k] = std::max(g.max_span[k], (size_t)(hi - lo));
-        }
-    }
+    block_ranges(g.delays, Dg, C, g.blk_range, g.max_span, g.mean_span);
     p->groups.push_back(std::move(g));
     dedisp_plan_struct::Group& G = p->groups.back();
     if (dev_malloc(&G.d_delays, G.delays.size() * sizeof(int)) != cudaSuccess)
@@ -144,13 +168,8 @@ static dedisp_error build_groups(dedisp_plan p) {
     if (cudaMemcpy(G.d_delays, G.delays.data(), G.delays.size() * sizeof(int),
                    cudaMemcpyHostToDevice) != cudaSuccess)
       return DEDISP_MEM_COPY_FAILED;
-    for (int k = 0; k < 3; k++) {
-      if (dev_malloc(&G.d_blk_min[k], G.blk_min[k].size() * sizeof(int)) != cudaSuccess)
-        return DEDISP_MEM_ALLOC_FAILED;
-      if (cudaMemcpy(G.d_blk_min[k], G.blk_min[k].data(), G.blk_min[k].size() * sizeof(int),
-                     cudaMemcpyHostToDevice) != cudaSuccess)
-        return DEDISP_MEM_COPY_FAILED;
-    }
+    const dedisp_error e = upload_ranges(G.blk_range, G.d_blk_range);
+    if (e != DEDISP_NO_ERROR) return e;
   }
   return DEDISP_NO_ERROR;
 }
@@ -168,22 +187,7 @@ dedisp_error plan_prepare(dedisp_plan p) {
       p->delays[d * C + c] = (int)v;
       p->max_delay = std::max(p->max_delay, v);
     }
-  for (int k = 0; k < 3; k++) {
-    const size_t DB = (size_t)kDedispDmBlocks[k];
-    const size_t nblk = (D + DB - 1) / DB;
-    p->blk_min[k].assign(nblk * C, 0);
-    p->max_span[k] = 0;
-    for (size_t b = 0; b < nblk; b++)
-      for (size_t c = 0; c < C; c++) {
-        int lo = 0x7FFFFFFF, hi = 0;
-        for (size_t d = b * DB; d < std::min(D, (b + 1) * DB); d++) {
-          lo = std::min(lo, p->delays[d * C + c]);
-          hi = std::max(hi, p->delays[d * C + c]);
-        }
-        p->blk_min[k][b * C + c] = lo;
-        p->max_span[k] = std::max(p->max_span[k], (size_t)(hi - lo));
-      }
-  }
+  block_ranges(p->delays, D, C, p->blk_range, p->max_span, p->mean_span);
   p->active.clear();
   for (size_t c = 0; c < C; c++)
     if (p->killmask[c]) p->active.push_back((int)c);
@@ -192,7 +196,7 @@ dedisp_error plan_prepare(dedisp_plan p) {
   cudaGetDevice(&dev);
   free_dev(p->d_delays); free_dev(p->d_active); free_dev(p->d_dm_list);
   p->d_delays = nullptr; p->d_active = nullptr; p->d_dm_list = nullptr;
-  for (auto& b : p->d_blk_min) {
+  for (auto& b : p->d_blk_range) {
     free_dev(b);
     b = nullptr;
   }
@@ -200,9 +204,6 @@ dedisp_error plan_prepare(dedisp_plan p) {
       hdb::dev_malloc(&p->d_active, (p->active.size() + 1) * sizeof(int)) != cudaSuccess ||
       hdb::dev_malloc(&p->d_dm_list, D * sizeof(float)) != cudaSuccess)
     return DEDISP_MEM_ALLOC_FAILED;
-  for (int k = 0; k < 3; k++)
-    if (hdb::dev_malloc(&p->d_blk_min[k], p->blk_min[k].size() * sizeof(int)) != cudaSuccess)
-      return DEDISP_MEM_ALLOC_FAILED;
   if (!p->d_err && hdb::dev_malloc(&p->d_err, sizeof(unsigned)) != cudaSuccess)
     return DEDISP_MEM_ALLOC_FAILED;
   cudaMemset(p->d_err, 0, sizeof(unsigned));
@@ -214,10 +215,8 @@ dedisp_error plan_prepare(dedisp_plan p) {
       cudaMemcpy(p->d_dm_list, p->dm_list.data(), D * sizeof(float), cudaMemcpyHostToDevice) !=
           cudaSuccess)
     return DEDISP_MEM_COPY_FAILED;
-  for (int k = 0; k < 3; k++)
-    if (cudaMemcpy(p->d_blk_min[k], p->blk_min[k].data(), p->blk_min[k].size() * sizeof(int),
-                   cudaMemcpyHostToDevice) != cudaSuccess)
-      return DEDISP_MEM_COPY_FAILED;
+  const dedisp_error re = upload_ranges(p->blk_range, p->d_blk_range);
+  if (re != DEDISP_NO_ERROR) return re;
   dedisp_error ge = build_groups(p);
   if (ge != DEDISP_NO_ERROR) return ge;
   p->device = dev;
@@ -227,36 +226,33 @@ dedisp_error plan_prepare(dedisp_plan p) {
 }
 
 static int dm_block_index(int dm_block) {
-  for (int k = 0; k < 3; k++)
+  for (int k = 0; k < kDedispDmBlockSizes; k++)
     if (kDedispDmBlocks[k] == dm_block) return k;
   return -1;
 }
 
-// Staged row bytes of a tile: the DM block's delay span for one channel, the
-// time block, the 16-byte alignment of the copy and one word of look-ahead.
-static int rowb_of(const size_t* max_span, int dm_block, int time_block) {
-  size_t r = max_span[dm_block_index(dm_block)] + 16 + (size_t)time_block + 8;
-  return (int)((r + 15) & ~(size_t)15);
+// Bytes of a tile's staged row whose DM block spans `span` samples of delay:
+// the span and the tile's words, from a 16-byte boundary on (2^18, more than
+// fits, from 2^16 words on).
+static int row_bytes(size_t span, int time_block) {
+  const size_t words = span + 3 + (size_t)time_block / 4;
+  return words >= (size_t)1 << 16 ? 1 << 18 : (int)((4 * words + 15) & ~(size_t)15);
 }
 
-// Row pitch of a channel-major input of nsamps samples whose trials reach
-// max_delay and produce nout samples: room for the longest staged row of
-// every candidate tile past the last time block.
-static size_t ft_pitch_for(const size_t* max_span, size_t max_delay, size_t nsamps,
-                           size_t nout) {
-  size_t need = nsamps + 4;
-  for (const auto& t : kDedispTiles) {
-    const size_t tb = (size_t)t[1];
-    const size_t ntb = (nout + tb - 1) / tb;
-    need = std::max(need, ntb * tb + max_delay + (size_t)rowb_of(max_span, t[0], t[1]));
+// Delay spans that dedispersion takes: one staged row of a DM block's span as
+// bytes, with 8, 16 or 32 trials per block, must fit 200 KB three times over.
+static bool spans_supported(const size_t* max_span) {
+  const size_t least[3] = {640, 384, 256};
+  for (int k = 0; k < 3; k++) {
+    const size_t rowb = (max_span[k] + 16 + least[k] + 8 + 15) & ~(size_t)15;
+    if (128 + 3 * (size_t)kDedispDmBlocks[k] * 8 + 3 * rowb <= (size_t)200 * 1024) return true;
   }
-  need += 64;
-  return (need + 63) & ~(size_t)63;
+  return false;
 }
 
-size_t ft_pitch(const dedisp_plan p, size_t nsamps) {
-  size_t nout = nsamps > p->max_delay ? nsamps - p->max_delay : 0;
-  return ft_pitch_for(p->max_span, p->max_delay, nsamps, nout);
+// Row pitch of a channel-major input of nsamps samples.
+size_t ft_pitch(const dedisp_plan, size_t nsamps) {
+  return (nsamps + 64 + 63) & ~(size_t)63;
 }
 
 // ---------------------------------------------------------------------------
@@ -274,7 +270,7 @@ size_t ft_pitch(const dedisp_plan p, size_t nsamps) {
 // ---------------------------------------------------------------------------
 namespace {
 // bump when the dedispersion kernel changes, so stale choices are not reused
-constexpr uint64_t kDedispKernelGeneration = 6;
+constexpr uint64_t kDedispKernelGeneration = 7;
 
 struct TileCache {
   std::mutex mu;
@@ -373,8 +369,9 @@ void tile_cache_put(uint64_t key, const std::array<int, 3>& t) {
 // samples per trial; the tile is tuned per (nsamps, units, tune_key) and kept
 // in the persistent tile cache.
 static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_delays,
-                                      const int* d_delays, int* const* d_blk_min,
-                                      const size_t* max_span, int dm_count, size_t nout,
+                                      const int* d_delays, int2* const* d_blk_range,
+                                      const size_t* max_span, const size_t* mean_span,
+                                      size_t max_delay, int dm_count, size_t nout,
                                       size_t tune_key, const uint8_t* d_ft, size_t pitch,
                                       size_t nsamps, float* d_out, size_t out_pitch,
                                       cudaStream_t s, size_t units, size_t in_unit,
@@ -387,20 +384,63 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
         return DEDISP_INTERNAL_GPU_ERROR;
     return DEDISP_NO_ERROR;
   }
-  DedispArgs a;
-  a.in = d_ft;
-  a.in_pitch = pitch;
+  if (units > 65535) return DEDISP_INVALID_STRIDE;
+  // one channel row of the widest block's delay span must fit shared memory
+  if (!spans_supported(max_span)) return DEDISP_NCHANS_EXCEEDS_LIMIT;
+  // candidate tiles {dm_block, time_block, mean rows per stage} whose staged
+  // rows fit shared memory
+  std::vector<std::array<int, 3>> cand;
+  auto stage_of = [&](int dm_block, int time_block) {
+    const int k = dm_block_index(dm_block);
+    return dedisp_stage_bytes(dm_block, time_block, row_bytes(mean_span[k], time_block),
+                              row_bytes(max_span[k], time_block));
+  };
+  auto offer = [&](const int* t) {
+    const int stage = stage_of(t[0], t[1]);
+    const int mean = row_bytes(mean_span[dm_block_index(t[0])], t[1]);
+    if (stage) cand.push_back({t[0], t[1], std::max(1, std::min(kDedispRows, stage / mean))});
+  };
+  for (const auto& t : kDedispTiles) offer(t);
+  if (cand.empty())
+    for (const auto& t : kDedispLongTiles) offer(t);
+  // ---- the four-sample words of the input ----
+  const size_t split = ((nout + 3) / 4 + 15) & ~(size_t)15;
+  const size_t nwords = (split + max_delay + 15) & ~(size_t)15;
+  size_t wpitch = nwords;
+  for (const auto& t : cand) {
+    const size_t tbw = (size_t)t[1] / 4, ntb = (split + tbw - 1) / tbw;
+    wpitch = std::max(wpitch, ntb * tbw + max_delay + 8);  // past the last tile's rows
+  }
+  wpitch = (wpitch + 15) & ~(size_t)15;
+  const size_t wunit = wpitch * p->nchans;
+  if (p->d_words_cap < units * wunit) {
+    free_dev(p->d_words);
+    p->d_words = nullptr;
+    p->d_words_cap = 0;
+    if (dev_malloc(&p->d_words, units * wunit * sizeof(uint32_t)) != cudaSuccess)
+      return DEDISP_MEM_ALLOC_FAILED;
+    p->d_words_cap = units * wunit;
+  }
+  if (nout > 0x7FFFFFFFull - 4096 ||
+      launch_split_words(d_ft, pitch, in_unit, (int)p->nchans, units, (int)split, nwords,
+                         p->d_words, wpitch, wunit, s) != cudaSuccess)
+    return DEDISP_INTERNAL_GPU_ERROR;
+  DedispArgs a{};
+  a.in = p->d_words;
+  a.in_pitch = wpitch;
+  a.split = (int)split;
   a.delays = d_delays;
   a.chans = p->d_active;
   a.nact = (int)p->active.size();
   a.nchans = (int)p->nchans;
   a.dm_count = dm_count;
-  a.nout = nout;
+  a.nout = (int)nout;
   a.out = d_out;
   a.out_pitch = out_pitch;
+  a.cap = 0;
   a.err = p->d_err;
   a.units = (int)units;
-  a.in_unit = in_unit;
+  a.in_unit = wunit;
   a.out_unit = out_unit;
   a.wait_limit = kDedispWaitLimit;
   a.withhold_last = 0;
@@ -412,20 +452,10 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
       a.withhold_last = 1;
       a.wait_limit = 1u << 12;
     }
-  if (units > 65535) return DEDISP_INVALID_STRIDE;
   auto with_tile = [&](const std::array<int, 3>& t) {
-    a.blk_min = d_blk_min[dm_block_index(t[0])];
-    a.rowb = rowb_of(max_span, t[0], t[1]);
-    return DedispTile{t[0], t[1], t[2]};
+    a.blk_range = d_blk_range[dm_block_index(t[0])];
+    return DedispTile{t[0], t[1], stage_of(t[0], t[1])};
   };
-  // candidate tiles whose staged rows fit shared memory
-  std::vector<std::array<int, 3>> cand;
-  for (const auto& t : kDedispTiles) {
-    const int rows = dedisp_rows_per_stage(t[0], rowb_of(max_span, t[0], t[1]));
-    if (rows) cand.push_back({t[0], t[1], rows});
-  }
-  // one channel row of the widest block's delay span must fit shared memory
-  if (cand.empty()) return DEDISP_NCHANS_EXCEEDS_LIMIT;
   const std::array<size_t, 3> key = {nsamps, units, tune_key};
   auto it = p->tiles.find(key);
   if (it == p->tiles.end()) {
@@ -498,8 +528,8 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
   if (nsamps < p->max_delay) return DEDISP_TOO_FEW_NSAMPS;
   const size_t nout = nsamps - p->max_delay;
   if (p->groups.empty())
-    return dedisperse_tables(p, p->delays, p->d_delays, p->d_blk_min, p->max_span,
-                             (int)p->dm_list.size(), nout, 0, d_ft, pitch, nsamps, d_out,
+    return dedisperse_tables(p, p->delays, p->d_delays, p->d_blk_range, p->max_span,
+                             p->mean_span, p->max_delay, (int)p->dm_list.size(), nout, 0, d_ft, pitch, nsamps, d_out,
                              out_pitch, s, units, in_unit, out_unit);
   // adaptive dt: group g's trials [d0, d1) of every unit are rows
   // units * d0 + u * (d1 - d0) + i of the output (group-major)
@@ -510,12 +540,13 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
     const size_t nout_s = nout / g.s;
     float* out_g = d_out + units * g.d0 * out_pitch;
     if (g.s == 1) {
-      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_min, g.max_span, (int)Dg, nout_s, gi + 1,
+      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span,
+                             g.mean_span, g.max_delay, (int)Dg, nout_s, gi + 1,
                              d_ft, pitch, nsamps, out_g, out_pitch, s, units, in_unit,
                              Dg * out_pitch);
     } else {
       const size_t ns = nsamps / g.s;
-      const size_t pitch_s = ft_pitch_for(g.max_span, g.max_delay, ns, nout_s);
+      const size_t pitch_s = ft_pitch(p, ns);
       const size_t need = units * pitch_s * C;
       if (p->d_scr_cap < need) {
         free_dev(p->d_scr);
@@ -527,7 +558,8 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
       if (launch_scrunch_ft(d_ft, pitch, nsamps, (int)C, (int)g.s, p->d_scr, pitch_s, units,
                             in_unit, pitch_s * C, s) != cudaSuccess)
         return DEDISP_INTERNAL_GPU_ERROR;
-      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_min, g.max_span, (int)Dg, nout_s, gi + 1,
+      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span,
+                             g.mean_span, g.max_delay, (int)Dg, nout_s, gi + 1,
                              p->d_scr, pitch_s, ns, out_g, out_pitch, s, units, pitch_s * C,
                              Dg * out_pitch);
     }
@@ -540,7 +572,7 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
 
 dedisp_plan_struct::~dedisp_plan_struct() {
   hdb::free_dev(d_delays);
-  for (int* b : d_blk_min) hdb::free_dev(b);
+  for (int2* b : d_blk_range) hdb::free_dev(b);
   hdb::free_dev(d_active);
   hdb::free_dev(d_dm_list);
   hdb::free_dev(d_err);
@@ -549,6 +581,7 @@ dedisp_plan_struct::~dedisp_plan_struct() {
   hdb::free_dev(d_out);
   hdb::free_dev(d_out_hi);
   hdb::free_dev(d_scr);
+  hdb::free_dev(d_words);
   hdb::free_groups(this);
   if (stream) cudaStreamDestroy(stream);
 }

@@ -14,6 +14,11 @@
 
 #include "dedisp.h"
 
+// Trials per block of the dedispersion tiles (the tables below hold one entry
+// per size)
+constexpr int kDedispDmBlockSizes = 5;
+constexpr int kDedispDmBlocks[kDedispDmBlockSizes] = {8, 16, 32, 2, 1};
+
 struct dedisp_plan_struct {
   dedisp_size nchans = 0;
   float dt = 0.f, f0 = 0.f, df = 0.f;
@@ -28,14 +33,16 @@ struct dedisp_plan_struct {
   bool dirty = true;
   unsigned long long gen = 0;      // counts the rebuilds of the device tables
   std::vector<int> delays;         // [dm][chan]
-  // per DM-block size (8, 16, 32 trials): [dm block][chan] minimum delay
-  std::vector<int> blk_min[3];
+  // per DM-block size (kDedispDmBlocks): [dm block][chan] least and largest
+  // delay
+  std::vector<int2> blk_range[kDedispDmBlockSizes];
   std::vector<int> active;         // channels with killmask != 0
   size_t max_delay = 0;
-  size_t max_span[3] = {0, 0, 0};  // max over blocks/chans of (max - min) delay
+  // over blocks and channels: the largest and the mean of (max - min) delay
+  size_t max_span[kDedispDmBlockSizes] = {}, mean_span[kDedispDmBlockSizes] = {};
   int* d_delays = nullptr;
-  int* d_blk_min[3] = {nullptr, nullptr, nullptr};
-  // dedispersion tile {dm_block, time_block, rows, source} per (nsamps,
+  int2* d_blk_range[kDedispDmBlockSizes] = {};
+  // dedispersion tile {dm_block, time_block, mean rows per stage, source} per (nsamps,
   // units, scrunch group): the fastest of the candidates, timed on first use
   // (autotuner) or read from the persistent tile cache
   std::map<std::array<size_t, 3>, std::array<int, 4>> tiles;
@@ -57,15 +64,17 @@ struct dedisp_plan_struct {
   struct Group {
     size_t d0 = 0, d1 = 0, s = 1;
     size_t max_delay = 0;            // largest scrunched delay of the group
-    size_t max_span[3] = {0, 0, 0};  // per DM-block size
+    size_t max_span[kDedispDmBlockSizes] = {}, mean_span[kDedispDmBlockSizes] = {};
     std::vector<int> delays;         // [d1 - d0][chan]
-    std::vector<int> blk_min[3];
+    std::vector<int2> blk_range[kDedispDmBlockSizes];
     int* d_delays = nullptr;
-    int* d_blk_min[3] = {nullptr, nullptr, nullptr};
+    int2* d_blk_range[kDedispDmBlockSizes] = {};
   };
   std::vector<Group> groups;          // built only with adaptive dt
   uint8_t* d_scr = nullptr;           // scrunched channel-major input
   size_t d_scr_cap = 0;
+  uint32_t* d_words = nullptr;        // four-sample words of the input being dedispersed
+  size_t d_words_cap = 0;             // words
 
   // scratch for dedisp_execute* with host pointers
   uint8_t* d_in_tf = nullptr;
