@@ -160,46 +160,65 @@ __global__ void k_weights_bf16(const float* __restrict__ w, int co, int kw, int 
   out[i] = __float2bfloat16(k < kw ? w[o * kw + k] : 0.f);
 }
 
-// im2col of a 3x3, pad-1 convolution: in [ci][b][h][w] -> col [kp][b*h*w]
-// (row ci*9 + ky*3 + kx; rows >= ci*9 are zero)
-__global__ void k_im2col3(const bf16* __restrict__ in, int ci, int nb, int h, int w, int kp,
-                          bf16* __restrict__ col) {
-  const size_t P = (size_t)nb * h * w;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P * kp) return;
-  const int r = (int)(i / P);
-  const size_t p = i % P;
-  bf16 v = __float2bfloat16(0.f);
-  if (r < ci * 9) {
-    const int c = r / 9, ky = (r % 9) / 3, kx = r % 3;
-    const int x = (int)(p % w), y = (int)((p / w) % h);
-    const size_t b = p / ((size_t)w * h);
-    const int yy = y + ky - 1, xx = x + kx - 1;
-    if (yy >= 0 && yy < h && xx >= 0 && xx < w)
-      v = in[(((size_t)c * nb + b) * h + yy) * w + xx];
+// im2col of a 3x3, pad-1 convolution: in [ci][b][h][w] -> col [ci*9][b*h*w],
+// row c*9 + ky*3 + kx (the weight gradient's operand).  Bound by its writes (9
+// values out per value in).  A thread makes the nine taps of eight pixels of
+// one image row from three 16-byte loads and their two neighbours, with
+// 16-byte stores (w is a multiple of 8): 45 us for 8 x 128 x 32 x 128 values
+// against 253 us with one value per thread.
+__global__ void __launch_bounds__(256) k_im2col3(const bf16* __restrict__ in, int h, int w,
+                                                 size_t P, bf16* __restrict__ col) {
+  const size_t p = 8 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+  if (p >= P) return;
+  const int c = blockIdx.y;
+  const int x = (int)(p % w), y = (int)((p / w) % h);
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(in) + (size_t)c * P + p;
+#pragma unroll
+  for (int ky = 0; ky < 3; ky++) {
+    const int yy = y + ky - 1;
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t left = 0, right = 0;  // pixel x - 1 in the upper half, x + 8 in the lower
+    if (yy >= 0 && yy < h) {
+      const uint16_t* r = src + (ptrdiff_t)(ky - 1) * w;
+      m = *reinterpret_cast<const uint4*>(r);
+      if (x > 0) left = (uint32_t)r[-1] << 16;
+      if (x + 8 < w) right = r[8];
+    }
+    const uint32_t a = __byte_perm(left, m.x, 0x5432), b = __byte_perm(m.x, m.y, 0x5432),
+                   d = __byte_perm(m.y, m.z, 0x5432), e = __byte_perm(m.z, m.w, 0x5432),
+                   f = __byte_perm(m.w, right, 0x5432);
+    bf16* o = col + (size_t)(c * 9 + ky * 3) * P + p;
+    *reinterpret_cast<uint4*>(o) = make_uint4(a, b, d, e);
+    *reinterpret_cast<uint4*>(o + P) = m;
+    *reinterpret_cast<uint4*>(o + 2 * P) = make_uint4(b, d, e, f);
   }
-  col[i] = v;
 }
 
-// im2col in K-major order for the tensor-core GEMM: colT [b*h*w][kp], the kp
-// taps of one output pixel contiguous (the same values as k_im2col3)
-__global__ void k_im2col3_t(const bf16* __restrict__ in, int ci, int nb, int h, int w, int kp,
-                            bf16* __restrict__ colT) {
-  const size_t P = (size_t)nb * h * w;
+// im2col in K-major order for the tensor-core GEMM: colT [b*h*w][KP], the KP
+// taps of one output pixel contiguous (tap k = c*9 + ky*3 + kx; zeros from
+// ci*9 on).  Bound by its writes.  A thread makes eight taps of one pixel, one
+// 16-byte store, neighbouring threads the next eight: every index is found
+// once per eight values and the stores are whole lines (82 us against 275 us
+// for 8 x 128 x 32 x 128 values in).
+template <int CI>
+__global__ void __launch_bounds__(256) k_im2col3_t(const bf16* __restrict__ in, int h, int w,
+                                                   size_t P, bf16* __restrict__ colT) {
+  constexpr int KP = (CI * 9 + 15) / 16 * 16, Q = KP / 8;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P * kp) return;
-  const size_t p = i / kp;
-  const int r = (int)(i % kp);
-  bf16 v = __float2bfloat16(0.f);
-  if (r < ci * 9) {
-    const int c = r / 9, ky = (r % 9) / 3, kx = r % 3;
-    const int x = (int)(p % w), y = (int)((p / w) % h);
-    const size_t b = p / ((size_t)w * h);
-    const int yy = y + ky - 1, xx = x + kx - 1;
-    if (yy >= 0 && yy < h && xx >= 0 && xx < w)
-      v = in[(((size_t)c * nb + b) * h + yy) * w + xx];
+  if (i >= P * Q) return;
+  const size_t p = i / Q;
+  const int q = (int)(i % Q);
+  const int x = (int)(p % w), y = (int)((p / w) % h);
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(in) + p;
+  uint32_t v[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const int k = 8 * q + j, c = k / 9, t = k % 9, dy = t / 3 - 1, dx = t % 3 - 1;
+    const bool in_image = k < CI * 9 && y + dy >= 0 && y + dy < h && x + dx >= 0 && x + dx < w;
+    v[j] = in_image ? src[(ptrdiff_t)c * (ptrdiff_t)P + dy * w + dx] : 0u;
   }
-  colT[i] = v;
+  reinterpret_cast<uint4*>(colT)[i] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16,
+                                                 v[4] | v[5] << 16, v[6] | v[7] << 16);
 }
 
 // col2im: dcol [kp][b*h*w] (FP32) -> din [ci][b][h][w], summing the 9 taps
@@ -251,58 +270,78 @@ __global__ void k_bias_relu_pool(const float* __restrict__ z, const float* __res
 }
 
 // backward of bias/ReLU/pool: dact [co][b][h/2][w/2] (FP32) -> dz [co][b][h][w]
-// (BF16, the next GEMM's operand), and the bias gradient
-__global__ void k_pool_relu_back(const float* __restrict__ dact, const bf16* __restrict__ act,
-                                 const unsigned char* __restrict__ arg, int co, int nb, int h,
-                                 int w, bf16* __restrict__ dz, float* __restrict__ dbias) {
-  const int h2 = h / 2, w2 = w / 2;
-  const size_t n = (size_t)co * nb * h * w;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float v = 0.f;
-  int c = -1;
-  if (i < n) {
-    const int x = (int)(i % w), y = (int)((i / w) % h);
-    const size_t cb = i / ((size_t)w * h);
-    c = (int)(cb / nb);
-    const size_t j = (cb * h2 + y / 2) * w2 + x / 2;
-    const int q = (y & 1) * 2 + (x & 1);
-    if (y / 2 < h2 && x / 2 < w2 && arg[j] == q && __bfloat162float(act[j]) > 0.f) v = dact[j];
-    dz[i] = __float2bfloat16(v);
+// (BF16, the next GEMM's operand), and the bias gradient's partial sums.  Each
+// pooled element passes its gradient to the one position that held its
+// maximum, so the bias gradient is the sum of dact over the positive pooled
+// activations: the kernel that reads them adds them up, a quarter of the
+// pre-pool elements.  A thread takes four pooled elements of a row (two 16-byte
+// stores; w is a multiple of 8); block (x, c) leaves its sum in part[c][x].
+// The former bias kernel walked all pre-pool elements with one block per
+// channel and was 80 % of a training step (8.5 ms of the largest layer; 12 us
+// now, the pre-activation gradient included).
+constexpr int kBiasParts = 64;
+__global__ void __launch_bounds__(256) k_pool_relu_back(const float* __restrict__ dact,
+                                                        const bf16* __restrict__ act,
+                                                        const unsigned char* __restrict__ arg,
+                                                        int nb, int h, int w,
+                                                        bf16* __restrict__ dz,
+                                                        float* __restrict__ part) {
+  const int c = blockIdx.y;
+  const int h2 = h / 2, q2 = w / 8;  // quads of a pooled row
+  const int nq = nb * h2 * q2;       // quads of this channel
+  float sum = 0.f;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < nq; i += gridDim.x * 256) {
+    const size_t j = ((size_t)c * nq + i) * 4;
+    const float4 d = *reinterpret_cast<const float4*>(dact + j);
+    const uint2 a = *reinterpret_cast<const uint2*>(act + j);
+    const uint32_t g = *reinterpret_cast<const uint32_t*>(arg + j);
+    const float dv[4] = {d.x, d.y, d.z, d.w};
+    const uint32_t ab[4] = {a.x & 0xFFFFu, a.x >> 16, a.y & 0xFFFFu, a.y >> 16};
+    uint32_t lo[4], hi[4];  // the two rows of the 2 x 2 windows
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      // a positive activation: the sign bit clear, the value not zero, not NaN
+      const bool on = ab[k] - 1u < 0x7F80u;
+      const int q = (int)((g >> (8 * k)) & 0xFFu);
+      const float v = on ? dv[k] : 0.f;
+      const uint32_t b = __bfloat16_as_ushort(__float2bfloat16(v));
+      if (on) sum += dv[k];
+      lo[k] = q < 2 ? b << (16 * q) : 0u;
+      hi[k] = q >= 2 ? b << (16 * (q - 2)) : 0u;
+    }
+    const int x8 = i % q2, row = i / q2;  // row = n * h2 + y2
+    bf16* o = dz + ((size_t)c * nb * h + 2 * (size_t)row) * w + 8 * x8;
+    *reinterpret_cast<uint4*>(o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    *reinterpret_cast<uint4*>(o + w) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   }
-  (void)c;
-  (void)dbias;
+  __shared__ float warp_sum[8];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float v = 0.f;
+    for (int k = 0; k < 8; k++) v += warp_sum[k];
+    part[c * kBiasParts + blockIdx.x] = v;
+  }
 }
 
-// bias gradient of the same layer: dbias[c] += the sum over c's pixels of the
-// pre-activation gradient, one block per channel, in a fixed order (each
-// thread's strided partial, then a fixed tree), so every run gives the same
-// bits
-__global__ void __launch_bounds__(256) k_bias_grad(const float* __restrict__ dact,
-                                                   const bf16* __restrict__ act,
-                                                   const unsigned char* __restrict__ arg,
-                                                   int nb, int h, int w,
-                                                   float* __restrict__ dbias) {
-  __shared__ float part[256];
-  const int c = blockIdx.x;
-  const int h2 = h / 2, w2 = w / 2;
-  const size_t per = (size_t)nb * h * w;
-  float acc = 0.f;
-  for (size_t k = threadIdx.x; k < per; k += blockDim.x) {
-    const size_t i = (size_t)c * per + k;
-    const int x = (int)(i % w), y = (int)((i / w) % h);
-    const size_t cb = i / ((size_t)w * h);
-    const size_t j = (cb * h2 + y / 2) * w2 + x / 2;
-    const int q = (y & 1) * 2 + (x & 1);
-    if (y / 2 < h2 && x / 2 < w2 && arg[j] == q && __bfloat162float(act[j]) > 0.f)
-      acc = __fadd_rn(acc, dact[j]);
-  }
-  part[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) part[threadIdx.x] = __fadd_rn(part[threadIdx.x], part[threadIdx.x + o]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) dbias[c] = __fadd_rn(dbias[c], part[0]);
+// the six layers' bias gradients, each channel's partial sums in a fixed order
+// (two per lane, then a fixed tree), so every run gives the same bits
+struct BiasSum {
+  int first[7];    // first channel of each layer among all channels
+  int parts[6];    // partial sums per channel
+  float* out[6];   // += the layer's bias gradient
+};
+__global__ void k_bias_sum(const float* __restrict__ part, BiasSum b) {
+  const int lane = threadIdx.x, c = blockIdx.x;
+  int l = 0;
+  while (c >= b.first[l + 1]) l++;
+  float v = lane < b.parts[l] ? part[c * kBiasParts + lane] : 0.f;
+  if (lane + 32 < b.parts[l]) v += part[c * kBiasParts + lane + 32];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) b.out[l][c - b.first[l]] += v;
 }
 
 // pooled activations of both branches -> x [b][10240] (A: 2048, B: 8192)
@@ -383,29 +422,43 @@ __global__ void k_head(const float* __restrict__ h, const float* __restrict__ w2
 }
 
 // loss (+= the per-sample terms), gb2, gw2 [2][16] and gb1 [16] from hs and
-// h, each a sum over the samples in order (thread per output)
-__global__ void k_head_reduce(const float* __restrict__ h, const float* __restrict__ hs, int nb,
-                              float* __restrict__ loss, float* __restrict__ gw2,
-                              float* __restrict__ gb2, float* __restrict__ gb1) {
+// h, each a sum over the samples in order (thread per output).  The chain of
+// adds is short; what took time (70 us at 128 samples) was a global load per
+// sample and output on it, so the block stages 128 samples at a time.
+constexpr int kHeadChunk = 128;
+__global__ void __launch_bounds__(256) k_head_reduce(const float* __restrict__ h,
+                                                     const float* __restrict__ hs, int nb,
+                                                     float* __restrict__ loss,
+                                                     float* __restrict__ gw2,
+                                                     float* __restrict__ gb2,
+                                                     float* __restrict__ gb1) {
+  __shared__ float sh[kHeadChunk * 16], st[kHeadChunk * kHeadTerms];
   const int k = threadIdx.x;  // 0: loss, 1-2: gb2, 3-34: gw2, 35-50: gb1
-  if (k > 50) return;
   float acc = 0.f;
-  for (int n = 0; n < nb; n++) {
-    const float* t = hs + (size_t)n * kHeadTerms;
-    const float d1 = t[1], d0 = -d1;
-    float v;
-    if (k == 0) v = t[0];
-    else if (k == 1) v = d0;
-    else if (k == 2) v = d1;
-    else if (k < 19) v = d0 * h[n * 16 + (k - 3)];
-    else if (k < 35) v = d1 * h[n * 16 + (k - 19)];
-    else v = t[2 + (k - 35)];
-    acc = __fadd_rn(acc, v);
+  for (int n0 = 0; n0 < nb; n0 += kHeadChunk) {
+    const int m = min(kHeadChunk, nb - n0);
+    __syncthreads();
+    for (int i = k; i < m * 16; i += 256) sh[i] = h[(size_t)n0 * 16 + i];
+    for (int i = k; i < m * kHeadTerms; i += 256) st[i] = hs[(size_t)n0 * kHeadTerms + i];
+    __syncthreads();
+    if (k > 50) continue;
+    for (int n = 0; n < m; n++) {
+      const float* t = st + n * kHeadTerms;
+      const float d1 = t[1], d0 = -d1;
+      float v;
+      if (k == 0) v = t[0];
+      else if (k == 1) v = d0;
+      else if (k == 2) v = d1;
+      else if (k < 19) v = d0 * sh[n * 16 + (k - 3)];
+      else if (k < 35) v = d1 * sh[n * 16 + (k - 19)];
+      else v = t[2 + (k - 35)];
+      acc = __fadd_rn(acc, v);
+    }
   }
   if (k == 0) loss[0] = __fadd_rn(loss[0], acc);
   else if (k < 3) gb2[k - 1] = __fadd_rn(gb2[k - 1], acc);
   else if (k < 35) gw2[k - 3] = __fadd_rn(gw2[k - 3], acc);
-  else gb1[k - 35] = __fadd_rn(gb1[k - 35], acc);
+  else if (k < 51) gb1[k - 35] = __fadd_rn(gb1[k - 35], acc);
 }
 
 // per-sample batch gather: dataset [n][len] (BF16) rows idx -> [b][len]
@@ -915,7 +968,7 @@ struct hd_classifier_t {
   // per-batch work buffers
   int cap_batch = 0;
   DBuf in[2], col, z, act[2][3], arg[2][3], dz, dcol, dact_a[2], dact_b[2], x, z1, h, dz1,
-      dx, prob, loss, labels, idx, hs;
+      dx, prob, loss, labels, idx, hs, bias_part;
   DBuf tc_ws, tc_err;               // tensor-core GEMM: split-K workspace, error word
   DBuf data_dm, data_ft, data_lab;  // resident training set
   DBuf stage_dm, stage_ft, sprob;    // scoring: host patches staged in FP32, scores
@@ -970,6 +1023,7 @@ cudaError_t alloc_batch(hd_classifier c, int nb) {
   CK(c->dz1.ensure((size_t)nb * kHid * sizeof(bf16)));
   CK(c->prob.ensure((size_t)nb * sizeof(float)));
   CK(c->hs.ensure((size_t)nb * kHeadTerms * sizeof(float)));
+  CK(c->bias_part.ensure((size_t)2 * (8 + 16 + 32) * kBiasParts * sizeof(float)));
   CK(c->loss.ensure(sizeof(float)));
   CK(c->labels.ensure((size_t)nb * sizeof(int)));
   CK(c->idx.ensure((size_t)nb * sizeof(int)));
@@ -1023,8 +1077,9 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
       const size_t P = (size_t)nb * sp.h * sp.w;
       // z [co][P] = W [co][kp] x col: on the tensor cores as z^T [P][co] =
       // colT [P][kp] x W^T, M = P pixels, N = co, K = kp
-      k_im2col3_t<<<nblk(P * sp.kp()), 256, 0, s>>>(cur, sp.ci, nb, sp.h, sp.w, sp.kp(),
-                                                     c->col.as<bf16>()); hdb::note_launch();
+      const auto im2col = sp.ci == 1 ? k_im2col3_t<1> : sp.ci == 8 ? k_im2col3_t<8>
+                                                                   : k_im2col3_t<16>;
+      im2col<<<nblk(P * sp.kp() / 8), 256, 0, s>>>(cur, sp.h, sp.w, P, c->col.as<bf16>()); hdb::note_launch();
       CK(tc_gemm(c, (int)P, sp.co, sp.kp(), c->col.as<bf16>(), sp.kp(),
                  c->wb_conv[br][l].as<bf16>(), sp.kp(), c->z.as<float>(), 1, (long long)P, 0,
                  1));
@@ -1048,7 +1103,7 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
                                        c->prob.as<float>(), c->dz1.as<bf16>(),
                                        c->hs.as<float>()); hdb::note_launch();
   if (!backward) return cudaGetLastError();
-  k_head_reduce<<<1, 64, 0, s>>>(c->h.as<float>(), c->hs.as<float>(), nb, c->loss.as<float>(),
+  k_head_reduce<<<1, 256, 0, s>>>(c->h.as<float>(), c->hs.as<float>(), nb, c->loss.as<float>(),
                                  g + c->off_w2, g + c->off_b2, g + c->off_b1); hdb::note_launch();
   // ---- backward ----
   {
@@ -1064,28 +1119,33 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
   k_unflatten<<<nblk((size_t)nb * kFeat), 256, 0, s>>>(c->dx.as<float>(), nb,
                                                        c->dact_a[0].as<float>(),
                                                        c->dact_a[1].as<float>()); hdb::note_launch();
+  BiasSum bias{};
+  int chan = 0, layer = 0;
   for (int br = 0; br < 2; br++) {
     float* dcur = c->dact_a[br].as<float>();   // gradient of this layer's pooled output
     float* dnext = c->dact_b[br].as<float>();  // gradient of its input
     for (int l = 2; l >= 0; l--) {
       const ConvSpec& sp = kConv[br][l];
       const size_t P = (size_t)nb * sp.h * sp.w;
-      k_pool_relu_back<<<nblk(P * sp.co), 256, 0, s>>>(
-          dcur, c->act[br][l].as<bf16>(), c->arg[br][l].as<unsigned char>(), sp.co, nb, sp.h,
-          sp.w, c->dz.as<bf16>(), g + c->off_b[br][l]); hdb::note_launch();
-      k_bias_grad<<<sp.co, 256, 0, s>>>(dcur, c->act[br][l].as<bf16>(),
-                                        c->arg[br][l].as<unsigned char>(), nb, sp.h, sp.w,
-                                        g + c->off_b[br][l]); hdb::note_launch();
+      const int parts = (int)std::min<size_t>(kBiasParts, nblk(P / 16));
+      k_pool_relu_back<<<dim3(parts, sp.co), 256, 0, s>>>(
+          dcur, c->act[br][l].as<bf16>(), c->arg[br][l].as<unsigned char>(), nb, sp.h, sp.w,
+          c->dz.as<bf16>(), c->bias_part.as<float>() + chan * kBiasParts); hdb::note_launch();
+      bias.first[layer] = chan;
+      bias.parts[layer] = parts;
+      bias.out[layer] = g + c->off_b[br][l];
+      chan += sp.co;
+      layer++;
       // the layer's input again, as im2col (recomputed rather than stored)
       const bf16* lin = l == 0 ? c->in[br].as<bf16>() : c->act[br][l - 1].as<bf16>();
-      k_im2col3<<<nblk(P * sp.kp()), 256, 0, s>>>(lin, sp.ci, nb, sp.h, sp.w, sp.kp(),
-                                                   c->col.as<bf16>()); hdb::note_launch();
+      k_im2col3<<<dim3(nblk(P / 8), sp.ci), 256, 0, s>>>(lin, sp.h, sp.w, P,
+                                                         c->col.as<bf16>()); hdb::note_launch();
       // dW [co][kw] += dz [co][P] x col^T; the padded columns kw..kp are dropped
       // by writing into a [co][kp] scratch is avoided: N = kw with row stride kw
       // on the tensor cores as dW^T [kw][co] += col [kw][P] x dz^T: M = kw
       // taps, N = co, K = P pixels split over the SMs; the splits are added
       // in order (the same gradient every run)
-      const int splits = (int)std::min<size_t>(296, (P + 8191) / 8192);
+      const int splits = (int)std::min<size_t>(296, (P + 1023) / 1024);
       CK(tc_gemm(c, sp.kw(), sp.co, (int)P, c->col.as<bf16>(), (long long)P, c->dz.as<bf16>(),
                  (long long)P, g + c->off_w[br][l], 1, sp.kw(), 1, splits));
       if (l > 0) {
@@ -1099,6 +1159,8 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
       }
     }
   }
+  bias.first[layer] = chan;
+  k_bias_sum<<<chan, 32, 0, s>>>(c->bias_part.as<float>(), bias); hdb::note_launch();
   return cudaGetLastError();
 }
 

@@ -12,7 +12,9 @@
 // 16-byte core-matrix slices in order, which is the K-major no-swizzle layout
 // tcgen05 reads (stride between 8-row groups SBO = 128 B, between the two
 // K halves of an MMA LBO = rows x 16 B).  Rows and K past the matrix are
-// zero-filled by TMA.
+// zero-filled by TMA.  With fewer than 128 rows A's box has only those (the
+// accumulator rows past them are computed from what the stage held and never
+// read: an MMA's rows do not mix).
 //
 // Warps 0-3: epilogue (each reads its 32 TMEM lanes with tcgen05.ld and
 // stores its rows); warp 4: TMA producer (one thread); warp 5: allocates the
@@ -23,8 +25,8 @@
 // bounded) and frees its TMEM before returning.
 //
 // Split-K (K ranges per tile column of the grid): each split writes its
-// partial tile to a workspace and k_umma_reduce adds the splits in order, so
-// the result does not depend on scheduling.
+// partial tile to a workspace and k_umma_reduce (k_umma_reduce_wide) adds the
+// splits in a fixed order, so the result does not depend on scheduling.
 #include <algorithm>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -44,6 +46,7 @@ constexpr uint32_t UM_WAIT = 1u << 24;
 
 struct UmmaArgs {
   int M, N, K, Npad;
+  int arows;            // rows of A's copy box (128, or M rounded up to 8 if that is less)
   int mtiles, splits;   // tiles = mtiles x splits
   int kblocks;          // K blocks of one split (the last split may have fewer)
   int kblocks_total;
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
           // the K chunks of 8 that the block's MMAs (K = 16 each) read; a
           // chunk past K is zero-filled by TMA
           const int nch = 2 * min(4, (g.K - kk + 15) / 16);
-          mbar_expect_tx(&full[s], (uint32_t)nch * (a_chunk + b_chunk));
+          mbar_expect_tx(&full[s], (uint32_t)nch * ((uint32_t)g.arows * 16 + b_chunk));
           uint8_t* st = base + (size_t)s * stage_bytes;
           for (int c = 0; c < nch; c++) {
             tma_load_2d(st + c * a_chunk, &map_a, kk + 8 * c, mt * UM_BM, &full[s]);
@@ -277,6 +280,29 @@ __global__ void k_umma_reduce(const float* __restrict__ ws, int splits, int M, i
   *c = accumulate ? __fadd_rn(*c, v) : v;
 }
 
+// The same with a warp per output: lane s adds splits s, s + 32, ... and a
+// fixed tree adds the lanes.  For many splits of a small output (a weight
+// gradient), where one thread's chain of loads is what takes time: 296 splits
+// of 9 x 8 outputs 7 us against 22.
+__global__ void __launch_bounds__(256) k_umma_reduce_wide(const float* __restrict__ ws,
+                                                          int splits, int M, int N, int Npad,
+                                                          float* __restrict__ C, long long scm,
+                                                          long long scn, int accumulate) {
+  const int i = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  if (i >= M * N) return;
+  const int m = i / N, n = i % N;
+  const float* w = ws + (size_t)m * Npad + n;
+  float v = 0.f;
+#pragma unroll 4
+  for (int s = lane; s < splits; s += 32) v = __fadd_rn(v, w[(size_t)s * M * Npad]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (lane == 0) {
+    float* c = C + (long long)m * scm + (long long)n * scn;
+    *c = accumulate ? __fadd_rn(*c, v) : v;
+  }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static std::once_flag once;
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -331,13 +357,15 @@ cudaError_t umma_gemm(int M, int N, int K, const void* A, long long lda, const v
   splits = (kblocks_total + kb - 1) / kb;
   if (splits > 1 && !ws) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
-  if (!make_map(&ma, A, M, K, lda, UM_BM) || !make_map(&mb, B, N, K, ldb, Npad))
+  const int arows = std::min(UM_BM, (M + 7) / 8 * 8);
+  if (!make_map(&ma, A, M, K, lda, arows) || !make_map(&mb, B, N, K, ldb, Npad))
     return cudaErrorNotSupported;
   UmmaArgs g{};
   g.M = M;
   g.N = N;
   g.K = K;
   g.Npad = Npad;
+  g.arows = arows;
   g.mtiles = (M + UM_BM - 1) / UM_BM;
   g.splits = splits;
   g.kblocks = kb;
@@ -362,8 +390,13 @@ cudaError_t umma_gemm(int M, int N, int K, const void* A, long long lda, const v
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (splits > 1) {
     const size_t n = (size_t)M * N;
-    k_umma_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ws, splits, M, N, Npad, C, scm,
-                                                               scn, accumulate);
+    // from 64 splits on a warp's 32 loads at a time win
+    if (splits >= 64 && n <= 65536)
+      k_umma_reduce_wide<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(ws, splits, M, N, Npad, C, scm,
+                                                                 scn, accumulate);
+    else
+      k_umma_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ws, splits, M, N, Npad, C, scm,
+                                                                 scn, accumulate);
     note_launch();
     e = cudaGetLastError();
   }
