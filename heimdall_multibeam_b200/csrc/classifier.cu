@@ -856,15 +856,20 @@ __device__ float warp_kth(const float* v, int lo, int hi, int k) {
 // arithmetic there (a division by zero: NaN or +-inf).
 template <bool ZERO_FLAT>
 __global__ void k_normalise_rows_t(float* __restrict__ data, int n, size_t nrows, size_t pitch,
-                                   int rows_per_group, size_t group_pitch) {
+                                   int rows_per_group, size_t group_pitch,
+                                   const size_t* __restrict__ at, size_t nlist,
+                                   size_t rest) {
   extern __shared__ float nr_smem[];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + wib;
   float* v = nr_smem + (size_t)wib * 2 * n;  // [n] values, [n] scratch
   float* a = v + n;
   if (row >= nrows) return;  // whole warp
-  // rows come in groups (e.g. the trials of one candidate's plot)
-  float* x = data + (row / rows_per_group) * group_pitch + (row % rows_per_group) * pitch;
+  // nlist rows at listed offsets, then, from `rest` on, rows in groups (e.g.
+  // the trials of one candidate's plot)
+  const size_t g = row < nlist ? 0 : row - nlist;
+  float* x = data + (row < nlist ? at[row] : rest + (g / rows_per_group) * group_pitch +
+                                                 (g % rows_per_group) * pitch);
   for (int j = lane; j < n; j += 32) v[j] = x[j];
   __syncwarp();
   const float m1 = warp_kth(v, 0, n / 2, n / 4);
@@ -885,26 +890,32 @@ __global__ void k_normalise_rows_t(float* __restrict__ data, int n, size_t nrows
     x[j] = (!ZERO_FLAT || stddev > 0.f) ? __fmul_rn(v[j], val) : 0.f;
 }
 
-cudaError_t normalise_rows(float* data, int n, size_t nrows, size_t pitch, int rows_per_group,
-                           size_t group_pitch, bool zero_flat, cudaStream_t s) {
+static cudaError_t launch_normalise(float* data, int n, size_t nrows, size_t pitch,
+                                    int rows_per_group, size_t group_pitch, bool zero_flat,
+                                    const size_t* at, size_t nlist, size_t rest, cudaStream_t s) {
   if (n < 2 || nrows == 0) return cudaSuccess;
   const size_t smem = 2 * (size_t)n * sizeof(float);
   // rows of up to 1024 values: four warps per block; longer: one
   const int wpb = n <= 1024 ? 4 : 1;
   if (smem * wpb > 200 * 1024) return cudaErrorInvalidValue;
-  const void* fn = zero_flat ? reinterpret_cast<const void*>(k_normalise_rows_t<true>)
-                             : reinterpret_cast<const void*>(k_normalise_rows_t<false>);
-  cudaError_t e = raise_smem_limit(fn, smem * wpb);
+  auto kern = zero_flat ? k_normalise_rows_t<true> : k_normalise_rows_t<false>;
+  cudaError_t e = raise_smem_limit(kern, smem * wpb);
   if (e != cudaSuccess) return e;
-  const unsigned nb = (unsigned)((nrows + wpb - 1) / wpb);
-  if (zero_flat)
-    k_normalise_rows_t<true><<<nb, 32 * wpb, smem * wpb, s>>>(data, n, nrows, pitch,
-                                                             rows_per_group, group_pitch);
-  else
-    k_normalise_rows_t<false><<<nb, 32 * wpb, smem * wpb, s>>>(data, n, nrows, pitch,
-                                                              rows_per_group, group_pitch);
+  kern<<<(unsigned)((nrows + wpb - 1) / wpb), 32 * wpb, smem * wpb, s>>>(
+      data, n, nrows, pitch, rows_per_group, group_pitch, at, nlist, rest);
   note_launch();
   return cudaGetLastError();
+}
+
+cudaError_t normalise_rows(float* data, int n, size_t nrows, size_t pitch, int rows_per_group,
+                           size_t group_pitch, bool zero_flat, cudaStream_t s) {
+  return launch_normalise(data, n, nrows, pitch, rows_per_group, group_pitch, zero_flat, nullptr,
+                          0, 0, s);
+}
+
+cudaError_t normalise_row_list(float* data, int n, const size_t* at, size_t nlist, size_t rest,
+                               size_t nrest, cudaStream_t s) {
+  return launch_normalise(data, n, nlist + nrest, 0, 1, (size_t)n, false, at, nlist, rest, s);
 }
 
 cudaError_t extract_patches(const float* scan, size_t scan_pitch, size_t len, const uint8_t* tf,

@@ -10,12 +10,21 @@ struct hd_pipeline_t;
 
 namespace hdb {
 
-// cudaMalloc that, when it fails, also clears the failure from the runtime's
-// last-error state (an allocation failure is not sticky; left there, it would
-// be reported by the next launch check of an unrelated call).
+// Gives the idle workspaces that calls left for later ones back to the device.
+void trim_pools();
+
+// cudaMalloc that, when it fails, tries once more without the idle workspaces
+// and otherwise clears the failure from the runtime's last-error state (an
+// allocation failure is not sticky; left there, it would be reported by the
+// next launch check of an unrelated call).
 template <class T>
 inline cudaError_t dev_malloc(T** p, size_t bytes) {
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pools();
+    e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  }
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
@@ -383,6 +392,11 @@ cudaError_t umma_gemm(int M, int N, int K, const void* A, long long lda, const v
 // (else the reference's division by zero is kept).
 cudaError_t normalise_rows(float* data, int n, size_t nrows, size_t pitch, int rows_per_group,
                            size_t group_pitch, bool zero_flat, cudaStream_t s);
+// The same, the reference's division by zero kept, on nlist rows at data +
+// at[r] (device offsets) and nrest rows lying one after another from data +
+// rest on.
+cudaError_t normalise_row_list(float* data, int n, const size_t* at, size_t nlist, size_t rest,
+                               size_t nrest, cudaStream_t s);
 // 256 entries of x / 255 * 255 in float (the profiler's sample scaling)
 __device__ __forceinline__ float prof_scale(unsigned x) {
   return __fmul_rn(__fdiv_rn((float)x, 255.f), 255.f);
