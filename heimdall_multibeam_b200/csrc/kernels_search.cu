@@ -479,7 +479,7 @@ size_t scan_smem_bytes(int ser, int nbeams, int ch) {
 // spread over more samples and each producer lane has CH / 128 independent
 // float4 values in flight.
 template <int CH>
-__global__ void __launch_bounds__(256, CH >= 512 ? 3 : 4) k_normalise_scan(
+__global__ void __launch_bounds__(CH >= 512 ? 160 : 256, CH >= 512 ? 3 : 4) k_normalise_scan(
     const float* __restrict__ data, size_t pitch, int nser, unsigned len, unsigned stride,
     int nbeams, const float* __restrict__ rms, float* __restrict__ scan, size_t scan_pitch,
     float* norm_out, int ser_per_block, unsigned* err) {
@@ -542,15 +542,47 @@ __global__ void __launch_bounds__(256, CH >= 512 ? 3 : 4) k_normalise_scan(
       // ---- the chains: stage k - 1 ----
       if (k >= 1 && k - 1 < nstage && lane < nb) {
         float* row = rows + ((size_t)((k - 1) % SC_NB) * S + lane) * ROW;
-#pragma unroll 8
-        for (int e = 0; e < CH; e += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(row + e);
-          float4 o;
-          o.x = sum; sum = __fadd_rn(sum, v.x);
-          o.y = sum; sum = __fadd_rn(sum, v.y);
-          o.z = sum; sum = __fadd_rn(sum, v.z);
-          o.w = sum; sum = __fadd_rn(sum, v.w);
-          *reinterpret_cast<float4*>(row + e) = o;
+        if constexpr (CH >= 512) {
+          // blocks of few series: the next 32 samples are loaded before the
+          // current ones are added, so the chain waits for its adds only (one
+          // series of 262144 samples: 0.67 ms against 0.75).  Takes 112
+          // registers, which the blocks of 8 series (CH = 256) don't have:
+          // there it spills and the headline gulp's scan slows from 0.50 to
+          // 0.73 ms.
+          constexpr int AH = 8;
+          float4 cur[AH], nxt[AH];
+#pragma unroll
+          for (int j = 0; j < AH; j++) cur[j] = *reinterpret_cast<const float4*>(row + 4 * j);
+#pragma unroll 2
+          for (int e = 0; e < CH; e += 4 * AH) {
+            // past the row's end the last values again (never added)
+            const float* ahead = row + min(e + 4 * AH, CH - 4 * AH);
+#pragma unroll
+            for (int j = 0; j < AH; j++) nxt[j] = *reinterpret_cast<const float4*>(ahead + 4 * j);
+#pragma unroll
+            for (int j = 0; j < AH; j++) {
+              const float4 v = cur[j];
+              float4 o;
+              o.x = sum; sum = __fadd_rn(sum, v.x);
+              o.y = sum; sum = __fadd_rn(sum, v.y);
+              o.z = sum; sum = __fadd_rn(sum, v.z);
+              o.w = sum; sum = __fadd_rn(sum, v.w);
+              *reinterpret_cast<float4*>(row + e + 4 * j) = o;
+            }
+#pragma unroll
+            for (int j = 0; j < AH; j++) cur[j] = nxt[j];
+          }
+        } else {
+  #pragma unroll 8
+          for (int e = 0; e < CH; e += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(row + e);
+            float4 o;
+            o.x = sum; sum = __fadd_rn(sum, v.x);
+            o.y = sum; sum = __fadd_rn(sum, v.y);
+            o.z = sum; sum = __fadd_rn(sum, v.z);
+            o.w = sum; sum = __fadd_rn(sum, v.w);
+            *reinterpret_cast<float4*>(row + e) = o;
+          }
         }
       }
     } else {
@@ -663,7 +695,7 @@ template <int CH>
 static cudaError_t launch_scan(const SeriesBatch& sb, const float* rms, float* scan,
                                size_t scan_pitch, float* norm_out, cudaStream_t s, unsigned* err,
                                int ser) {
-  const int np = ser < 7 ? ser : 7;
+  const int np = ser < 7 ? ser : 7;  // 4 at most with 512-sample stages
   const size_t smem = scan_smem_bytes(ser, sb.nbeams, CH);
   cudaError_t e = raise_smem_limit(k_normalise_scan<CH>, smem);
   if (e != cudaSuccess) return e;

@@ -117,8 +117,7 @@ struct hd_pipeline_t {
   DevBuf root_flag, root_off, mkey, rows, unit_off;
   DevBuf h_small_dev;
 
-  // Gulps captured as CUDA graphs (hd_execute_beams with device input and
-  // hd_execute_prefetched).  The first gulp of a shape runs on the
+  // Gulps captured as CUDA graphs.  The first gulp of a shape runs on the
   // host-sized path and fixes the shape's hit and giant capacities and its
   // number of clustering sweep pairs; later gulps of the shape replay one
   // graph per set of device buffers.
@@ -176,6 +175,34 @@ struct hd_pipeline_t {
   // merged candidate rows read back (pinned)
   hdb::GroupRow* h_rows = nullptr;
   size_t h_rows_cap = 0;
+  // the widths in `winfo`: a gulp of the same widths uploads nothing
+  std::vector<hdb::WidthInfo> winfo_now;
+  const void* winfo_at = nullptr;
+  cudaError_t upload_widths(const std::vector<hdb::WidthInfo>& wi, cudaStream_t s) {
+    if (winfo_at == winfo.p && winfo_now.size() == wi.size() &&
+        std::memcmp(winfo_now.data(), wi.data(), wi.size() * sizeof(hdb::WidthInfo)) == 0)
+      return cudaSuccess;
+    winfo_at = nullptr;
+    const cudaError_t e = cudaMemcpyAsync(winfo.p, wi.data(), wi.size() * sizeof(hdb::WidthInfo),
+                                          cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    winfo_now = wi;
+    winfo_at = winfo.p;
+    return cudaSuccess;
+  }
+  unsigned* h_first = nullptr;  // pinned: first giant of each unit
+  size_t h_first_cap = 0;
+  cudaError_t ensure_first_host(size_t n) {
+    if (n <= h_first_cap) return cudaSuccess;
+    if (h_first) cudaFreeHost(h_first);
+    h_first = nullptr;
+    h_first_cap = 0;
+    const size_t want = std::max<size_t>(n, 256);
+    const cudaError_t e = cudaMallocHost(&h_first, want * sizeof(unsigned));
+    if (e == cudaSuccess) h_first_cap = want;
+    else cudaGetLastError();
+    return e;
+  }
   cudaError_t ensure_rows_host(size_t n) {
     if (n <= h_rows_cap) return cudaSuccess;
     if (h_rows) cudaFreeHost(h_rows);
@@ -198,6 +225,7 @@ struct hd_pipeline_t {
     if (copy_stream) cudaStreamDestroy(copy_stream);
     if (h_small) cudaFreeHost(h_small);
     if (h_rows) cudaFreeHost(h_rows);
+    if (h_first) cudaFreeHost(h_first);
   }
 };
 
@@ -552,21 +580,22 @@ static void emit_candidates(hd_pipeline pl, size_t U, const hdb::GroupRow* rows,
 }
 
 // ---- the gulp as a CUDA graph -------------------------------------------------
-// Capture-safe enqueue of one gulp of U device-resident 8-bit filterbanks at
-// native resolution: no host synchronisation, no allocation (every buffer was
-// sized by graph_gulp), hits and giants at the shape's capacities, clustering
-// as `pairs` sweep pairs that stop themselves at the fixed point.
+// Capture-safe enqueue of one gulp of U filterbanks of 1, 2, 4 or 8-bit samples
+// that lie in pl->fb_tf, at native resolution: no host synchronisation, no
+// allocation (every buffer was sized by graph_gulp), hits and giants at the
+// shape's capacities, clustering as `pairs` sweep pairs that stop themselves
+// at the fixed point.
 struct GulpGeom {
-  size_t U, nsamps, nbeams, C, D, max_delay, dm_tol, gap, nc, fb_bytes, pitch, ft_unit,
+  size_t U, nsamps, nbits, nbeams, C, D, max_delay, dm_tol, gap, nc, fb_bytes, pitch, ft_unit,
       dd_pitch, NS, stride, bcount, scan_pitch, nsmooth, nsw, gcap_groups;
   unsigned ntiles;
 };
 
 // With `events`, the stage boundaries of hd_get_timing are recorded by event
 // nodes of the graph (the events of the host-sized path, at the same points).
-static hd_error enqueue_gulp(hd_pipeline pl, const hd_byte* const* fbs, bool resident,
-                             const GulpGeom& g, const std::vector<hdb::WidthInfo>& wi,
-                             unsigned hcap, unsigned gcap, unsigned pairs, bool events) {
+static hd_error enqueue_gulp(hd_pipeline pl, const GulpGeom& g,
+                             const std::vector<hdb::WidthInfo>& wi, unsigned hcap, unsigned gcap,
+                             unsigned pairs, bool events) {
   const hd_params& P = pl->params;
   dedisp_plan plan = pl->plan;
   cudaStream_t s = pl->stream;
@@ -575,9 +604,6 @@ static hd_error enqueue_gulp(hd_pipeline pl, const hd_byte* const* fbs, bool res
                   : cudaSuccess;
   };
   HD_TRY(cudaMemsetAsync(plan->d_err, 0, sizeof(unsigned), s));
-  if (!resident)
-    HD_TRY(copy_units(pl->fb_tf.as<uint8_t>(), fbs, 0, g.U, g.fb_bytes, cudaMemcpyDeviceToDevice,
-                      s));
   HD_TRY(mark(1));
   if (pl->cleaning) {
     hd_error he = clean_units(pl, g.U, pl->fb_tf.as<uint8_t>(), g.nsamps, g.C, P.dt,
@@ -585,7 +611,7 @@ static hd_error enqueue_gulp(hd_pipeline pl, const hd_byte* const* fbs, bool res
                               pl->fb_ft.as<uint8_t>(), g.pitch, nullptr);
     if (he != HD_NO_ERROR) return he;
   } else {
-    HD_TRY(hdb::input_to_ft(pl->fb_tf.as<uint8_t>(), g.nsamps, (int)g.C, 8,
+    HD_TRY(hdb::input_to_ft(pl->fb_tf.as<uint8_t>(), g.nsamps, (int)g.C, (int)g.nbits,
                             pl->fb_ft.as<uint8_t>(), g.pitch, s, g.U, g.ft_unit));
   }
   HD_TRY(mark(2));
@@ -678,14 +704,19 @@ static unsigned graph_capacity(unsigned n, unsigned floor) {
 // clustering needed more sweeps than were captured (the capacities grow for
 // the next gulp of the shape, and no clamped result is reported).  Returns
 // true with *result set when the graph's results stand or a CUDA call failed.
+//
+// The input is copied into the pipeline's own buffer before the replay, so a
+// graph holds no caller's address: gulps in new buffers replay as gulps in the
+// old ones do.
 static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool resident,
-                       size_t nsamps, size_t nbeams, size_t first_idx, const hd_size* beams,
+                       cudaMemcpyKind kind, size_t nsamps, size_t nbits, size_t nbeams, size_t first_idx, const hd_size* beams,
                        hd_error* statuses, size_t nsamps_processed, hd_error* result) {
   const hd_params& P = pl->params;
   dedisp_plan plan = pl->plan;
   GulpGeom g{};
   g.U = U;
   g.nsamps = nsamps;
+  g.nbits = nbits;
   g.nbeams = nbeams;
   g.C = P.nchans;
   g.D = plan->dm_list.size();
@@ -695,7 +726,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   if (g.max_delay >= g.stride || g.max_delay + Bmax > g.stride) return false;
   bool withhold = false;
   if (const char* e = std::getenv("HDB_TEST_WITHHOLD_STAGE")) withhold = e[0] == '1';
-  const std::vector<size_t> shape = {U, nsamps, nbeams, g.C, g.D, g.max_delay,
+  const std::vector<size_t> shape = {U, nsamps, nbits, nbeams, g.C, g.D, g.max_delay,
                                      (size_t)pl->cleaning, (size_t)resident,
                                      (size_t)plan->forced_dm_block,
                                      (size_t)plan->forced_time_block, (size_t)plan->tune,
@@ -713,7 +744,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   g.dm_tol = std::min<size_t>(P.cand_sep_dm, g.D);
   g.gap = g.D + g.dm_tol + 2;
   g.nc = nsamps - g.max_delay;
-  g.fb_bytes = nsamps * g.C;
+  g.fb_bytes = nsamps * g.C * nbits / 8;
   g.pitch = hdb::ft_pitch(plan, nsamps);
   g.ft_unit = g.pitch * g.C;
   g.dd_pitch = round_up(g.nc + 1, 4);
@@ -787,7 +818,6 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   key.push_back(hcap);
   key.push_back(gcap);
   key.push_back(pairs);
-  for (size_t u = 0; u < U; u++) key.push_back(resident ? 0 : (size_t)fbs[u]);
   for (const DevBuf* b : {&pl->fb_tf, &pl->fb_ft, &pl->dm0, &pl->dm0_scan, &pl->base, &pl->rms,
                           &pl->mask, &pl->fmask, &pl->rms0, &pl->dd, &pl->scan, &pl->ws_a,
                           &pl->ws_b, &pl->winfo, &pl->norm, &pl->gmax, &pl->tile_list,
@@ -821,7 +851,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
       const unsigned long long l0 = hdb::launch_count();
       ce = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
       if (ce == cudaSuccess) {
-        he = enqueue_gulp(pl, fbs, resident, g, wi, hcap, gcap, pairs, events != 0);
+        he = enqueue_gulp(pl, g, wi, hcap, gcap, pairs, events != 0);
         cudaGraph_t graph = nullptr;
         ce = cudaStreamEndCapture(s, &graph);
         if (he == HD_NO_ERROR && ce == cudaSuccess && graph)
@@ -864,28 +894,30 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   } while (0)
   // the width table is the pipeline's (another shape's gulp may have
   // replaced it since the capture)
-  GG_TRY(cudaMemcpyAsync(pl->winfo.p, wi.data(), nw * sizeof(hdb::WidthInfo),
-                         cudaMemcpyHostToDevice, s));
+  GG_TRY(pl->upload_widths(wi, s));
   cudaEventRecord(pl->ev[0], s);
+  if (!resident) GG_TRY(copy_units(pl->fb_tf.as<uint8_t>(), fbs, 0, U, g.fb_bytes, kind, s));
   GG_TRY(cudaGraphLaunch(gg->exec, s));
   hdb::add_launches(gg->launches);
-  std::vector<unsigned>& first = pl->unit_first;
-  first.assign(U + 1, 0);
+  GG_TRY(pl->ensure_first_host(U + 1));
   GG_TRY(cudaMemcpyAsync(pl->h_small, pl->small.p, 64 * sizeof(unsigned), cudaMemcpyDeviceToHost,
                          s));
   GG_TRY(cudaMemcpyAsync(pl->h_small + 20, plan->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
                          s));
-  GG_TRY(cudaMemcpyAsync(first.data(), pl->unit_off.p, (U + 1) * sizeof(unsigned),
+  GG_TRY(cudaMemcpyAsync(pl->h_first, pl->unit_off.p, (U + 1) * sizeof(unsigned),
                          cudaMemcpyDeviceToHost, s));
   GG_TRY(cudaMemcpyAsync(pl->h_rows, pl->rows.p, spec * sizeof(hdb::GroupRow),
                          cudaMemcpyDeviceToHost, s));
   cudaEventRecord(pl->ev[7], s);
   GG_TRY(cudaStreamSynchronize(s));
+  std::vector<unsigned>& first = pl->unit_first;
+  first.assign(pl->h_first, pl->h_first + U + 1);
   const unsigned nh = pl->h_small[0], ngi = pl->h_small[1];
   if (nh > hcap || ngi > gcap) {
     gs->hcap = std::max(hcap, graph_capacity(nh, hcap));
     gs->gcap = std::max(gcap, graph_capacity(ngi, gcap));
     pl->drop_graphs(shape);
+    first.assign(U + 1, 0);
     return false;
   }
   int conv = -1;
@@ -895,6 +927,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
     gs->pairs = std::min(pairs + 2, 16u);
     if (gs->pairs == pairs) gs->broken = true;
     pl->drop_graphs(shape);
+    first.assign(U + 1, 0);
     return false;
   }
   if (pl->h_small[20]) {
@@ -1012,14 +1045,16 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
   *nsamps_processed = nsamps - nbeams * (P.boxcar_max + max_delay);
   if (nsamps < nbeams * (P.boxcar_max + max_delay)) *nsamps_processed = 0;
 
-  // the batched forms with device-resident input: a shape seen before runs as
-  // one CUDA graph replay
+  // a shape seen before runs as one CUDA graph replay, except several
+  // filterbanks in host memory whose copies overlap their transpose and
+  // dedispersion below
+  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   pl->last_graph = false;
   pl->pending_shape.clear();
-  if (graph && on_device && nbits == 8 && pl->use_graphs && pl->plan->groups.empty() &&
-      !pl->narrow_band) {
+  if (graph && (on_device || U == 1 || pl->cleaning) && nbits <= 8 && pl->use_graphs &&
+      pl->plan->groups.empty() && !pl->narrow_band) {
     hd_error ge = HD_NO_ERROR;
-    if (graph_gulp(pl, fbs, U, resident, nsamps, nbeams, first_idx, beams, statuses,
+    if (graph_gulp(pl, fbs, U, resident, kind, nsamps, nbits, nbeams, first_idx, beams, statuses,
                    *nsamps_processed, &ge))
       return ge;
   }
@@ -1037,7 +1072,6 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
   HD_TRY(pl->fb_ft.ensure(U * ft_unit * (nbits == 16 ? 2 : 1)));
   HD_TRY(pl->dd.ensure(NS * dd_pitch * sizeof(float)));
   float* dd = pl->dd.as<float>();
-  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   if (!on_device && !pl->cleaning && U > 1 && pl->plan->groups.empty() && nbits == 8) {
     // pipelined: copy chunk k on the copy stream while chunk k - 1 is
     // transposed and dedispersed on the compute stream (the unit-major series
@@ -1185,8 +1219,7 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
     const int nw = (int)wi.size();
     if (nw == 0) continue;  // the trials' factor exceeds the widest boxcar
     HD_TRY(pl->winfo.ensure(nw * sizeof(hdb::WidthInfo)));
-    HD_TRY(cudaMemcpyAsync(pl->winfo.p, wi.data(), nw * sizeof(hdb::WidthInfo),
-                           cudaMemcpyHostToDevice, s));
+    HD_TRY(pl->upload_widths(wi, s));
     HD_TRY(pl->norm.ensure(NSg * nw * sizeof(float)));
     wctx.scan = scan_g;
     wctx.scan_pitch = scan_pitch;
@@ -1472,7 +1505,7 @@ hd_error hd_execute(hd_pipeline pl, const hd_byte* h_filterbank, hd_size nsamps,
                     hd_size first_idx, hd_size nbeams, hd_size* nsamps_processed) {
   if (!h_filterbank) return pl ? HD_INVALID_POINTER : HD_INVALID_PIPELINE;
   return execute_units(pl, &h_filterbank, 1, false, nsamps, nbits, first_idx, nbeams, nullptr,
-                       nullptr, nsamps_processed);
+                       nullptr, nsamps_processed, true);
 }
 
 hd_error hd_execute_device(hd_pipeline pl, const hd_byte* d_filterbank, hd_size nsamps,
@@ -1480,7 +1513,7 @@ hd_error hd_execute_device(hd_pipeline pl, const hd_byte* d_filterbank, hd_size 
                            hd_size* nsamps_processed) {
   if (!d_filterbank) return pl ? HD_INVALID_POINTER : HD_INVALID_PIPELINE;
   return execute_units(pl, &d_filterbank, 1, true, nsamps, nbits, first_idx, nbeams, nullptr,
-                       nullptr, nsamps_processed);
+                       nullptr, nsamps_processed, true);
 }
 
 hd_error hd_execute_beams(hd_pipeline pl, const hd_byte* const* filterbanks,

@@ -417,21 +417,23 @@ int hd_get_dedisp_tile_source(hd_pipeline pipeline);
  * graph's kernels counted at each replay). */
 unsigned long long hd_get_launch_count(void);
 
-/* The batched calls with device-resident input (hd_execute_beams with
- * on_device != 0, hd_execute_prefetched) run each gulp as one CUDA graph
- * replay once its shape (filterbank count, spectra, beams, cleaning, DM
- * trials) has been searched once: the first gulp of a shape runs on the
- * host-sized path and fixes the shape's hit and giant capacities and its
- * number of clustering sweeps; later gulps of the shape launch one captured
- * graph (one per set of input buffers) with every total kept on the device,
- * and the host reads the results once.  A gulp whose totals exceed the
- * capacities, or whose clustering needs more sweeps, is searched again on
- * the host-sized path and the shape's capacities grow: results never depend
- * on the form.  Adaptive dt, narrow-band zapping and input other than 8-bit
- * stay on the host-sized path.  hd_set_graphs(p, 0) turns the graph form off
- * (the environment variable HDB_NO_GRAPH=1 does so for new pipelines);
- * hd_get_graph_replays counts the gulps it served.  No reference
- * counterpart (the reference synchronises after every stage). */
+/* hd_execute, hd_execute_device, hd_execute_prefetched and hd_execute_beams
+ * (with on_device != 0, one filterbank, or cleaning on) run each gulp as one
+ * CUDA graph replay once its shape (filterbank count, spectra, sample width,
+ * beams, cleaning, DM trials) has been searched once: the first gulp of a
+ * shape runs on the host-sized path and fixes the shape's hit and giant
+ * capacities and its number of clustering sweeps; later gulps of the shape
+ * copy their input into the pipeline's buffer, wherever it comes from, and
+ * launch one captured graph with every total kept on the device, and the host
+ * reads the results once.  A gulp whose totals exceed the capacities, or whose
+ * clustering needs more sweeps, is searched again on the host-sized path and
+ * the shape's capacities grow: results never depend on the form.  Adaptive dt,
+ * narrow-band zapping and 16-bit input stay on the host-sized path, and so do
+ * several filterbanks in host memory without cleaning (their copies overlap
+ * the dedispersion).  hd_set_graphs(p, 0) turns the graph form off (the
+ * environment variable HDB_NO_GRAPH=1 does so for new pipelines);
+ * hd_get_graph_replays counts the gulps it served.  No reference counterpart
+ * (the reference synchronises after every stage). */
 hd_error hd_set_graphs(hd_pipeline pipeline, int enable);
 unsigned long long hd_get_graph_replays(hd_pipeline pipeline);
 
