@@ -219,6 +219,7 @@ struct WidthInfo {
   int scr;            // cur_scrunch: trial scrunch x ts (index rescale)
 };
 
+constexpr int TS_GMAX = 4;  // time-scrunched widths whose group maxima are kept
 struct WidthCtx {
   const float* scan;
   size_t scan_pitch;
@@ -245,6 +246,10 @@ struct WidthCtx {
   size_t gmax_cap;
   unsigned gsize, ngroups;
   int gmax_nw;
+  // the same of the k-th width after those (time-scrunched; one beam): group
+  // maxima [nser][ts_ngroups[k]] from gmax + ts_gmax[k] on (0 groups: none)
+  size_t ts_gmax[TS_GMAX];
+  unsigned ts_ngroups[TS_GMAX], ts_gsize[TS_GMAX];
 };
 
 // Block RMS of width wi for every series (get_rms.cu:274-301 on the filtered
@@ -293,6 +298,9 @@ struct GiantBuffers {
   int* filter;
   int* dm;
   int* label;
+  // clustering's own copies (cluster_init): [giants], [giants / 128 + 1]
+  int4* pack;
+  int* tile_first;
   size_t cap;
 };
 cudaError_t giant_heads(const WidthCtx& ctx, const HitBuffers& hb, unsigned nhits,
@@ -316,7 +324,7 @@ struct ClusterArgs {
   // sizes the sweep grid's chunks of earlier giants (0: ngiants)
   int max_unit_giants;
 };
-cudaError_t cluster_init(GiantBuffers& gb, int ngiants, cudaStream_t s);
+cudaError_t cluster_init(const ClusterArgs& a, GiantBuffers& gb, cudaStream_t s);
 cudaError_t cluster_sweep(const ClusterArgs& a, GiantBuffers& gb, unsigned* changed,
                           cudaStream_t s);
 

@@ -747,18 +747,80 @@ __device__ __forceinline__ float rms_window_value(const float* sc, int offset,
 
 // Pass 1 of the block RMS: level-m medians of |window| over aligned groups of
 // the reblocked index q (get_rms.cu:274-301; reblock_abs_beam with a float
-// delta).  Widths [w0, w0 + gridDim.y) of every series.
-__global__ void k_block_rms_pass1(WidthCtx ctx, int w0, int m, float* __restrict__ out,
-                                  size_t out_pitch) {
+// delta).  Widths [w0, w0 + gridDim.y) of every series.  Most groups lie in
+// one beam, with consecutive window indices and one source (the width's own
+// output, or one earlier width's where it leaves stale values): the index
+// arithmetic and the choice of source are then done once per group instead of
+// once per value (the time-scrunched width of the survey gulp: 333 us against
+// 829).  With gmax ([series][groups], one width), a group of the width's own
+// output leaves its largest |value| there, every other group +inf.
+__global__ void __launch_bounds__(TREE_THREADS) k_block_rms_pass1(WidthCtx ctx, int w0, int m,
+                                                                  float* __restrict__ out,
+                                                                  size_t out_pitch,
+                                                                  float* __restrict__ gmax) {
   __shared__ float sm[625 + 125];
   const int wi = w0 + blockIdx.y;
   const size_t ser = blockIdx.z;
   const size_t g = blockIdx.x;
-  const WidthInfo& w = ctx.winfo[wi];
+  const WidthInfo w = ctx.winfo[wi];
   const float* sc = ctx.scan + ser * ctx.scan_pitch;
   const float* norm = ctx.norm + ser * ctx.nw;
   const float delta = (float)(ctx.stride - w.bn);
   const size_t q0 = g * pow5(m);
+  const size_t q1 = q0 + pow5(m) - 1;
+  const size_t b0 = (unsigned)q0 / w.bn, b1 = (unsigned)q1 / w.bn;
+  const size_t i0 = reblock_index(b0, delta, (unsigned)q0);
+  const size_t i1 = reblock_index(b1, delta, (unsigned)q1);
+  // below 2^24 every float index is exact, so the indices are i0 + k
+  if (b0 == b1 && i1 < (1u << 24) && (i1 < w.n || i0 >= w.n)) {
+    int src = wi;
+    if (i0 >= w.n) {
+      int p0 = w.prev_cover, p1 = w.prev_cover;
+      while (p0 >= 0 && i0 >= ctx.winfo[p0].n) p0 = ctx.winfo[p0].prev_cover;
+      while (p1 >= 0 && i1 >= ctx.winfo[p1].n) p1 = ctx.winfo[p1].prev_cover;
+      src = p0 == p1 ? p0 : -2;
+    }
+    if (src != -2) {
+      float r;
+      if (src < 0) {
+        r = block_tree([&](int) { return 0.f; }, m, sm);
+      } else {
+        const WidthInfo ws = ctx.winfo[src];
+        const unsigned ts = (unsigned)ws.ts;
+        const float* lo = sc + (ctx.offset - ws.behind) + i0 * ts;
+        const float* hi = sc + (ctx.offset + ws.ahead) + i0 * ts;
+        if (src == wi) {
+          float mx = 0.f;
+          r = block_tree([&](int k) {
+            const float v = fabsf(__fsub_rn(hi[(unsigned)k * ts], lo[(unsigned)k * ts]));
+            mx = fmaxf(mx, v);  // a NaN is dropped: it never passes the threshold
+            return v;
+          }, m, sm);
+          if (gmax) {
+            // non-negative floats order as their bits
+            unsigned* top = reinterpret_cast<unsigned*>(sm);
+            if (threadIdx.x == 0) *top = 0u;
+            __syncthreads();
+            const unsigned mk = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+            if ((threadIdx.x & 31) == 0) atomicMax(top, mk);
+            __syncthreads();
+            if (threadIdx.x == 0) gmax[ser * gridDim.x + g] = __uint_as_float(*top);
+          }
+        } else {
+          const float nrm = norm[src];
+          r = block_tree([&](int k) {
+            return fabsf(__fmul_rn(__fsub_rn(hi[(unsigned)k * ts], lo[(unsigned)k * ts]), nrm));
+          }, m, sm);
+        }
+      }
+      if (threadIdx.x == 0) {
+        out[(ser * gridDim.y + blockIdx.y) * out_pitch + g] = r;
+        if (gmax && src != wi) gmax[ser * gridDim.x + g] = INFINITY;
+      }
+      return;
+    }
+  }
+  if (gmax && threadIdx.x == 0) gmax[ser * gridDim.x + g] = INFINITY;
   float r = block_tree([&](int k) {
     unsigned q = (unsigned)(q0 + k);
     size_t beam = q / w.bn;
@@ -1068,7 +1130,10 @@ __global__ void k_block_rms_final(WidthCtx ctx, int w0, int nwb, const float* __
 
 cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end,
                       TreeScratch& ws, cudaStream_t s) {
-  if (w_begin == 0) ctx.ngroups = 0;  // no group maxima unless recorded below
+  if (w_begin == 0) {  // no group maxima unless recorded below
+    ctx.ngroups = 0;
+    for (unsigned& n : ctx.ts_ngroups) n = 0;
+  }
   const int nwb = w_end - w_begin;
   const size_t cnt = (size_t)ctx.nbeams * hw[w_begin].bn;
   for (int wi = w_begin; wi < w_end; wi++)
@@ -1114,8 +1179,9 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
         ctx.ngroups = (unsigned)ng1;
         ctx.gmax_nw = nwb;
       }
-      // about 8 consecutive groups per block, spread evenly
-      const size_t nblk_x = (ng1 + 7) / 8;
+      // about 8 consecutive groups per block, spread evenly; fewer where that
+      // leaves the SMs without two blocks each
+      const size_t nblk_x = std::max((ng1 + 7) / 8, std::min<size_t>(ng1, 296 / ctx.nser + 1));
       const size_t gpb = (ng1 + nblk_x - 1) / nblk_x;
       const unsigned nthreads = 32u * (unsigned)std::min(nwb, BRV_THREADS / 32);
       kern<<<dim3((unsigned)((ng1 + gpb - 1) / gpb), ctx.nser), nthreads, smem, s>>>(
@@ -1138,8 +1204,21 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
     k_block_rms_pass1_multi<<<dim3((unsigned)ng1, ctx.nser), TREE_THREADS, smem, s>>>(
         ctx, w_begin, nwb, m1, (int)win, ws.a, ng1); note_launch();
   } else {
-    k_block_rms_pass1<<<seg_grid(ng1, nwb, ctx.nser), TREE_THREADS, 0, s>>>(ctx, w_begin, m1,
-                                                                           ws.a, ng1); note_launch();
+    // the group maxima of a time-scrunched width, after the unscrunched ones
+    float* gm = nullptr;
+    const int k = w_begin - ctx.gmax_nw;
+    if (ctx.gmax && ctx.ngroups > 0 && ctx.nbeams == 1 && nwb == 1 && k >= 0 && k < TS_GMAX) {
+      size_t at = (size_t)ctx.nser * ctx.gmax_nw * ctx.ngroups;
+      for (int j = 0; j < k; j++) at += (size_t)ctx.nser * ctx.ts_ngroups[j];
+      if (at + (size_t)ctx.nser * ng1 <= ctx.gmax_cap) {
+        gm = ctx.gmax + at;
+        ctx.ts_gmax[k] = at;
+        ctx.ts_ngroups[k] = (unsigned)ng1;
+        ctx.ts_gsize[k] = (unsigned)pow5(m1);
+      }
+    }
+    k_block_rms_pass1<<<seg_grid(ng1, nwb, ctx.nser), TREE_THREADS, 0, s>>>(
+        ctx, w_begin, m1, ws.a, ng1, gm); note_launch();
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   float* fin;
@@ -1168,20 +1247,51 @@ __device__ __forceinline__ bool hit_at(const WidthCtx& ctx, const float* sc, flo
   return v > ctx.thresh;
 }
 
+// Counts of one tile; consecutive threads take consecutive samples (the order
+// does not matter to a count), and each thread finds its sample's place in the
+// beam once and steps it.  A tile whose block-RMS groups' maxima stay below the
+// threshold counts nothing and reads nothing (the survey gulp's time-scrunched
+// width: 180 us; 370 without the maxima, 687 with a 64-bit remainder per
+// sample and 8 strided samples per thread too).
 __global__ void __launch_bounds__(HIT_THREADS) k_count_hits(WidthCtx ctx, HitBuffers hb,
                                                             int w_base) {
   const int wi = w_base + blockIdx.y;
   const size_t ser = blockIdx.z;
   const unsigned tile = blockIdx.x;
-  const WidthInfo& w = ctx.winfo[wi];
-  const float* sc = ctx.scan + ser * ctx.scan_pitch;
+  const WidthInfo w = ctx.winfo[wi];
   const float norm = ctx.norm[ser * ctx.nw + wi];
-  const size_t i0 = (size_t)tile * HIT_TILE + (size_t)threadIdx.x * HIT_PER_THREAD;
+  const unsigned ts = (unsigned)w.ts, stride = (unsigned)ctx.stride;
+  const unsigned i0 = tile * HIT_TILE + threadIdx.x;
+  const float* lo = ctx.scan + ser * ctx.scan_pitch + (ctx.offset - w.behind) + (size_t)i0 * ts;
+  const float* hi = lo + w.behind + w.ahead;
   unsigned c = 0;
-  float v;
-  if (i0 < w.n) {
+  bool need = tile * HIT_TILE < w.n;
+  const int tk = wi - ctx.gmax_nw;
+  if (need && tk >= 0 && tk < TS_GMAX && ctx.ts_ngroups[tk] > 0) {
+    // the groups' window indices are the filtered indices (one beam)
+    const unsigned ng = ctx.ts_ngroups[tk], gs = ctx.ts_gsize[tk];
+    const unsigned g0 = tile * HIT_TILE / gs, g1 = (tile * HIT_TILE + HIT_TILE - 1) / gs;
+    if (g1 < ng) {
+      const float* gm = ctx.gmax + ctx.ts_gmax[tk] + ser * ng;
+      float mx = 0.f;
+      for (unsigned g = g0; g <= g1; g++) mx = fmaxf(mx, gm[g]);
+      // RN(d * norm) is monotone in d for a positive norm
+      need = !(norm > 0.f && __fmul_rn(mx, norm) <= ctx.thresh);
+    }
+  }
+  if (need) {
+    unsigned at = i0 % stride;  // sample within its beam
+    const unsigned step = HIT_THREADS % stride;
 #pragma unroll
-    for (int k = 0; k < HIT_PER_THREAD; k++) c += hit_at(ctx, sc, norm, w, i0 + k, &v);
+    for (int k = 0; k < HIT_PER_THREAD; k++) {
+      const unsigned i = i0 + k * HIT_THREADS;
+      if (i < w.n && at < w.bn) {
+        const size_t p = (size_t)(k * HIT_THREADS) * ts;
+        c += __fmul_rn(__fsub_rn(hi[p], lo[p]), norm) > ctx.thresh;
+      }
+      at += step;
+      if (at >= stride) at -= stride;
+    }
   }
   __shared__ unsigned red[HIT_THREADS / 32];
 #pragma unroll
@@ -1824,8 +1934,10 @@ cudaError_t count_hits(const WidthCtx& ctx, HitBuffers& hb, unsigned ntiles, cud
       if ((e = cudaMemsetAsync(hb.tile_list_n, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
       hb.list_valid = true;
     }
-    // about 8 consecutive tiles per block (at most 8), spread evenly
-    const unsigned nbx = (ntiles + 7) / 8;
+    // about 8 consecutive tiles per block (at most 8), spread evenly; fewer
+    // where that leaves the SMs without two blocks each (55 series of 4 tiles:
+    // 11 us with a tile per block against 19 with four)
+    const unsigned nbx = std::max((ntiles + 7) / 8, std::min(ntiles, 296u / (unsigned)ctx.nser + 1));
     const unsigned tpb = (ntiles + nbx - 1) / nbx;
     k_count_hits_vec<<<dim3((ntiles + tpb - 1) / tpb, ctx.nser), HIT_THREADS,
                        2 * span4 * sizeof(float), s>>>(ctx, hb, nw1, slen, span4, (int)tpb); note_launch();
@@ -1871,7 +1983,10 @@ cudaError_t write_hits(const WidthCtx& ctx, HitBuffers& hb, cudaStream_t s) {
     nw1 = 0;
   }
   if (nw1 < ctx.nw) {
-    k_write_hits<<<dim3(hb.ntiles, ctx.nw - nw1, ctx.nser), HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
+    unsigned n = 1;  // tiles past every such width's samples hold nothing
+    for (int w = nw1; w < ctx.nw; w++) n = std::max(n, ctx.host_winfo[w].n);
+    k_write_hits<<<dim3(std::min(hb.ntiles, (n + HIT_TILE - 1) / HIT_TILE), ctx.nw - nw1,
+                        ctx.nser), HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
   }
   return cudaGetLastError();
 }
@@ -2113,9 +2228,36 @@ cudaError_t giant_fill(const WidthCtx& ctx, const HitBuffers& hb, unsigned nhits
 constexpr int CL_TILE = 128;
 constexpr int CL_YBLOCKS = 8;  // chunks of earlier giants per window, about
 
-__global__ void k_cluster_init(int* label, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) label[i] = i;
+// What a sweep compares, once per giant: {sample, time tolerance of its
+// boxcar, beam, DM key} and its filter (are_coincident_beam,
+// are_coincident.cuh:47-68; sample indices fit 31 bits, checked by the host),
+// and per tile of CL_TILE giants the first earlier giant inside its DM window.
+// Each sweep found these for itself: a 64-bit division per giant and a binary
+// search of dependent loads per block, most of a short sweep's time.
+__device__ __forceinline__ void cluster_prepare(const ClusterArgs& a, const GiantBuffers& gb,
+                                                int i) {
+  const unsigned long long ind = gb.ind[i];
+  const int f = gb.filter[i], d = gb.dm[i];
+  const unsigned long long tt = a.time_tol << f;
+  gb.label[i] = i;
+  gb.pack[i] = make_int4((int)(unsigned)ind, (int)(unsigned)min(tt, 0xFFFFFFFFull),
+                         (int)(unsigned)(ind / a.nsamps_beam), d);
+  if (i % CL_TILE == 0) {
+    // giants are in ascending DM order: the first candidate neighbour is the
+    // first giant within dm_tol of the tile's smallest DM
+    int lo = 0, hi = i;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if ((long long)gb.dm[mid] + (long long)a.dm_tol < (long long)d) lo = mid + 1;
+      else hi = mid;
+    }
+    gb.tile_first[i / CL_TILE] = lo;
+  }
+}
+
+__global__ void k_cluster_init(ClusterArgs a, GiantBuffers gb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.ngiants) cluster_prepare(a, gb, i);
 }
 
 // Block (x, y): giants [x*CL_TILE, +CL_TILE) against the y-th chunk of
@@ -2127,36 +2269,21 @@ __global__ void k_cluster_init(int* label, int n) {
 __device__ __forceinline__ void cluster_sweep_block(const ClusterArgs& a, const GiantBuffers& gb,
                                                     const int n, unsigned* changed,
                                                     const int jchunk) {
-  __shared__ unsigned s_samp[CL_TILE], s_beam[CL_TILE];
-  __shared__ int s_f[CL_TILE], s_dm[CL_TILE], s_lab[CL_TILE];
+  __shared__ int4 s_pack[CL_TILE];
+  __shared__ int2 s_fl[CL_TILE];  // filter, label
   const int i_first = blockIdx.x * CL_TILE;
   const int i = i_first + threadIdx.x;
   const int i_last = min(i_first + CL_TILE, n) - 1;
   if ((long long)blockIdx.y * jchunk > (long long)i_last) return;  // uniform: past the tile
-  // giants are in ascending DM order: the first candidate neighbour is the
-  // first giant within dm_tol of the tile's smallest DM
-  const int dm_first = gb.dm[i_first];
-  int lo = 0, hi = i_first;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if ((long long)gb.dm[mid] + (long long)a.dm_tol < (long long)dm_first) lo = mid + 1;
-    else hi = mid;
-  }
-  const long long jb = (long long)lo + (long long)blockIdx.y * jchunk;
+  const long long jb = (long long)gb.tile_first[blockIdx.x] + (long long)blockIdx.y * jchunk;
   if (jb > (long long)i_last) return;  // uniform: this chunk lies past the tile
   const int j_begin = (int)jb;
   const int j_end = (int)min((long long)j_begin + jchunk, (long long)i_last + 1);
-  // sample indices fit 31 bits (checked by the host); the test below is
-  // are_coincident_beam (are_coincident.cuh:47-68): same beam, time within
-  // time_tol x the wider boxcar (a power of two), filter and DM within tolerance.
-  // A giant's beam is computed once, when it is staged.
-  unsigned si = 0, bi = 0;
-  int fi = 0, di = 0, best = 0x7FFFFFFF;
+  int4 p = make_int4(0, 0, 0, 0);
+  int f = 0, best = 0x7FFFFFFF;
   if (i < n) {
-    si = (unsigned)gb.ind[i];
-    bi = (unsigned)(gb.ind[i] / a.nsamps_beam);
-    fi = gb.filter[i];
-    di = gb.dm[i];
+    p = gb.pack[i];
+    f = gb.filter[i];
     best = gb.label[i];
   }
   const int start_best = best;
@@ -2166,25 +2293,24 @@ __device__ __forceinline__ void cluster_sweep_block(const ClusterArgs& a, const 
     const int j = j0 + threadIdx.x;
     __syncthreads();
     if (j < j_end) {
-      const unsigned long long sj = gb.ind[j];
-      s_samp[threadIdx.x] = (unsigned)sj;
-      s_beam[threadIdx.x] = (unsigned)(sj / a.nsamps_beam);
-      s_f[threadIdx.x] = gb.filter[j];
-      s_dm[threadIdx.x] = gb.dm[j];
-      s_lab[threadIdx.x] = *((volatile int*)&gb.label[j]);
+      s_pack[threadIdx.x] = gb.pack[j];
+      s_fl[threadIdx.x] = make_int2(gb.filter[j], *((volatile int*)&gb.label[j]));
     }
     __syncthreads();
     if (i < n) {
       const int jn = min(min(CL_TILE, j_end - j0), i - j0);  // only j < i
+#pragma unroll 4
       for (int jj = 0; jj < jn; jj++) {
-        const unsigned sj = s_samp[jj];
-        const int fj = s_f[jj];
+        const int4 q = s_pack[jj];
+        const int2 fl = s_fl[jj];
+        const unsigned si = (unsigned)p.x, sj = (unsigned)q.x;
         const unsigned dt = sj > si ? sj - si : si - sj;
-        const unsigned long long tt = a.time_tol << max(fi, fj);
-        const bool coinc = s_beam[jj] == bi && (unsigned long long)dt <= tt &&
-                           (unsigned)abs(fj - fi) <= ftol &&
-                           (unsigned)abs(s_dm[jj] - di) <= dtol;
-        if (coinc && s_lab[jj] < best) best = s_lab[jj];
+        // the wider boxcar's tolerance is the larger one; every test is made
+        // (no short circuit), so that the loop has no branches
+        const int coinc = (int)(dt <= max((unsigned)p.y, (unsigned)q.y)) & (int)(q.z == p.z) &
+                          (int)((unsigned)abs(fl.x - f) <= ftol) &
+                          (int)((unsigned)abs(q.w - p.w) <= dtol);
+        best = min(best, coinc ? fl.y : 0x7FFFFFFF);
       }
     }
   }
@@ -2212,9 +2338,9 @@ __global__ void k_cluster_jump(int* label, int n, unsigned* changed) {
   }
 }
 
-cudaError_t cluster_init(GiantBuffers& gb, int n, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  k_cluster_init<<<(n + 255) / 256, 256, 0, s>>>(gb.label, n); note_launch();
+cudaError_t cluster_init(const ClusterArgs& a, GiantBuffers& gb, cudaStream_t s) {
+  if (a.ngiants == 0) return cudaSuccess;
+  k_cluster_init<<<(a.ngiants + 255) / 256, 256, 0, s>>>(a, gb); note_launch();
   return cudaGetLastError();
 }
 
@@ -2384,10 +2510,10 @@ __global__ void k_cluster_geom(const unsigned* __restrict__ offs, int units,
   geo[1] = (int)chunk;
 }
 
-__global__ void k_cluster_init_dev(int* label, const int* geo) {
+__global__ void k_cluster_init_dev(ClusterArgs a, GiantBuffers gb, const int* geo) {
   const int n = geo[0];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    label[i] = i;
+    cluster_prepare(a, gb, i);
 }
 
 // Sweep `which` (0, 1) of pair `pair`: nothing to do once the previous
@@ -2471,7 +2597,7 @@ cudaError_t cluster_merge_dev(const ClusterArgs& a, GiantBuffers& gb, unsigned g
   note_launch();
   k_cluster_geom<<<1, 32, 0, s>>>(unit_off, units, ngiants, gcap, geo);
   note_launch();
-  k_cluster_init_dev<<<grid_for(gcap, 256), 256, 0, s>>>(gb.label, geo);
+  k_cluster_init_dev<<<grid_for(gcap, 256), 256, 0, s>>>(a, gb, geo);
   note_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

@@ -113,6 +113,7 @@ struct hd_pipeline_t {
   GiantSet main_giants;           // the gulp's giant list
   std::vector<GiantSet> gsets;    // per scrunch group (adaptive dt)
   DevBuf place_base;
+  DevBuf cl_pack, cl_first;       // clustering's copies of the giant list
   DevBuf scan_tmp, small;  // small: totals / flags
   DevBuf root_flag, root_off, mkey, rows, unit_off;
   DevBuf h_small_dev;
@@ -677,6 +678,8 @@ static hd_error enqueue_gulp(hd_pipeline pl, const GulpGeom& g,
   pl->main_giants.view(gb);
   gb.head = pl->head.as<unsigned>();
   gb.gid = pl->gid.as<unsigned>();
+  gb.pack = pl->cl_pack.as<int4>();
+  gb.tile_first = pl->cl_first.as<int>();
   gb.cap = gcap;
   HD_TRY(hdb::giants_dev(wctx, hb, small, hcap, gb, gcap, small + 1, scan_tmp, s));
   HD_TRY(mark(6));
@@ -803,6 +806,8 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   need(m.label, G * sizeof(int));
   need(pl->scan_tmp,
        hdb::scan_tmp_words(std::max({g.nsw, (size_t)hcap, (size_t)gcap})) * sizeof(unsigned));
+  need(pl->cl_pack, G * sizeof(int4));
+  need(pl->cl_first, (G / 128 + 2) * sizeof(int));
   need(pl->root_flag, G * sizeof(unsigned));
   need(pl->root_off, G * sizeof(unsigned));
   need(pl->mkey, 2 * G * sizeof(unsigned long long));
@@ -825,7 +830,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
                           &pl->hit_val, &pl->hit_sw, &pl->head, &pl->gid, &m.key, &m.peak,
                           &m.ind, &m.begin, &m.end, &m.filter, &m.dm, &m.label, &pl->scan_tmp,
                           &pl->small, &pl->root_flag, &pl->root_off, &pl->mkey, &pl->rows,
-                          &pl->unit_off, &pl->geo}) {
+                          &pl->unit_off, &pl->geo, &pl->cl_pack, &pl->cl_first}) {
     key.push_back((size_t)b->p);
     key.push_back(b->cap);
   }
@@ -1394,11 +1399,15 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
   pl->obs_pairs = 0;
   if (any_ok && ngiants > 0) {
     // ---- clustering ----------------------------------------------------------
-    HD_TRY(hdb::cluster_init(gb, (int)ngiants, s));
+    HD_TRY(pl->cl_pack.ensure(((size_t)ngiants + 1) * sizeof(int4)));
+    HD_TRY(pl->cl_first.ensure(((size_t)ngiants / 128 + 2) * sizeof(int)));
+    gb.pack = pl->cl_pack.as<int4>();
+    gb.tile_first = pl->cl_first.as<int>();
     unsigned max_unit = 0;
     for (size_t u = 0; u < U; u++) max_unit = std::max(max_unit, first[u + 1] - first[u]);
     hdb::ClusterArgs ca{(int)ngiants, P.cand_sep_time, P.cand_sep_filter, dm_tol,
                         (unsigned long long)(nsamps / nbeams), (int)max_unit};
+    HD_TRY(hdb::cluster_init(ca, gb, s));
     // sweeps until one changes nothing; the fixed point is idempotent, so
     // the sweeps run in pairs, each with its own flag, and the host reads
     // both flags once per pair: the loop ends when the pair's second sweep
