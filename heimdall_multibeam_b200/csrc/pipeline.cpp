@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -72,6 +73,23 @@ struct hd_pipeline_t {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host->device copies overlapped with compute
+  // adaptive dt: a scrunch group's series are baselined, normalised and summed
+  // on a side stream (the sums are serial chains that leave most of the GPU
+  // idle) while other groups are dedispersed and searched on `stream`
+  static constexpr int kSide = 3;
+  cudaStream_t side[kSide] = {};
+  std::vector<cudaEvent_t> side_ev;  // two per group: dedispersed, summed
+  cudaError_t ensure_side(size_t ngroups) {
+    for (auto& q : side)
+      if (!q)
+        if (cudaError_t e = cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking)) return e;
+    while (side_ev.size() < 2 * ngroups) {
+      cudaEvent_t v = nullptr;
+      if (cudaError_t e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) return e;
+      side_ev.push_back(v);
+    }
+    return cudaSuccess;
+  }
   cudaEvent_t ev[10] = {};
   cudaEvent_t chunk_ev[kMaxChunks] = {};
   // double-buffered ingest (hd_prefetch_beams / hd_execute_prefetched): two
@@ -222,6 +240,8 @@ struct hd_pipeline_t {
     for (auto& e : ev) if (e) cudaEventDestroy(e);
     for (auto& e : chunk_ev) if (e) cudaEventDestroy(e);
     for (auto& q : pf) if (q.done) cudaEventDestroy(q.done);
+    for (auto& v : side_ev) cudaEventDestroy(v);
+    for (auto& q : side) if (q) cudaStreamDestroy(q);
     if (stream) cudaStreamDestroy(stream);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     if (h_small) cudaFreeHost(h_small);
@@ -1125,23 +1145,18 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
                                    D * dd_pitch);
       if (de != DEDISP_NO_ERROR) return dedisp_err(de);
     }
-    de = hdb::plan_dedisperse_ft(pl->plan, pl->fb_ft.as<uint8_t>(), pitch, nsamps, dd, dd_pitch,
-                                 s, U, ft_unit, D * dd_pitch);
-    if (de != DEDISP_NO_ERROR) return dedisp_err(de);
+    if (pl->plan->groups.empty()) {
+      de = hdb::plan_dedisperse_ft(pl->plan, pl->fb_ft.as<uint8_t>(), pitch, nsamps, dd,
+                                   dd_pitch, s, U, ft_unit, D * dd_pitch);
+      if (de != DEDISP_NO_ERROR) return dedisp_err(de);
+    }
     if (nbits == 16)
       HD_TRY(hdb::launch_combine_planes(dd, pl->dd_hi.as<float>(), dd_pitch, nc, NS, s));
   }
   // the element after each series is read (never used) by the baseline stretch
-  if (pl->plan->groups.empty()) {
+  if (pl->plan->groups.empty())
     HD_TRY(cudaMemset2DAsync(dd + nc, dd_pitch * sizeof(float), 0, sizeof(float), NS, s));
-  } else {
-    for (const auto& g : pl->plan->groups)
-      HD_TRY(cudaMemset2DAsync(dd + U * g.d0 * dd_pitch + nc / g.s, dd_pitch * sizeof(float), 0,
-                               sizeof(float), U * (g.d1 - g.d0), s));
-  }
-  cudaEventRecord(pl->ev[3], s);
 
-  const size_t stride = nsamps / nbeams;
   const size_t Bmax = P.boxcar_max;
   // scrunch groups: trials [d0, d1) searched at factor s (one group of factor
   // 1 without adaptive dt); the series rows are group-major, group g's U * (d1
@@ -1175,19 +1190,34 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
   hdb::GiantBuffers gb{};
   std::vector<unsigned> group_giants(ngs, 0);
   const size_t scan_pitch = round_up(nc + 1, 4);
+  // Series of group gi: baseline, RMS and normalise + scan on stream q, with
+  // its own part of the scratch buffers (the groups may run at once).
+  struct GroupScratch { size_t tree_at, tree_cap, base_at, rms_at; };
+  std::vector<GroupScratch> scratch(ngs);
+  size_t tree_total = 0, base_total = 0, rms_total = 0, tree_search = 0;
+  for (size_t gi = 0; gi < ngs; gi++) {
+    const size_t scr = groups[gi].s, NSg = U * (groups[gi].d1 - groups[gi].d0);
+    const size_t stride_s = nsamps / nbeams / scr;
+    const float cur_dt = P.dt * (float)scr;
+    const size_t nsmooth = (size_t)(P.baseline_length / (2 * cur_dt));
+    GroupScratch& g = scratch[gi];
+    g.tree_at = tree_total;
+    g.tree_cap = round_up(std::max(tree_cap(NSg * nbeams, stride_s),
+                                   hdb::baseline_scratch(stride_s, nsmooth, NSg * nbeams)), 64);
+    tree_total += g.tree_cap;
+    g.base_at = base_total;
+    base_total += round_up(NSg * nbeams * hdb::baseline_samples(stride_s, nsmooth) + 64, 64);
+    g.rms_at = rms_total;
+    rms_total += round_up(NSg * nbeams + 16, 64);
+    tree_search = std::max(tree_search,
+                           tree_cap(NSg * (log2u(Bmax) + 1), nbeams * stride_s));
+  }
   if (search) {
-    const size_t cap = std::max({tree_cap(NS * nbeams, stride),
-                                 tree_cap(NS * (log2u(Bmax) + 1), nbeams * stride),
-                                 hdb::baseline_scratch(stride, (size_t)(P.baseline_length /
-                                                                        (2 * P.dt)),
-                                                       NS * nbeams)});
-    HD_TRY(pl->ws_a.ensure(cap * sizeof(float)));
-    HD_TRY(pl->ws_b.ensure(cap * sizeof(float)));
-    HD_TRY(pl->base.ensure((NS * nbeams *
-                                hdb::baseline_samples(stride, (size_t)(P.baseline_length /
-                                                                       (2 * P.dt))) +
-                            64) * sizeof(float)));
-    HD_TRY(pl->rms.ensure(NS * nbeams * sizeof(float) + 64));
+    // the search of one group at a time has its own part after the groups'
+    HD_TRY(pl->ws_a.ensure((tree_total + tree_search) * sizeof(float)));
+    HD_TRY(pl->ws_b.ensure((tree_total + tree_search) * sizeof(float)));
+    HD_TRY(pl->base.ensure(base_total * sizeof(float)));
+    HD_TRY(pl->rms.ensure(rms_total * sizeof(float)));
     HD_TRY(pl->scan.ensure(NS * scan_pitch * sizeof(float)));
     HD_TRY(pl->small.ensure(64 * sizeof(unsigned)));
     pl->searched = !multi;  // patches read unscrunched series only
@@ -1197,25 +1227,70 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
     pl->last_units = U;
     if (multi && pl->gsets.size() < ngs) pl->gsets.resize(ngs);
   }
-  for (size_t gi = 0; gi < ngs; gi++) {
+  auto series_of = [&](size_t gi, cudaStream_t q) {
+    const GroupSpec& G = groups[gi];
+    const size_t scr = G.s, NSg = U * (G.d1 - G.d0), row0 = U * G.d0;
+    const size_t stride_s = nsamps / nbeams / scr;
+    const size_t bcount = stride_s - max_delay / scr;
+    hdb::SeriesBatch sb{dd + row0 * dd_pitch, dd_pitch, (int)NSg, nc / scr, stride_s, bcount,
+                        (int)nbeams};
+    const float cur_dt = P.dt * (float)scr;
+    const size_t nsmooth = (size_t)(P.baseline_length / (2 * cur_dt));
+    const GroupScratch& g = scratch[gi];
+    hdb::TreeScratch ws{pl->ws_a.as<float>() + g.tree_at, pl->ws_b.as<float>() + g.tree_at,
+                        g.tree_cap};
+    float* rms = pl->rms.as<float>() + g.rms_at;
+    cudaError_t e = hdb::remove_baseline(sb, nsmooth, pl->base.as<float>() + g.base_at, ws, q);
+    if (e == cudaSuccess) e = hdb::rms_beams(sb, rms, ws, q);
+    if (e == cudaSuccess)
+      e = hdb::normalise_scan(sb, rms, pl->scan.as<float>() + row0 * scan_pitch, scan_pitch,
+                              nullptr, q, pl->plan->d_err);
+    return e;
+  };
+  // side-stream work of this call never outlives it (an error return included)
+  struct SideGuard {
+    hd_pipeline pl;
+    ~SideGuard() {
+      for (auto& q : pl->side)
+        if (q) cudaStreamSynchronize(q);
+    }
+  };
+  std::unique_ptr<SideGuard> side_guard;
+  if (!pl->plan->groups.empty()) {
+    // group by group: dedisperse on s, then the series on a side stream (the
+    // native-resolution group, with the longest chains, has one for itself)
+    side_guard.reset(new SideGuard{pl});
+    HD_TRY(pl->ensure_side(groups.size()));
+    for (size_t gi = 0; gi < groups.size(); gi++) {
+      const GroupSpec& G = groups[gi];
+      de = hdb::plan_dedisperse_group(pl->plan, gi, pl->fb_ft.as<uint8_t>(), pitch, nsamps, dd,
+                                      dd_pitch, s, U, ft_unit);
+      if (de != DEDISP_NO_ERROR) return dedisp_err(de);
+      HD_TRY(cudaMemset2DAsync(dd + U * G.d0 * dd_pitch + nc / G.s, dd_pitch * sizeof(float), 0,
+                               sizeof(float), U * (G.d1 - G.d0), s));
+      if (gi >= ngs) continue;
+      const cudaStream_t q = pl->side[gi == 0 ? 0 : 1 + gi % (hd_pipeline_t::kSide - 1)];
+      HD_TRY(cudaEventRecord(pl->side_ev[2 * gi], s));
+      HD_TRY(cudaStreamWaitEvent(q, pl->side_ev[2 * gi], 0));
+      HD_TRY(series_of(gi, q));
+      HD_TRY(cudaEventRecord(pl->side_ev[2 * gi + 1], q));
+    }
+  }
+  cudaEventRecord(pl->ev[3], s);
+  // the coarsest group's series are ready first
+  for (size_t go = 0; go < ngs; go++) {
+    const size_t gi = ngs - 1 - go;
     const GroupSpec& G = groups[gi];
     const size_t scr = G.s, Dg = G.d1 - G.d0, NSg = U * Dg, row0 = U * G.d0;
     const size_t nc_s = nc / scr;
     const size_t cur_delay = max_delay / scr;
     const size_t stride_s = nsamps / nbeams / scr;
     const size_t rel_bmax = Bmax / scr;
-    // ---- per-DM baseline, RMS, normalise + scan ------------------------------
-    const size_t bcount = stride_s - cur_delay;
-    float* ddg = dd + row0 * dd_pitch;
     float* scan_g = pl->scan.as<float>() + row0 * scan_pitch;
-    hdb::SeriesBatch sb{ddg, dd_pitch, (int)NSg, nc_s, stride_s, bcount, (int)nbeams};
-    const float cur_dt = P.dt * (float)scr;
-    const size_t nsmooth = (size_t)(P.baseline_length / (2 * cur_dt));
-    hdb::TreeScratch ws{pl->ws_a.as<float>(), pl->ws_b.as<float>(), pl->ws_a.cap / sizeof(float)};
-    HD_TRY(hdb::remove_baseline(sb, nsmooth, pl->base.as<float>(), ws, s));
-    HD_TRY(hdb::rms_beams(sb, pl->rms.as<float>(), ws, s));
-    HD_TRY(hdb::normalise_scan(sb, pl->rms.as<float>(), scan_g, scan_pitch, nullptr, s,
-                               pl->plan->d_err));
+    hdb::TreeScratch ws{pl->ws_a.as<float>() + tree_total, pl->ws_b.as<float>() + tree_total,
+                        pl->ws_a.cap / sizeof(float) - tree_total};
+    if (pl->plan->groups.empty()) HD_TRY(series_of(gi, s));
+    else HD_TRY(cudaStreamWaitEvent(s, pl->side_ev[2 * gi + 1], 0));
     if (gi == 0) cudaEventRecord(pl->ev[4], s);
 
     // ---- widths (pipeline.cu:657-776 at this group's factor) ------------------

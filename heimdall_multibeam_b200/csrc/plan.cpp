@@ -531,41 +531,44 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
     return dedisperse_tables(p, p->delays, p->d_delays, p->d_blk_range, p->max_span,
                              p->mean_span, p->max_delay, (int)p->dm_list.size(), nout, 0, d_ft, pitch, nsamps, d_out,
                              out_pitch, s, units, in_unit, out_unit);
-  // adaptive dt: group g's trials [d0, d1) of every unit are rows
-  // units * d0 + u * (d1 - d0) + i of the output (group-major)
-  const size_t C = p->nchans;
   for (size_t gi = 0; gi < p->groups.size(); gi++) {
-    const dedisp_plan_struct::Group& g = p->groups[gi];
-    const size_t Dg = g.d1 - g.d0;
-    const size_t nout_s = nout / g.s;
-    float* out_g = d_out + units * g.d0 * out_pitch;
-    if (g.s == 1) {
-      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span,
-                             g.mean_span, g.max_delay, (int)Dg, nout_s, gi + 1,
-                             d_ft, pitch, nsamps, out_g, out_pitch, s, units, in_unit,
-                             Dg * out_pitch);
-    } else {
-      const size_t ns = nsamps / g.s;
-      const size_t pitch_s = ft_pitch(p, ns);
-      const size_t need = units * pitch_s * C;
-      if (p->d_scr_cap < need) {
-        free_dev(p->d_scr);
-        p->d_scr = nullptr;
-        p->d_scr_cap = 0;
-        if (dev_malloc(&p->d_scr, need) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
-        p->d_scr_cap = need;
-      }
-      if (launch_scrunch_ft(d_ft, pitch, nsamps, (int)C, (int)g.s, p->d_scr, pitch_s, units,
-                            in_unit, pitch_s * C, s) != cudaSuccess)
-        return DEDISP_INTERNAL_GPU_ERROR;
-      de = dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span,
-                             g.mean_span, g.max_delay, (int)Dg, nout_s, gi + 1,
-                             p->d_scr, pitch_s, ns, out_g, out_pitch, s, units, pitch_s * C,
-                             Dg * out_pitch);
-    }
+    de = plan_dedisperse_group(p, gi, d_ft, pitch, nsamps, d_out, out_pitch, s, units, in_unit);
     if (de != DEDISP_NO_ERROR) return de;
   }
   return DEDISP_NO_ERROR;
+}
+
+// adaptive dt: group gi's trials [d0, d1) of every unit are rows
+// units * d0 + u * (d1 - d0) + i of the output (group-major)
+dedisp_error plan_dedisperse_group(dedisp_plan p, size_t gi, const uint8_t* d_ft, size_t pitch,
+                                   size_t nsamps, float* d_out, size_t out_pitch, cudaStream_t s,
+                                   size_t units, size_t in_unit) {
+  const size_t C = p->nchans;
+  const size_t nout = nsamps - p->max_delay;
+  const dedisp_plan_struct::Group& g = p->groups[gi];
+  const size_t Dg = g.d1 - g.d0;
+  const size_t nout_s = nout / g.s;
+  float* out_g = d_out + units * g.d0 * out_pitch;
+  if (g.s == 1)
+    return dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span, g.mean_span,
+                             g.max_delay, (int)Dg, nout_s, gi + 1, d_ft, pitch, nsamps, out_g,
+                             out_pitch, s, units, in_unit, Dg * out_pitch);
+  const size_t ns = nsamps / g.s;
+  const size_t pitch_s = ft_pitch(p, ns);
+  const size_t need = units * pitch_s * C;
+  if (p->d_scr_cap < need) {
+    free_dev(p->d_scr);
+    p->d_scr = nullptr;
+    p->d_scr_cap = 0;
+    if (dev_malloc(&p->d_scr, need) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
+    p->d_scr_cap = need;
+  }
+  if (launch_scrunch_ft(d_ft, pitch, nsamps, (int)C, (int)g.s, p->d_scr, pitch_s, units,
+                        in_unit, pitch_s * C, s) != cudaSuccess)
+    return DEDISP_INTERNAL_GPU_ERROR;
+  return dedisperse_tables(p, g.delays, g.d_delays, g.d_blk_range, g.max_span, g.mean_span,
+                           g.max_delay, (int)Dg, nout_s, gi + 1, p->d_scr, pitch_s, ns, out_g,
+                           out_pitch, s, units, pitch_s * C, Dg * out_pitch);
 }
 
 }  // namespace hdb

@@ -116,4 +116,11 @@ dedisp_error plan_dedisperse_ft(dedisp_plan p, const uint8_t* d_ft, size_t pitch
                                 float* d_out, size_t out_pitch, cudaStream_t s, size_t units = 1,
                                 size_t in_unit = 0, size_t out_unit = 0);
 
+// The same for the trials of one scrunch group of a plan with adaptive dt
+// (its plan prepared, nsamps >= max_delay; the groups share the plan's
+// scratch, so they run on one stream).
+dedisp_error plan_dedisperse_group(dedisp_plan p, size_t gi, const uint8_t* d_ft, size_t pitch,
+                                   size_t nsamps, float* d_out, size_t out_pitch, cudaStream_t s,
+                                   size_t units, size_t in_unit);
+
 }  // namespace hdb
