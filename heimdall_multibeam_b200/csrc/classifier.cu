@@ -517,8 +517,15 @@ constexpr int kWarps = 16, kThreads = kWarps * 32;
 // are dense.
 template <int C>
 __host__ __device__ constexpr int pix_stride() { return C == 16 ? 24 : C; }
-constexpr int kR0 = 18 * 66 * 24 * 2;   // B input [66][258]; B pool-2 [18][66][24]; A pool-1 [34][34][8]
-constexpr int kR1 = 34 * 130 * 8 * 2;   // B pool-1 [34][130][8]; A input [66][66]; A pool-2 [18][18][24]
+// Pixels from one row of a layer's input to the next, and the padded row's
+// first: 1-channel rows are W + 16 apart (8 banks apart modulo 32, so the four
+// taps that a fragment load takes from three rows miss one another) and start
+// 7 in, which puts the image on 16-byte boundaries.
+__host__ __device__ constexpr int row_pitch(int c, int w) { return c == 1 ? w + 16 : w + 2; }
+__host__ __device__ constexpr int row_start(int c) { return c == 1 ? 7 : 0; }
+constexpr int kR0 = 18 * 66 * 24 * 2;   // B input [66][272]; B pool-2 [18][66][24]; A pool-1 [34][34][8]
+constexpr int kR1 = 34 * 130 * 8 * 2;   // B pool-1 [34][130][8]; A input [66][80]; A pool-2 [18][18][24]
+static_assert(66 * 272 * 2 <= kR0 && 66 * 80 * 2 <= kR1, "input regions");
 constexpr int kF = 10240 * 2;           // flattened features
 // weight fragments per layer: ksteps x (c_out / 8) x 32 lanes of uint2
 constexpr int kFragL1 = 1 * 1 * 32, kFragL2 = 5 * 2 * 32, kFragL3 = 9 * 4 * 32;
@@ -570,34 +577,46 @@ __device__ void build_frags(const float* W, uint2* wf) {
   }
 }
 
-// zero ring of a [H2 + 2][W2 + 2][C] buffer
-__device__ void zero_ring(bf16* buf, int H2, int W2, int C) {
-  const int Wp = W2 + 2, Hp = H2 + 2;
-  const int ring = 2 * Wp + 2 * H2;  // pixels
-  const bf16 z = __float2bfloat16(0.f);
-  for (int e = threadIdx.x; e < ring * C; e += blockDim.x) {
-    const int px = e / C, c = e % C;
+// zero ring of a [H2 + 2][W2 + 2][C] buffer (C a multiple of 8)
+template <int H2, int W2, int C>
+__device__ void zero_ring(bf16* buf) {
+  constexpr int Wp = W2 + 2, Hp = H2 + 2, Q = C / 8;  // 16-byte pieces of a pixel
+  constexpr int ring = 2 * Wp + 2 * H2;               // pixels
+  for (int e = threadIdx.x; e < ring * Q; e += kThreads) {
+    const int px = e / Q;
     int y, x;
     if (px < Wp) { y = 0; x = px; }
     else if (px < 2 * Wp) { y = Hp - 1; x = px - Wp; }
     else { const int q = px - 2 * Wp; y = 1 + (q >> 1); x = (q & 1) ? Wp - 1 : 0; }
-    buf[((size_t)y * Wp + x) * C + c] = z;
+    reinterpret_cast<uint4*>(buf + ((size_t)y * Wp + x) * C)[e % Q] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
-// patch rows (FP32, global) -> BF16 [66][W + 2] with a zero ring, limited to
-// +-kInputClip as the training input
-__device__ void load_input(const float* __restrict__ src, int W, bf16* dst) {
-  zero_ring(dst, 64, W, 1);
-  const int n4 = 64 * W / 4;
-  for (int e = threadIdx.x; e < n4; e += blockDim.x) {
-    const float4 v = reinterpret_cast<const float4*>(src)[e];
-    const int y = (4 * e) / W, x = (4 * e) % W;
-    bf16* o = dst + (size_t)(y + 1) * (W + 2) + x + 1;
-    o[0] = __float2bfloat16(fminf(fmaxf(v.x, -kInputClip), kInputClip));
-    o[1] = __float2bfloat16(fminf(fmaxf(v.y, -kInputClip), kInputClip));
-    o[2] = __float2bfloat16(fminf(fmaxf(v.z, -kInputClip), kInputClip));
-    o[3] = __float2bfloat16(fminf(fmaxf(v.w, -kInputClip), kInputClip));
+// patch rows (FP32, global) -> BF16 [66][W + 16] with a zero ring around the
+// image (row_start), limited to +-kInputClip as the training input
+template <int W>
+__device__ void load_input(const float* __restrict__ src, bf16* dst) {
+  constexpr int P = row_pitch(1, W);
+  const bf16 z = __float2bfloat16(0.f);
+  for (int e = threadIdx.x; e < P; e += kThreads) {
+    dst[e] = z;
+    dst[65 * P + e] = z;
+  }
+  for (int y = threadIdx.x; y < 64; y += kThreads) {
+    dst[(y + 1) * P + 7] = z;
+    dst[(y + 1) * P + 8 + W] = z;
+  }
+  constexpr int n4 = 64 * W / 4, N = n4 / kThreads;  // all loads in flight at once
+  float4 v[N];
+#pragma unroll
+  for (int k = 0; k < N; k++)
+    v[k] = __ldg(reinterpret_cast<const float4*>(src) + threadIdx.x + k * kThreads);
+  auto clip = [](float x) { return __float2bfloat16(fminf(fmaxf(x, -kInputClip), kInputClip)); };
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int e = threadIdx.x + k * kThreads, y = (4 * e) / W, x = (4 * e) % W;
+    *reinterpret_cast<uint2*>(dst + (y + 1) * P + 8 + x) =
+        make_uint2(pack2(clip(v[k].x), clip(v[k].y)), pack2(clip(v[k].z), clip(v[k].w)));
   }
 }
 
@@ -605,23 +624,32 @@ __device__ void load_input(const float* __restrict__ src, int W, bf16* dst) {
 // (pixels pix_stride<CI>() elements apart).
 // out: [H/2 + 2][W/2 + 2][pix_stride<CO>()] interior, or (feat) the flattened features at
 // feat[c * (H/2 * W/2) + y * W/2 + x].
-template <int CI, int CO>
-__device__ void conv_layer(const bf16* __restrict__ in, int H, int W, const uint2* __restrict__ wf,
+// A warp's weight fragments stay in registers over its tiles (two wavefronts
+// of shared memory per fragment and tile otherwise, twice the pixels' share in
+// the last layer).
+template <int CI, int CO, int H, int W>
+__device__ void conv_layer(const bf16* __restrict__ in_, const uint2* __restrict__ wf,
                            const float* __restrict__ bias, bf16* __restrict__ out,
                            bf16* __restrict__ feat) {
   constexpr int KS = CI == 16 ? 9 : (CI == 8 ? 5 : 1);
   constexpr int NT = CO / 8;
   constexpr int PSI = pix_stride<CI>(), PSO = pix_stride<CO>();
+  constexpr int Wp = row_pitch(CI, W), W2 = W / 2, H2 = H / 2;
+  constexpr int ntx = W / 8, ntiles = H2 * ntx;
+  const bf16* in = in_ + row_start(CI) * PSI;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int Wp = W + 2, W2 = W / 2, H2 = H / 2;
-  const int ntx = W / 8, ntiles = H2 * ntx;
   float bia[NT][2];
 #pragma unroll
   for (int j = 0; j < NT; j++) {
     bia[j][0] = bias[8 * j + 2 * t];
     bia[j][1] = bias[8 * j + 2 * t + 1];
   }
+  uint2 frag[KS][NT];
+#pragma unroll
+  for (int s = 0; s < KS; s++)
+#pragma unroll
+    for (int j = 0; j < NT; j++) frag[s][j] = wf[(s * NT + j) * 32 + lane];
   for (int tile = warp; tile < ntiles; tile += kWarps) {
     const int ty = tile / ntx, tx = tile % ntx;
     // pixel rows of the MMA tile: row g -> (2ty, 8tx + g), row g + 8 -> (2ty + 1, 8tx + g);
@@ -665,8 +693,7 @@ __device__ void conv_layer(const bf16* __restrict__ in, int H, int W, const uint
       }
 #pragma unroll
       for (int j = 0; j < NT; j++) {
-        const uint2 b = wf[(s * NT + j) * 32 + lane];
-        const uint32_t bb[2] = {b.x, b.y};
+        const uint32_t bb[2] = {frag[s][j].x, frag[s][j].y};
         mma_bf16(acc[j], a, bb);
       }
     }
@@ -709,30 +736,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_clf_infer(Args a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int cand = blockIdx.x; cand < a.n; cand += gridDim.x) {
     __syncthreads();  // fragments ready / previous candidate's FC done
+    // the next candidate's patches into L2 while this one is computed
+    if (cand + (int)gridDim.x < a.n) {
+      const size_t nx = (size_t)cand + gridDim.x;
+      const char* p = reinterpret_cast<const char*>(a.ft + nx * 16384) + threadIdx.x * 128;
+      asm volatile("prefetch.global.L2 [%0];" :: "l"(p));  // 512 lines of 128 bytes
+      if (threadIdx.x < 128) {
+        p = reinterpret_cast<const char*>(a.dm + nx * 4096) + threadIdx.x * 128;
+        asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
+      }
+    }
     // ---- branch B (freq-time, 64 x 256): features 2048.. ----
     const uint2* fB = wf + kFragBranch;
-    load_input(a.ft + (size_t)cand * 16384, 256, r0);
-    zero_ring(r1, 32, 128, 8);
+    load_input<256>(a.ft + (size_t)cand * 16384, r0);
+    zero_ring<32, 128, 8>(r1);
     __syncthreads();
-    conv_layer<1, 8>(r0, 64, 256, fB, a.w + a.off_b[1][0], r1, nullptr);
+    conv_layer<1, 8, 64, 256>(r0, fB, a.w + a.off_b[1][0], r1, nullptr);
     __syncthreads();
-    zero_ring(r0, 16, 64, pix_stride<16>());
-    conv_layer<8, 16>(r1, 32, 128, fB + kFragL1, a.w + a.off_b[1][1], r0, nullptr);
+    zero_ring<16, 64, pix_stride<16>()>(r0);
+    conv_layer<8, 16, 32, 128>(r1, fB + kFragL1, a.w + a.off_b[1][1], r0, nullptr);
     __syncthreads();
-    conv_layer<16, 32>(r0, 16, 64, fB + kFragL1 + kFragL2, a.w + a.off_b[1][2], nullptr,
-                       feat + 2048);
-    __syncthreads();
+    conv_layer<16, 32, 16, 64>(r0, fB + kFragL1 + kFragL2, a.w + a.off_b[1][2], nullptr,
+                               feat + 2048);
     // ---- branch A (DM-time, 64 x 64): features 0..2047 ----
     const uint2* fA = wf;
-    load_input(a.dm + (size_t)cand * 4096, 64, r1);
-    zero_ring(r0, 32, 32, 8);
+    load_input<64>(a.dm + (size_t)cand * 4096, r1);
     __syncthreads();
-    conv_layer<1, 8>(r1, 64, 64, fA, a.w + a.off_b[0][0], r0, nullptr);
+    zero_ring<32, 32, 8>(r0);
+    conv_layer<1, 8, 64, 64>(r1, fA, a.w + a.off_b[0][0], r0, nullptr);
     __syncthreads();
-    zero_ring(r1, 16, 16, pix_stride<16>());
-    conv_layer<8, 16>(r0, 32, 32, fA + kFragL1, a.w + a.off_b[0][1], r1, nullptr);
+    zero_ring<16, 16, pix_stride<16>()>(r1);
+    conv_layer<8, 16, 32, 32>(r0, fA + kFragL1, a.w + a.off_b[0][1], r1, nullptr);
     __syncthreads();
-    conv_layer<16, 32>(r1, 16, 16, fA + kFragL1 + kFragL2, a.w + a.off_b[0][2], nullptr, feat);
+    conv_layer<16, 32, 16, 16>(r1, fA + kFragL1 + kFragL2, a.w + a.off_b[0][2], nullptr, feat);
     __syncthreads();
     // ---- FC1: warp o computes hidden unit o ----
     {
@@ -740,8 +776,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_clf_infer(Args a) {
       const uint4* wrow = reinterpret_cast<const uint4*>(a.wb1 + (size_t)o * 10240);
       const uint4* x = reinterpret_cast<const uint4*>(feat);
       float sum = 0.f;
+#pragma unroll 8
       for (int i = lane; i < 10240 / 8; i += 32) {
-        const uint4 wv = wrow[i], xv = x[i];
+        const uint4 wv = __ldg(wrow + i), xv = x[i];
         const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w}, xa[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
         for (int q = 0; q < 4; q++) {
