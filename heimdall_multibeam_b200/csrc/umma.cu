@@ -7,14 +7,16 @@
 // A CTA owns tiles of 128 rows of D (the M of one tcgen05.mma) by Npad
 // columns (N rounded up to 16, at most 128), looping over tiles (persistent;
 // grid = min(tiles, 2 per SM)).  K runs in blocks of 64 through a ring of
-// shared-memory stages that TMA fills from 2-D tensor maps, one box of
-// 8 K-elements x rows per 8-wide K chunk, no swizzle: a box lands as the rows'
-// 16-byte core-matrix slices in order, which is the K-major no-swizzle layout
-// tcgen05 reads (stride between 8-row groups SBO = 128 B, between the two
-// K halves of an MMA LBO = rows x 16 B).  Rows and K past the matrix are
-// zero-filled by TMA.  With fewer than 128 rows A's box has only those (the
-// accumulator rows past them are computed from what the stage held and never
-// read: an MMA's rows do not mix).
+// shared-memory stages that TMA fills from 2-D tensor maps, one box of 64 K
+// elements (128 bytes) x rows per operand with the 128-byte swizzle, which is
+// the K-major layout tcgen05 reads (SBO = 1024 B between 8-row groups; an MMA's
+// 16 K elements are 32 bytes further into the swizzled rows).  Rows and K past
+// the matrix are zero-filled by TMA.  With fewer than 128 rows A's box has only
+// those (the accumulator rows past them are computed from what the stage held
+// and never read: an MMA's rows do not mix).
+// What bounds it: the copies' requests, one per row of a box.  Boxes of 8
+// elements (16-byte rows, no swizzle) made eight times as many and took
+// 470 us over a 128-sample training step's GEMMs; 298 us so.
 //
 // Warps 0-3: epilogue (each reads its 32 TMEM lanes with tcgen05.ld and
 // stores its rows); warp 4: TMA producer (one thread); warp 5: allocates the
@@ -64,12 +66,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       :: "r"(smem_addr(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)) : "memory");
 }
 
-// shared-memory matrix descriptor: K-major, no swizzle (layout type 0),
-// version 1, start/LBO/SBO in 16-byte units
-__device__ __forceinline__ uint64_t umma_desc(const void* p, uint32_t lbo, uint32_t sbo) {
+// shared-memory matrix descriptor: K-major, 128-byte swizzle (layout type 2),
+// version 1, start and SBO (8 rows x 128 bytes) in 16-byte units; LBO is not
+// used by a swizzled K-major operand
+__device__ __forceinline__ uint64_t umma_desc(const void* p) {
   const uint64_t a = smem_addr(p);
-  return ((a >> 4) & 0x3FFFull) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+  return ((a >> 4) & 0x3FFFull) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+         (2ull << 61);
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
@@ -101,11 +104,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
     k_umma_gemm(const __grid_constant__ CUtensorMap map_a,
                 const __grid_constant__ CUtensorMap map_b, UmmaArgs g) {
   extern __shared__ __align__(1024) uint8_t um_smem[];
-  // [stage][A: 8 chunks x 128 rows x 16 B][B: 8 chunks x Npad rows x 16 B]
+  // [stage][A: 128 rows x 128 B][B: Npad rows x 128 B], swizzled, 1024-aligned
   uint8_t* base = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(um_smem) + 1023) & ~(uintptr_t)1023);
-  const uint32_t a_chunk = UM_BM * 16, b_chunk = (uint32_t)g.Npad * 16;
-  const uint32_t a_bytes = 8 * a_chunk, stage_bytes = a_bytes + 8 * b_chunk;
+  const uint32_t a_bytes = UM_BM * 128, b_bytes = (uint32_t)g.Npad * 128;
+  const uint32_t stage_bytes = a_bytes + b_bytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(base + UM_ST * stage_bytes);
   uint64_t* empty = full + UM_ST;
   uint64_t* tfull = empty + UM_ST;   // [2] accumulator ready
@@ -157,15 +160,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
             break;
           }
           const int kk = k0 + b * UM_BK;
-          // the K chunks of 8 that the block's MMAs (K = 16 each) read; a
-          // chunk past K is zero-filled by TMA
-          const int nch = 2 * min(4, (g.K - kk + 15) / 16);
-          mbar_expect_tx(&full[s], (uint32_t)nch * ((uint32_t)g.arows * 16 + b_chunk));
+          // (K past the matrix is zero-filled and counted)
+          mbar_expect_tx(&full[s], (uint32_t)g.arows * 128 + b_bytes);
           uint8_t* st = base + (size_t)s * stage_bytes;
-          for (int c = 0; c < nch; c++) {
-            tma_load_2d(st + c * a_chunk, &map_a, kk + 8 * c, mt * UM_BM, &full[s]);
-            tma_load_2d(st + a_bytes + c * b_chunk, &map_b, kk + 8 * c, 0, &full[s]);
-          }
+          tma_load_2d(st, &map_a, kk, mt * UM_BM, &full[s]);
+          tma_load_2d(st + a_bytes, &map_b, kk, 0, &full[s]);
         }
       }
       // every copy issued must land before the thread leaves
@@ -205,8 +204,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
           const int nstep = min(4, (g.K - kk + 15) / 16);
           const uint8_t* st = base + (size_t)s * stage_bytes;
           for (int j = 0; j < nstep; j++) {
-            const uint64_t ad = umma_desc(st + 2 * j * a_chunk, a_chunk, 128);
-            const uint64_t bd = umma_desc(st + a_bytes + 2 * j * b_chunk, b_chunk, 128);
+            const uint64_t ad = umma_desc(st + 32 * j);
+            const uint64_t bd = umma_desc(st + a_bytes + 32 * j);
             umma_bf16(dacc, ad, bd, idesc, accum);
             accum = 1;
           }
@@ -318,17 +317,17 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // 2-D map of a K-major BF16 matrix (rows x K, row pitch ld elements), boxes of
-// 8 elements x box_rows
+// 64 elements x box_rows, 128-byte swizzle
 bool make_map(CUtensorMap* map, const void* ptr, long long rows, long long K, long long ld,
               int box_rows) {
   auto fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {8, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {UM_BK, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
-            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
          CUDA_SUCCESS;
 }
@@ -375,7 +374,7 @@ cudaError_t umma_gemm(int M, int N, int K, const void* A, long long lda, const v
   g.scn = scn;
   g.accumulate = accumulate;
   g.err = err;
-  const size_t stage = (size_t)8 * UM_BM * 16 + (size_t)8 * Npad * 16;
+  const size_t stage = (size_t)(UM_BM + Npad) * 128;
   const size_t smem = 1024 + UM_ST * stage + 8 * (2 * UM_ST + 5) + 16;
   cudaError_t e = raise_smem_limit(k_umma_gemm, smem);
   if (e != cudaSuccess) return e;
