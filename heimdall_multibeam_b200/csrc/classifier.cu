@@ -196,77 +196,246 @@ __global__ void __launch_bounds__(256) k_im2col3(const bf16* __restrict__ in, in
 
 // im2col in K-major order for the tensor-core GEMM: colT [b*h*w][KP], the KP
 // taps of one output pixel contiguous (tap k = c*9 + ky*3 + kx; zeros from
-// ci*9 on).  Bound by its writes.  A thread makes eight taps of one pixel, one
-// 16-byte store, neighbouring threads the next eight: every index is found
-// once per eight values and the stores are whole lines (82 us against 275 us
-// for 8 x 128 x 32 x 128 values in).
+// ci*9 on).  Bound by its writes.  A thread gathers all taps of one pixel: a
+// warp's loads are 32 neighbouring pixels of one tap (with the taps across a
+// warp's lanes each load touched about 20 sectors), and every index but the
+// pixel's is a constant.  The rows go out through shared memory, pitched by an
+// odd number of 16-byte units, so that stores are whole lines: 8 x 128 x 32 x
+// 128 values in took 85 us with the taps across lanes, 57 us with each thread
+// storing its own row, 26 us so.
 template <int CI>
-__global__ void __launch_bounds__(256) k_im2col3_t(const bf16* __restrict__ in, int h, int w,
+__global__ void __launch_bounds__(128) k_im2col3_t(const bf16* __restrict__ in, int h, int w,
                                                    size_t P, bf16* __restrict__ colT) {
-  constexpr int KP = (CI * 9 + 15) / 16 * 16, Q = KP / 8;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P * Q) return;
-  const size_t p = i / Q;
-  const int q = (int)(i % Q);
-  const int x = (int)(p % w), y = (int)((p / w) % h);
-  const uint16_t* src = reinterpret_cast<const uint16_t*>(in) + p;
-  uint32_t v[8];
+  constexpr int KP = (CI * 9 + 15) / 16 * 16, Q = KP / 8, PITCH = Q | 1;
+  __shared__ uint4 rows[128 * PITCH];
+  const size_t p0 = (size_t)blockIdx.x * 128, p = p0 + threadIdx.x;
+  if (p < P) {
+    const int x = (int)(p % w), y = (int)((p / w) % h);
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(in) + p;
+    bool ok[9];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int k = 8 * q + j, c = k / 9, t = k % 9, dy = t / 3 - 1, dx = t % 3 - 1;
-    const bool in_image = k < CI * 9 && y + dy >= 0 && y + dy < h && x + dx >= 0 && x + dx < w;
-    v[j] = in_image ? src[(ptrdiff_t)c * (ptrdiff_t)P + dy * w + dx] : 0u;
-  }
-  reinterpret_cast<uint4*>(colT)[i] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16,
+    for (int t = 0; t < 9; t++) {
+      const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
+      ok[t] = yy >= 0 && yy < h && xx >= 0 && xx < w;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      uint32_t v[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int k = 8 * q + j, c = k / 9, t = k % 9;
+        v[j] = (k < CI * 9 && ok[t])
+                   ? src[(ptrdiff_t)c * (ptrdiff_t)P + (t / 3 - 1) * w + (t % 3 - 1)] : 0u;
+      }
+      rows[threadIdx.x * PITCH + q] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16,
                                                  v[4] | v[5] << 16, v[6] | v[7] << 16);
+    }
+  }
+  __syncthreads();
+  const int n = (int)(P - p0 < 128 ? P - p0 : 128) * Q;
+  uint4* out = reinterpret_cast<uint4*>(colT) + p0 * Q;
+  for (int e = threadIdx.x; e < n; e += 128) out[e] = rows[e / Q * PITCH + e % Q];
 }
 
-// col2im: dcol [kp][b*h*w] (FP32) -> din [ci][b][h][w], summing the 9 taps
-// that read each input pixel
-__global__ void k_col2im3(const float* __restrict__ dcol, int ci, int nb, int h, int w,
-                          float* __restrict__ din) {
-  const size_t P = (size_t)nb * h * w;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P * ci) return;
-  const int c = (int)(i / P);
-  const size_t p = i % P;
-  const int x = (int)(p % w), y = (int)((p / w) % h);
-  const size_t bo = (p / ((size_t)w * h)) * (size_t)w * h;
-  float sum = 0.f;
-#pragma unroll
-  for (int ky = 0; ky < 3; ky++)
-#pragma unroll
-    for (int kx = 0; kx < 3; kx++) {
-      // output pixel (y - ky + 1, x - kx + 1) read this input through tap (ky, kx)
-      const int yo = y - ky + 1, xo = x - kx + 1;
-      if (yo >= 0 && yo < h && xo >= 0 && xo < w)
-        sum += dcol[(size_t)(c * 9 + ky * 3 + kx) * P + bo + (size_t)yo * w + xo];
+// Data gradient of a convolution, straight from the layer's pre-activation
+// gradient dz [CO][b][H][W] (BF16) to its input's gradient din [CI][b][H][W]:
+// for each tap the product over the output channels (mma.sync m16n8k16, FP32),
+// the nine taps added in order, as a GEMM to dcol [CI*9][b*H*W] and a col2im
+// did through 168 MB of dcol.  A block takes R rows of one sample and stages
+// their dz and a ring of zeros pixel-major in shared memory; a warp's 16 MMA
+// rows are 16 neighbouring pixels, read shifted by each tap, and the weights'
+// fragments stay in registers.  Bound by dz and din in memory, not by the
+// product (K = 16 or 32).  The four layers of a 128-sample step: 354 us for the
+// GEMMs and the col2ims, 63 us here (8 -> 16 channels of 32 x 128: 25 us).
+template <int CI, int CO, int H, int W, int R>
+__global__ void __launch_bounds__(256) k_dgrad3(const bf16* __restrict__ dz,
+                                                const bf16* __restrict__ wb, size_t P,
+                                                float* __restrict__ din) {
+  constexpr int KP = (CI * 9 + 15) / 16 * 16;
+  constexpr int NT = CI / 8, KS = CO / 16, PS = CO + 8, Wp = W + 2;
+  extern __shared__ __align__(16) uint32_t dg_smem[];  // [R + 2][Wp][PS] BF16
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int n = blockIdx.x / (H / R), y0 = blockIdx.x % (H / R) * R;
+  // zero columns left and right; rows outside the image are zeroed below
+  for (int e = threadIdx.x; e < (R + 2) * 2 * (PS / 2); e += 256) {
+    const int r = e / (PS), o = e % PS;
+    dg_smem[(r * Wp + (o < PS / 2 ? 0 : W + 1)) * (PS / 2) + o % (PS / 2)] = 0u;
+  }
+  // lane: channel pair cp, pixel group (8 pixels) gr
+  constexpr int CPN = CO / 2, GR = 32 / CPN;  // pairs, groups per warp step
+  const int cp = lane % CPN, gr = lane / CPN;
+  for (int it = warp; it < (R + 2) * (W / 8 / GR); it += 8) {
+    const int r = it / (W / 8 / GR), x8 = (it % (W / 8 / GR)) * GR + gr;
+    const int y = y0 + r - 1;
+    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+    if (y >= 0 && y < H) {
+      const bf16* src = dz + (size_t)(2 * cp) * P + ((size_t)n * H + y) * W + 8 * x8;
+      a = *reinterpret_cast<const uint4*>(src);
+      b = *reinterpret_cast<const uint4*>(src + P);
     }
-  din[i] = sum;
+    uint32_t v[8];
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      v[2 * j] = __byte_perm(aw[j], bw[j], 0x5410);
+      v[2 * j + 1] = __byte_perm(aw[j], bw[j], 0x7632);
+    }
+    uint32_t* d = dg_smem + (size_t)(r * Wp + 1 + 8 * x8) * (PS / 2) + cp;
+#pragma unroll
+    for (int j = 0; j < 8; j++) d[j * (PS / 2)] = v[j];
+  }
+  // weights: fragment (k = output channel, n = input channel) of every tap
+  uint2 frag[9][KS][NT];
+#pragma unroll
+  for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+    for (int s = 0; s < KS; s++)
+#pragma unroll
+      for (int j = 0; j < NT; j++) {
+        const uint16_t* wp = reinterpret_cast<const uint16_t*>(wb) + (8 * j + g) * 9 + tap;
+        const int k = 16 * s + 2 * t;
+        frag[tap][s][j].x = wp[k * KP] | (uint32_t)wp[(k + 1) * KP] << 16;
+        frag[tap][s][j].y = wp[(k + 8) * KP] | (uint32_t)wp[(k + 9) * KP] << 16;
+      }
+  __syncthreads();
+  for (int tile = warp; tile < R * W / 16; tile += 8) {
+    const int r = tile / (W / 16), x0 = (tile % (W / 16)) * 16;
+    float sum[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; j++) sum[j][0] = sum[j][1] = sum[j][2] = sum[j][3] = 0.f;
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++) {
+      // input pixel (y, x) was read through tap (ky, kx) by output pixel
+      // (y - ky + 1, x - kx + 1); +1 each for the ring
+      const int rr = r + 2 - tap / 3, xx = x0 + 2 - tap % 3;
+      const uint32_t* p = dg_smem + (size_t)(rr * Wp + xx + g) * (PS / 2) + t;
+      float acc[NT][4];
+#pragma unroll
+      for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+#pragma unroll
+      for (int s = 0; s < KS; s++) {
+        const uint32_t a[4] = {p[8 * s], p[8 * (PS / 2) + 8 * s], p[8 * s + 4],
+                               p[8 * (PS / 2) + 8 * s + 4]};
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+          const uint32_t b[2] = {frag[tap][s][j].x, frag[tap][s][j].y};
+          mma_bf16(acc[j], a, b);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) sum[j][q] = __fadd_rn(sum[j][q], acc[j][q]);
+    }
+    float* o = din + ((size_t)n * H + y0 + r) * W + x0 + g;
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      const size_t c = 8 * j + 2 * t;
+      o[c * P] = sum[j][0];
+      o[(c + 1) * P] = sum[j][1];
+      o[c * P + 8] = sum[j][2];
+      o[(c + 1) * P + 8] = sum[j][3];
+    }
+  }
+}
+
+template <int CI, int CO, int H, int W, int R>
+cudaError_t launch_dgrad3(const bf16* dz, const bf16* wb, int nb, float* din, cudaStream_t s) {
+  constexpr size_t smem = (size_t)(R + 2) * (W + 2) * (CO + 8) * sizeof(bf16);
+  auto kern = k_dgrad3<CI, CO, H, W, R>;
+  cudaError_t e = raise_smem_limit(kern, smem);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)nb * (H / R), 256, smem, s>>>(dz, wb, (size_t)nb * H * W, din); note_launch();
+  return cudaGetLastError();
+}
+
+// FC1 weight gradient: g [16][10240] += sum over the batch of dz1 [16][b] x
+// x [b][10240].  A thread takes two features of a quarter of the samples, 64
+// at a time with the 16 gradients in shared memory; the quarters are added in
+// order.  For 128 samples 33 us as a GEMM of 32 x 64 tiles, 28 us with one
+// thread for all samples (two warps a block: bound by its loads' latency),
+// 11 us so.
+__global__ void __launch_bounds__(256) k_fc1_wgrad(const bf16* __restrict__ dz1,
+                                                   const bf16* __restrict__ x, int nb,
+                                                   float* __restrict__ g) {
+  constexpr int FC_PART = 64;
+  __shared__ float d[FC_PART][16];
+  __shared__ float2 part[3][16][64];
+  const int l = threadIdx.x % 64, q = threadIdx.x / 64;
+  const int f = 2 * (blockIdx.x * 64 + l);
+  float acc[16][2];
+#pragma unroll
+  for (int o = 0; o < 16; o++) acc[o][0] = acc[o][1] = 0.f;
+  for (int n0 = 0; n0 < nb; n0 += FC_PART) {
+    const int m = min(FC_PART, nb - n0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 16 * m; e += 256) {
+      const int o = e / m, n = e % m;
+      d[n][o] = __bfloat162float(dz1[(size_t)o * nb + n0 + n]);
+    }
+    __syncthreads();
+    const int end = min(m, (q + 1) * (FC_PART / 4));
+#pragma unroll 8
+    for (int n = q * (FC_PART / 4); n < end; n++) {
+      const float2 v = __bfloat1622float2(
+          *reinterpret_cast<const __nv_bfloat162*>(x + (size_t)(n0 + n) * 10240 + f));
+#pragma unroll
+      for (int o = 0; o < 16; o++) {
+        acc[o][0] = __fmaf_rn(d[n][o], v.x, acc[o][0]);
+        acc[o][1] = __fmaf_rn(d[n][o], v.y, acc[o][1]);
+      }
+    }
+  }
+  if (q > 0)
+#pragma unroll
+    for (int o = 0; o < 16; o++) part[q - 1][o][l] = make_float2(acc[o][0], acc[o][1]);
+  __syncthreads();
+  if (q > 0) return;
+#pragma unroll
+  for (int o = 0; o < 16; o++) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      acc[o][0] = __fadd_rn(acc[o][0], part[k][o][l].x);
+      acc[o][1] = __fadd_rn(acc[o][1], part[k][o][l].y);
+    }
+    float2* p = reinterpret_cast<float2*>(g + (size_t)o * 10240 + f);
+    const float2 old = *p;
+    *p = make_float2(__fadd_rn(old.x, acc[o][0]), __fadd_rn(old.y, acc[o][1]));
+  }
 }
 
 // conv output [co][b][h][w] (FP32) + bias -> ReLU -> 2x2 max pool ->
-// act [co][b][h/2][w/2] (BF16), arg = position of the maximum (0..3)
-__global__ void k_bias_relu_pool(const float* __restrict__ z, const float* __restrict__ bias,
-                                 int co, int nb, int h, int w, bf16* __restrict__ act,
-                                 unsigned char* __restrict__ arg) {
-  const int h2 = h / 2, w2 = w / 2;
-  const size_t n = (size_t)co * nb * h2 * w2;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int x2 = (int)(i % w2), y2 = (int)((i / w2) % h2);
-  const size_t cb = i / ((size_t)w2 * h2);  // c * nb + b
-  const int c = (int)(cb / nb);
-  const float* zp = z + cb * (size_t)h * w;
-  float best = -INFINITY;
-  int bi = 0;
+// act [co][b][h/2][w/2] (BF16), arg = position of the maximum (0..3).  Bound by
+// its reads; a thread takes two pooled elements of a row (16-byte loads).
+__global__ void __launch_bounds__(256) k_bias_relu_pool(const float* __restrict__ z,
+                                                        const float* __restrict__ bias, int nb,
+                                                        int h, int w, bf16* __restrict__ act,
+                                                        unsigned char* __restrict__ arg) {
+  const int c = blockIdx.y, q2 = w / 4;              // pairs of a pooled row
+  const unsigned i = blockIdx.x * 256 + threadIdx.x;  // pair of this channel
+  if (i >= (unsigned)(nb * (h / 2) * q2)) return;
+  const unsigned x4 = i % q2, row = i / q2;           // row = n * h/2 + y2
+  const float* zp = z + ((size_t)c * nb * h + 2 * (size_t)row) * w + 4 * x4;
+  const float4 a = *reinterpret_cast<const float4*>(zp), b = *reinterpret_cast<const float4*>(zp + w);
+  const float v[2][4] = {{a.x, a.y, b.x, b.y}, {a.z, a.w, b.z, b.w}};
+  const float bc = bias[c];
+  uint32_t o = 0, g = 0;
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const float v = fmaxf(zp[(size_t)(2 * y2 + (q >> 1)) * w + 2 * x2 + (q & 1)] + bias[c], 0.f);
-    if (v > best) { best = v; bi = q; }
+  for (int k = 0; k < 2; k++) {
+    float best = -INFINITY;
+    int bi = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float x = fmaxf(v[k][q] + bc, 0.f);
+      if (x > best) { best = x; bi = q; }
+    }
+    o |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16(best)) << (16 * k);
+    g |= (uint32_t)bi << (8 * k);
   }
-  act[i] = __float2bfloat16(best);
-  arg[i] = (unsigned char)bi;
+  const size_t j = (size_t)c * nb * (h / 2) * (w / 2) + 2 * (size_t)i;
+  *reinterpret_cast<uint32_t*>(act + j) = o;
+  *reinterpret_cast<uint16_t*>(arg + j) = (uint16_t)g;
 }
 
 // backward of bias/ReLU/pool: dact [co][b][h/2][w/2] (FP32) -> dz [co][b][h][w]
@@ -434,6 +603,12 @@ __global__ void __launch_bounds__(256) k_head_reduce(const float* __restrict__ h
                                                      float* __restrict__ gb1) {
   __shared__ float sh[kHeadChunk * 16], st[kHeadChunk * kHeadTerms];
   const int k = threadIdx.x;  // 0: loss, 1-2: gb2, 3-34: gw2, 35-50: gb1
+  // every output's term is +-(one of the sample's terms) times 1 or one of its
+  // hidden units, so that no thread branches in the loop (dL/dl0 = -dL/dl1)
+  const int term = k == 0 ? 0 : k < 35 ? 1 : k - 33;
+  const float sign = k == 1 || (k >= 3 && k < 19) ? -1.f : 1.f;
+  const bool hidden = k >= 3 && k < 35;
+  const int unit = hidden ? (k - 3) % 16 : 0;
   float acc = 0.f;
   for (int n0 = 0; n0 < nb; n0 += kHeadChunk) {
     const int m = min(kHeadChunk, nb - n0);
@@ -442,17 +617,10 @@ __global__ void __launch_bounds__(256) k_head_reduce(const float* __restrict__ h
     for (int i = k; i < m * kHeadTerms; i += 256) st[i] = hs[(size_t)n0 * kHeadTerms + i];
     __syncthreads();
     if (k > 50) continue;
+#pragma unroll 8
     for (int n = 0; n < m; n++) {
-      const float* t = st + n * kHeadTerms;
-      const float d1 = t[1], d0 = -d1;
-      float v;
-      if (k == 0) v = t[0];
-      else if (k == 1) v = d0;
-      else if (k == 2) v = d1;
-      else if (k < 19) v = d0 * sh[n * 16 + (k - 3)];
-      else if (k < 35) v = d1 * sh[n * 16 + (k - 19)];
-      else v = t[2 + (k - 35)];
-      acc = __fadd_rn(acc, v);
+      const float hv = hidden ? sh[n * 16 + unit] : 1.f;
+      acc = __fadd_rn(acc, __fmul_rn(sign * st[n * kHeadTerms + term], hv));
     }
   }
   if (k == 0) loss[0] = __fadd_rn(loss[0], acc);
@@ -1015,7 +1183,7 @@ struct hd_classifier_t {
   long long step = 0;
   // per-batch work buffers
   int cap_batch = 0;
-  DBuf in[2], col, z, act[2][3], arg[2][3], dz, dcol, dact_a[2], dact_b[2], x, z1, h, dz1,
+  DBuf in[2], col, z, act[2][3], arg[2][3], dz, in_f32, dact_a[2], dact_b[2], x, z1, h, dz1,
       dx, prob, loss, labels, idx, hs, bias_part;
   DBuf tc_ws, tc_err;               // tensor-core GEMM: split-K workspace, error word
   DBuf data_dm, data_ft, data_lab;  // resident training set
@@ -1057,7 +1225,6 @@ cudaError_t alloc_batch(hd_classifier c, int nb) {
   CK(c->in[0].ensure((size_t)nb * 64 * 64 * sizeof(bf16)));
   CK(c->in[1].ensure((size_t)nb * 64 * 256 * sizeof(bf16)));
   CK(c->col.ensure(maxcol * sizeof(bf16)));
-  CK(c->dcol.ensure(maxcol * sizeof(float)));
   CK(c->z.ensure(maxz * sizeof(float)));
   CK(c->dz.ensure(maxz * sizeof(bf16)));
   for (int br = 0; br < 2; br++) {
@@ -1127,12 +1294,12 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
       // colT [P][kp] x W^T, M = P pixels, N = co, K = kp
       const auto im2col = sp.ci == 1 ? k_im2col3_t<1> : sp.ci == 8 ? k_im2col3_t<8>
                                                                    : k_im2col3_t<16>;
-      im2col<<<nblk(P * sp.kp() / 8), 256, 0, s>>>(cur, sp.h, sp.w, P, c->col.as<bf16>()); hdb::note_launch();
+      im2col<<<nblk(P, 128), 128, 0, s>>>(cur, sp.h, sp.w, P, c->col.as<bf16>()); hdb::note_launch();
       CK(tc_gemm(c, (int)P, sp.co, sp.kp(), c->col.as<bf16>(), sp.kp(),
                  c->wb_conv[br][l].as<bf16>(), sp.kp(), c->z.as<float>(), 1, (long long)P, 0,
                  1));
-      k_bias_relu_pool<<<nblk(P / 4 * sp.co), 256, 0, s>>>(
-          c->z.as<float>(), w + c->off_b[br][l], sp.co, nb, sp.h, sp.w,
+      k_bias_relu_pool<<<dim3(nblk(P / 8), sp.co), 256, 0, s>>>(
+          c->z.as<float>(), w + c->off_b[br][l], nb, sp.h, sp.w,
           c->act[br][l].as<bf16>(), c->arg[br][l].as<unsigned char>()); hdb::note_launch();
       cur = c->act[br][l].as<bf16>();
     }
@@ -1155,10 +1322,8 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
                                  g + c->off_w2, g + c->off_b2, g + c->off_b1); hdb::note_launch();
   // ---- backward ----
   {
-    // dW1 [16][10240] += dz1 [16][b] x x [b][10240]
-    GemmArgs ga{kHid, kFeat, nb, c->dz1.as<bf16>(), nb, 1, c->x.as<bf16>(), kFeat, 1,
-                g + c->off_w1, kFeat, 1, 1, 0};
-    CK(gemm(ga, 1, s));
+    k_fc1_wgrad<<<kFeat / 128, 256, 0, s>>>(c->dz1.as<bf16>(), c->x.as<bf16>(), nb,
+                                           g + c->off_w1); hdb::note_launch();
     // dx [b][10240] = dz1^T x W1
     GemmArgs gd{kFeat, nb, kHid, c->wb1.as<bf16>(), 1, kFeat, c->dz1.as<bf16>(), nb, 1,
                 c->dx.as<float>(), 1, kFeat, 0, 0};
@@ -1188,8 +1353,7 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
       const bf16* lin = l == 0 ? c->in[br].as<bf16>() : c->act[br][l - 1].as<bf16>();
       k_im2col3<<<dim3(nblk(P / 8), sp.ci), 256, 0, s>>>(lin, sp.h, sp.w, P,
                                                          c->col.as<bf16>()); hdb::note_launch();
-      // dW [co][kw] += dz [co][P] x col^T; the padded columns kw..kp are dropped
-      // by writing into a [co][kp] scratch is avoided: N = kw with row stride kw
+      // dW [co][kw] += dz [co][P] x col^T, without the padded taps kw..kp:
       // on the tensor cores as dW^T [kw][co] += col [kw][P] x dz^T: M = kw
       // taps, N = co, K = P pixels split over the SMs; the splits are added
       // in order (the same gradient every run)
@@ -1197,12 +1361,13 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
       CK(tc_gemm(c, sp.kw(), sp.co, (int)P, c->col.as<bf16>(), (long long)P, c->dz.as<bf16>(),
                  (long long)P, g + c->off_w[br][l], 1, sp.kw(), 1, splits));
       if (l > 0) {
-        // dcol [kp][P] = W^T x dz, then col2im into the previous layer's output gradient
-        GemmArgs gd{sp.kp(), (int)P, sp.co, c->wb_conv[br][l].as<bf16>(), 1, sp.kp(),
-                    c->dz.as<bf16>(), (long long)P, 1, c->dcol.as<float>(), (long long)P, 1, 0, 0};
-        CK(gemm(gd, 1, s));
-        k_col2im3<<<nblk(P * sp.ci), 256, 0, s>>>(c->dcol.as<float>(), sp.ci, nb, sp.h, sp.w,
-                                                 dnext); hdb::note_launch();
+        // the gradient of the previous layer's output
+        const bf16* dz = c->dz.as<bf16>();
+        const bf16* wb = c->wb_conv[br][l].as<bf16>();
+        CK(br == 0 ? (l == 1 ? launch_dgrad3<8, 16, 32, 32, 8>(dz, wb, nb, dnext, s)
+                             : launch_dgrad3<16, 32, 16, 16, 16>(dz, wb, nb, dnext, s))
+                   : (l == 1 ? launch_dgrad3<8, 16, 32, 128, 4>(dz, wb, nb, dnext, s)
+                             : launch_dgrad3<16, 32, 16, 64, 4>(dz, wb, nb, dnext, s)));
         std::swap(dcur, dnext);
       }
     }
@@ -1214,13 +1379,13 @@ cudaError_t run_batch(hd_classifier c, int nb, bool backward) {
 
 cudaError_t upload_patches(hd_classifier c, const float* dm, const float* ft, int nb) {
   cudaStream_t s = c->stream;
-  // host floats -> device BF16 through a temporary FP32 copy in dcol
-  CK(c->dcol.ensure((size_t)nb * 16384 * sizeof(float)));
-  CK(cudaMemcpyAsync(c->dcol.p, dm, (size_t)nb * 4096 * sizeof(float), cudaMemcpyHostToDevice, s));
-  k_input_bf16<<<nblk((size_t)nb * 4096), 256, 0, s>>>(c->dcol.as<float>(), c->in[0].as<bf16>(),
+  // host floats -> device BF16 through a temporary FP32 copy
+  CK(c->in_f32.ensure((size_t)nb * 16384 * sizeof(float)));
+  CK(cudaMemcpyAsync(c->in_f32.p, dm, (size_t)nb * 4096 * sizeof(float), cudaMemcpyHostToDevice, s));
+  k_input_bf16<<<nblk((size_t)nb * 4096), 256, 0, s>>>(c->in_f32.as<float>(), c->in[0].as<bf16>(),
                                                        (size_t)nb * 4096); hdb::note_launch();
-  CK(cudaMemcpyAsync(c->dcol.p, ft, (size_t)nb * 16384 * sizeof(float), cudaMemcpyHostToDevice, s));
-  k_input_bf16<<<nblk((size_t)nb * 16384), 256, 0, s>>>(c->dcol.as<float>(), c->in[1].as<bf16>(),
+  CK(cudaMemcpyAsync(c->in_f32.p, ft, (size_t)nb * 16384 * sizeof(float), cudaMemcpyHostToDevice, s));
+  k_input_bf16<<<nblk((size_t)nb * 16384), 256, 0, s>>>(c->in_f32.as<float>(), c->in[1].as<bf16>(),
                                                         (size_t)nb * 16384); hdb::note_launch();
   return cudaGetLastError();
 }
