@@ -435,8 +435,8 @@ cudaError_t rms_beams(const SeriesBatch& sb, float* rms, TreeScratch& ws, cudaSt
 //                chain over one stage of its row in shared memory;
 //   warps 1..np  a stage's rows arrive by TMA bulk copies requested SC_DEPTH
 //                stages ahead; these warps divide them in place by their
-//                beam's RMS, and write them out once the chain warp has
-//                replaced them with their prefix sums.
+//                beam's RMS, and write their prefix sums out once the chain
+//                warp has left every fourth of them in the row.
 // Stage k lives in buffer k % SC_NB.  At step k the producers normalise stage
 // k and store stage k - 2 while the chain warp scans stage k - 1, and stage
 // k + SC_DEPTH is requested into the buffer that held stage k - 3 (stored at
@@ -458,13 +458,21 @@ constexpr uint32_t SC_WAIT_LIMIT = 1u << 22;
 // theorem needs the quotient and residual clear of underflow and overflow,
 // which |a|, |b| in [2^-40, 2^40] guarantees; other operands (zeros, tiny,
 // huge and non-finite values) take __fdiv_rn.
+__device__ __forceinline__ float div_rn_in_range(float a, float b, float y) {
+  const float q0 = __fmul_rn(a, y);
+  const float r = __fmaf_rn(-b, q0, a);
+  return __fmaf_rn(r, y, q0);
+}
+
+// |v|'s bits above those of 2^-40: at most kDivSpan for |v| in [2^-40, 2^40],
+// more for all else (smaller values wrap around)
+constexpr unsigned kDivLow = 0x2B800000u, kDivSpan = 0x53800000u - kDivLow;
+__device__ __forceinline__ unsigned div_range(float v) {
+  return (__float_as_uint(v) & 0x7FFFFFFFu) - kDivLow;
+}
+
 __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
-  const float aa = fabsf(a), ab = fabsf(b);
-  if (aa >= 0x1p-40f && aa <= 0x1p40f && ab >= 0x1p-40f && ab <= 0x1p40f) {
-    const float q0 = __fmul_rn(a, y);
-    const float r = __fmaf_rn(-b, q0, a);
-    return __fmaf_rn(r, y, q0);
-  }
+  if (div_range(a) <= kDivSpan && div_range(b) <= kDivSpan) return div_rn_in_range(a, b, y);
   return __fdiv_rn(a, b);
 }
 
@@ -542,47 +550,34 @@ __global__ void __launch_bounds__(CH >= 512 ? 160 : 256, CH >= 512 ? 3 : 4) k_no
       // ---- the chains: stage k - 1 ----
       if (k >= 1 && k - 1 < nstage && lane < nb) {
         float* row = rows + ((size_t)((k - 1) % SC_NB) * S + lane) * ROW;
-        if constexpr (CH >= 512) {
-          // blocks of few series: the next 32 samples are loaded before the
-          // current ones are added, so the chain waits for its adds only (one
-          // series of 262144 samples: 0.67 ms against 0.75).  Takes 112
-          // registers, which the blocks of 8 series (CH = 256) don't have:
-          // there it spills and the headline gulp's scan slows from 0.50 to
-          // 0.73 ms.
-          constexpr int AH = 8;
-          float4 cur[AH], nxt[AH];
+        // The next 4*AH samples are loaded before the current ones are added,
+        // so that the chain waits for its adds only.  Of four prefix sums the
+        // lane stores the first, in the place of the fourth sample (which only
+        // the chain needs); the warp that stores the stage adds the other
+        // three again.  Cycles a sample of one chain by itself, its adds being
+        // 4.2: 5.9 with 16-byte stores of all four and AH = 8, 4.6 so (4.8 with
+        // AH = 4, which the 64 registers of the 8-series blocks allow).
+        constexpr int AH = CH >= 512 ? 8 : 4;
+        float4 cur[AH], nxt[AH];
 #pragma unroll
-          for (int j = 0; j < AH; j++) cur[j] = *reinterpret_cast<const float4*>(row + 4 * j);
+        for (int j = 0; j < AH; j++) cur[j] = *reinterpret_cast<const float4*>(row + 4 * j);
 #pragma unroll 2
-          for (int e = 0; e < CH; e += 4 * AH) {
-            // past the row's end the last values again (never added)
-            const float* ahead = row + min(e + 4 * AH, CH - 4 * AH);
+        for (int e = 0; e < CH; e += 4 * AH) {
+          // past the row's end the last values again (never added)
+          const float* ahead = row + min(e + 4 * AH, CH - 4 * AH);
 #pragma unroll
-            for (int j = 0; j < AH; j++) nxt[j] = *reinterpret_cast<const float4*>(ahead + 4 * j);
+          for (int j = 0; j < AH; j++) nxt[j] = *reinterpret_cast<const float4*>(ahead + 4 * j);
 #pragma unroll
-            for (int j = 0; j < AH; j++) {
-              const float4 v = cur[j];
-              float4 o;
-              o.x = sum; sum = __fadd_rn(sum, v.x);
-              o.y = sum; sum = __fadd_rn(sum, v.y);
-              o.z = sum; sum = __fadd_rn(sum, v.z);
-              o.w = sum; sum = __fadd_rn(sum, v.w);
-              *reinterpret_cast<float4*>(row + e + 4 * j) = o;
-            }
-#pragma unroll
-            for (int j = 0; j < AH; j++) cur[j] = nxt[j];
+          for (int j = 0; j < AH; j++) {
+            const float4 v = cur[j];
+            row[e + 4 * j + 3] = sum;
+            sum = __fadd_rn(sum, v.x);
+            sum = __fadd_rn(sum, v.y);
+            sum = __fadd_rn(sum, v.z);
+            sum = __fadd_rn(sum, v.w);
           }
-        } else {
-  #pragma unroll 8
-          for (int e = 0; e < CH; e += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(row + e);
-            float4 o;
-            o.x = sum; sum = __fadd_rn(sum, v.x);
-            o.y = sum; sum = __fadd_rn(sum, v.y);
-            o.z = sum; sum = __fadd_rn(sum, v.z);
-            o.w = sum; sum = __fadd_rn(sum, v.w);
-            *reinterpret_cast<float4*>(row + e) = o;
-          }
+#pragma unroll
+          for (int j = 0; j < AH; j++) cur[j] = nxt[j];
         }
       }
     } else {
@@ -598,7 +593,13 @@ __global__ void __launch_bounds__(CH >= 512 ? 160 : 256, CH >= 512 ? 3 : 4) k_no
           for (int q = 0; q < QN; q++) {
             const unsigned e = 4u * lane + 128u * q;
             const unsigned i = st * CH + e;
-            const float4 v = *reinterpret_cast<const float4*>(rrow + e);
+            // the chain's sum before these samples stands in the fourth
+            const float4 x = *reinterpret_cast<const float4*>(rrow + e);
+            float4 v;
+            v.x = x.w;
+            v.y = __fadd_rn(v.x, x.x);
+            v.z = __fadd_rn(v.y, x.y);
+            v.w = __fadd_rn(v.z, x.z);
             float* o = orow + i;
             if (i + 3 <= len) {
               *reinterpret_cast<float4*>(o) = v;
@@ -632,12 +633,32 @@ __global__ void __launch_bounds__(CH >= 512 ? 160 : 256, CH >= 512 ? 3 : 4) k_no
             float4 x[QN];
 #pragma unroll
             for (int q = 0; q < QN; q++) x[q] = *reinterpret_cast<const float4*>(crow + 4 * lane + 128 * q);
+            // one test for all of a lane's values: a branch at each of them
+            // kept their divisions from overlapping
+            unsigned far = div_range(rb);
+#pragma unroll
+            for (int q = 0; q < QN; q++)
+              far = max(max(far, max(div_range(x[q].x), div_range(x[q].y))),
+                        max(div_range(x[q].z), div_range(x[q].w)));
+            if (far <= kDivSpan) {
+#pragma unroll
+              for (int q = 0; q < QN; q++) {
+                x[q].x = div_rn_in_range(x[q].x, rb, y);
+                x[q].y = div_rn_in_range(x[q].y, rb, y);
+                x[q].z = div_rn_in_range(x[q].z, rb, y);
+                x[q].w = div_rn_in_range(x[q].w, rb, y);
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < QN; q++) {
+                x[q].x = div_rn_by(x[q].x, rb, y);
+                x[q].y = div_rn_by(x[q].y, rb, y);
+                x[q].z = div_rn_by(x[q].z, rb, y);
+                x[q].w = div_rn_by(x[q].w, rb, y);
+              }
+            }
 #pragma unroll
             for (int q = 0; q < QN; q++) {
-              x[q].x = div_rn_by(x[q].x, rb, y);
-              x[q].y = div_rn_by(x[q].y, rb, y);
-              x[q].z = div_rn_by(x[q].z, rb, y);
-              x[q].w = div_rn_by(x[q].w, rb, y);
               *reinterpret_cast<float4*>(crow + 4 * lane + 128 * q) = x[q];
               if (norm_out)
                 *reinterpret_cast<float4*>(norm_out + (size_t)(s0 + sl) * pitch + base + 4 * lane +
