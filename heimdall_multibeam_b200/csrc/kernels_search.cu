@@ -897,160 +897,162 @@ __global__ void k_block_rms_pass1_multi(WidthCtx ctx, int w0, int nwb, int m, in
   }
 }
 
-// Pass 1 for several unscrunched widths, one median level of every width per
-// block barrier.  Level 1 works on runs of 4 consecutive medians (20
-// consecutive samples): with the boxcar offset a multiple of 4, both ends of a
-// width >= 8 boxcar are 16-byte aligned in the staged window and load as
-// float4 (a thread stride of 80 bytes keeps the 8 lanes of each access phase
-// on distinct banks); widths 1, 2 and 4 read one 28-value window.
+// Pass 1 for several unscrunched widths.  A lane takes 25 consecutive samples of
+// one width and folds them to a second-level median in registers: 50 loads of
+// the staged window at a lane stride of 25 words, which no two lanes' banks
+// share, and no level-1 medians in shared memory.  Widths 1, 2, 4 and 8 share
+// one 33-value window.
 constexpr int BRV_THREADS = 512;  // at most 16 warps: one per boxcar width
+constexpr int BRV_MAXW = 32;  // width slots with a group maximum
+constexpr int BRV_GPB = 8;    // groups of a block at most
 constexpr int VH_MAXW = 16;  // unscrunched widths the vector kernels handle at once
 
-template <int AH, int BH>
-__device__ __forceinline__ void brv_small(const float* win, float* v) {
-#pragma unroll
-  for (int r = 0; r < 20; r++) v[r] = fabsf(__fsub_rn(win[4 + r + AH], win[4 + r - BH]));
+// Three-input min and max: one instruction each on sm_100.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 
+// Median of 5, and *top raised to the largest.  MM: without NaN among them, the
+// two middle values of a..d are lo and hi = min(M1, M2) in some order, and the
+// median is that of lo, hi and e: the largest of their pairwise minima.
 template <bool MM>
-__device__ __forceinline__ float brv_med5(float a, float b, float c, float d, float e) {
-  return MM ? med5_mm(a, b, c, d, e) : med5(a, b, c, d, e);
-}
-
-__device__ __forceinline__ float max5(float a, float b, float c, float d, float e) {
-  return fmaxf(fmaxf(fmaxf(a, b), fmaxf(c, d)), e);
+__device__ __forceinline__ float brv_med5(float a, float b, float c, float d, float e, float* top) {
+  const float M1 = fmaxf(a, b), M2 = fmaxf(c, d);
+  *top = max3(*top, e, fmaxf(M1, M2));
+  if (!MM) return med5(a, b, c, d, e);
+  const float lo = fmaxf(fminf(a, b), fminf(c, d));
+  return max3(min3(lo, M1, M2), fminf(lo, e), min3(M1, M2, e));
 }
 
 __host__ __device__ constexpr int pow5c(int k) { return k <= 0 ? 1 : 5 * pow5c(k - 1); }
 
-// The median levels of one group for every width slot, M levels in the block
-// (compile-time).  Warp w takes width slots w, w + nwarps, ... (the launcher
-// gives a block one warp per slot, up to 16), and each slot's work -- level
-// 1 over the staged window, levels 2..M in the slot's own rows of la and lb,
-// and the group maximum -- stays inside its warp: branches are uniform, and
-// no block barrier is needed until the next group's window.
+// Lane runs (25 samples) of one group, and the warp steps over them.
+__host__ __device__ constexpr int brv_runs(int m) { return pow5c(m - 2); }
+__host__ __device__ constexpr int brv_steps(int m) { return (brv_runs(m) + 31) / 32; }
+constexpr int BRV_SMALL = 4;  // widths 1, 2, 4, 8: one window, one warp
+
+// Median of the five medians of 25 boxcar magnitudes val(0..24); *top is raised
+// to the largest.
+template <bool MM, class F>
+__device__ __forceinline__ float brv_fold(F val, float* top) {
+  float m[5], none = 0.f;
+#pragma unroll
+  for (int j = 0; j < 5; j++) {
+    float v[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) v[k] = fabsf(val(5 * j + k));
+    m[j] = brv_med5<MM>(v[0], v[1], v[2], v[3], v[4], top);
+  }
+  return brv_med5<MM>(m[0], m[1], m[2], m[3], m[4], &none);
+}
+
+// The largest value of a width slot's step to smax[wl].  Values are
+// non-negative or NaN, so their bit patterns order as unsigned; fmaxf drops a
+// NaN unless all its operands are NaN, and no sample is then left out of a
+// maximum that decides a skip: a NaN boxcar never passes the test.
+__device__ __forceinline__ void brv_top(float top, unsigned* smax, int wl, int lane) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+  if (lane == 0) atomicMax(&smax[wl], m);
+}
+
+// Levels 1 and 2 of one group, whose first sample is at `tile`, for every width
+// slot, to l2 [nwb][brv_runs(M)].  The work is cut into steps of 32 runs of one width, the four small
+// widths' step counting as four, and dealt out so that the warps (one per slot)
+// get equal shares.
 template <bool MM, int M>
-__device__ void brv_levels(const WidthCtx& ctx, const float* tile, int offset, int w0, int nwb,
-                           float* la, float* lb, float* __restrict__ out, size_t out_pitch,
-                           size_t ser, size_t g, float* srun, bool rec) {
-  constexpr int n1 = pow5c(M - 1);
-  constexpr int n1p = (n1 + 3) & ~3;
-  constexpr int lbp = n1 / 5 + 1;
-  // srun[wl][q]: largest |boxcar| of level-1 item q of width slot wl (runs of
-  // 20 samples, then the < 4 remaining single medians)
-  constexpr int nq = n1 / 4, rem = n1 - 4 * nq;
-  constexpr int rp = nq + 4;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = blockDim.x >> 5;
-  for (int wl = threadIdx.x >> 5; wl < nwb; wl += nwarps) {
-    const int wi = w0 + wl;
-    float* la_w = la + wl * n1p;
-    float* srun_w = srun + wl * rp;
-
-    // ---- level 1: runs of 4 medians (20 consecutive samples) per lane ----
-    if (wi < 3) {
-      for (int q = lane; q < nq; q += 32) {
-        const int k0 = 4 * q;
-        float v[20], wv[28];
-        const float4* p = reinterpret_cast<const float4*>(tile + 5 * k0 + offset - 4);
+__device__ __forceinline__ void brv_level12(const float* tile, int offset, int nwb, float* l2,
+                                            unsigned* smax) {
+  constexpr int RUNS = brv_runs(M), STEPS = brv_steps(M);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+#pragma unroll 1
+  for (int c = warp; c < STEPS; c += nwarps) {
+    const int q = 32 * c + lane;
+    const bool in = q < RUNS;
+    const float* p = tile + 25 * min(q, RUNS - 1) + offset - 4;
+    float w[33];
 #pragma unroll
-        for (int r = 0; r < 7; r++) {
-          const float4 x = p[r];
-          wv[4 * r] = x.x; wv[4 * r + 1] = x.y; wv[4 * r + 2] = x.z; wv[4 * r + 3] = x.w;
-        }
-        if (wi == 0) brv_small<1, 0>(wv, v);
-        else if (wi == 1) brv_small<1, 1>(wv, v);
-        else brv_small<2, 2>(wv, v);
-        float4 o;
-        o.x = brv_med5<MM>(v[0], v[1], v[2], v[3], v[4]);
-        o.y = brv_med5<MM>(v[5], v[6], v[7], v[8], v[9]);
-        o.z = brv_med5<MM>(v[10], v[11], v[12], v[13], v[14]);
-        o.w = brv_med5<MM>(v[15], v[16], v[17], v[18], v[19]);
-        *reinterpret_cast<float4*>(la_w + k0) = o;
-        if (rec)
-          srun_w[q] = fmaxf(fmaxf(max5(v[0], v[1], v[2], v[3], v[4]), max5(v[5], v[6], v[7], v[8], v[9])),
-                            fmaxf(max5(v[10], v[11], v[12], v[13], v[14]),
-                                  max5(v[15], v[16], v[17], v[18], v[19])));
-      }
-    } else {
-      const int h = 1 << (wi - 1);  // ahead = behind = width / 2 (the launcher checks)
-      const float* ta = tile + offset + h;
-      const float* tb = tile + offset - h;
-      for (int q = lane; q < nq; q += 32) {
-        const float4* pa = reinterpret_cast<const float4*>(ta + 20 * q);
-        const float4* pb = reinterpret_cast<const float4*>(tb + 20 * q);
-        float v[20];
-#pragma unroll
-        for (int r = 0; r < 5; r++) {
-          const float4 a = pa[r], b = pb[r];
-          v[4 * r] = fabsf(__fsub_rn(a.x, b.x));
-          v[4 * r + 1] = fabsf(__fsub_rn(a.y, b.y));
-          v[4 * r + 2] = fabsf(__fsub_rn(a.z, b.z));
-          v[4 * r + 3] = fabsf(__fsub_rn(a.w, b.w));
-        }
-        float4 o;
-        o.x = brv_med5<MM>(v[0], v[1], v[2], v[3], v[4]);
-        o.y = brv_med5<MM>(v[5], v[6], v[7], v[8], v[9]);
-        o.z = brv_med5<MM>(v[10], v[11], v[12], v[13], v[14]);
-        o.w = brv_med5<MM>(v[15], v[16], v[17], v[18], v[19]);
-        *reinterpret_cast<float4*>(la_w + 4 * q) = o;
-        if (rec)
-          srun_w[q] = fmaxf(fmaxf(max5(v[0], v[1], v[2], v[3], v[4]), max5(v[5], v[6], v[7], v[8], v[9])),
-                            fmaxf(max5(v[10], v[11], v[12], v[13], v[14]),
-                                  max5(v[15], v[16], v[17], v[18], v[19])));
-      }
+    for (int r = 0; r < 33; r++) w[r] = p[r];
+    auto slot = [&](int wl, auto val) {
+      if (wl >= nwb) return;  // uniform
+      float top = 0.f;
+      const float m = brv_fold<MM>(val, &top);
+      if (in) l2[wl * RUNS + q] = m;
+      brv_top(top, smax, wl, lane);
+    };
+    slot(0, [&](int r) { return __fsub_rn(w[r + 5], w[r + 4]); });
+    slot(1, [&](int r) { return __fsub_rn(w[r + 5], w[r + 3]); });
+    slot(2, [&](int r) { return __fsub_rn(w[r + 6], w[r + 2]); });
+    slot(3, [&](int r) { return __fsub_rn(w[r + 8], w[r]); });
+  }
+  const int nsteps = (nwb - BRV_SMALL) * STEPS;  // of the other widths
+  const int spare = max(nwarps - STEPS, 0);      // warps without a small step
+#pragma unroll 1
+  for (int r = warp >= STEPS ? 0 : BRV_SMALL;; r++) {
+    const int u = r < BRV_SMALL ? r * spare + warp - STEPS
+                                : BRV_SMALL * spare + (r - BRV_SMALL) * nwarps + warp;
+    if (u >= nsteps) {
+      if (r >= BRV_SMALL) break;
+      continue;
     }
-    if constexpr (rem > 0)
-      if (lane < rem) {
-        const int k = 4 * nq + lane;
-        const WidthInfo& w = ctx.winfo[wi];
-        const int a = offset + w.ahead, b = offset - w.behind;
-        float v[5];
-#pragma unroll
-        for (int r = 0; r < 5; r++) v[r] = fabsf(__fsub_rn(tile[5 * k + r + a], tile[5 * k + r + b]));
-        la_w[k] = brv_med5<MM>(v[0], v[1], v[2], v[3], v[4]);
-        if (rec) srun_w[nq + lane] = max5(v[0], v[1], v[2], v[3], v[4]);
-      }
-    __syncwarp();  // the slot's level-1 row and run maxima are complete
-
-    if (rec) {
-      // values are non-negative or NaN, so their bit patterns order as
-      // unsigned (a NaN maximum only ever keeps a tile from being skipped);
-      // fmaxf above drops a NaN unless all its operands are NaN, and no sample
-      // is then left out of a maximum that decides a skip: a NaN boxcar never
-      // passes the test
-      unsigned mk = 0;
-      for (int q = lane; q < nq + rem; q += 32) mk = max(mk, __float_as_uint(srun_w[q]));
-      mk = __reduce_max_sync(0xffffffffu, mk);
-      if (lane == 0) ctx.gmax[(ser * nwb + wl) * ctx.ngroups + g] = __uint_as_float(mk);
-    }
-
-    // ---- levels 2..M: rows alternate between the slot's lb and la rows ----
-    float* rows[2] = {lb + wl * lbp, la_w};
-    const float* cur = la_w;
-    int n = n1;
-#pragma unroll
-    for (int lev = 2; lev <= M; lev++) {
-      float* nxt = rows[lev & 1 ? 1 : 0];
-      const int nn = n / 5;
-      for (int k = lane; k < nn; k += 32) {
-        const float* c = cur + 5 * k;
-        nxt[k] = brv_med5<MM>(c[0], c[1], c[2], c[3], c[4]);
-      }
-      __syncwarp();  // every lane reaches it: the level is complete
-      cur = nxt;
-      n = nn;
-    }
-    // n == 1: one value per width
-    if (lane == 0) out[(ser * nwb + wl) * out_pitch + g] = cur[0];
-    __syncwarp();  // the rows are free for the slot's next use
+    const int wl = BRV_SMALL + u / STEPS, q = 32 * (u % STEPS) + lane;
+    const bool in = q < RUNS;
+    const int h = 1 << (wl - 1);  // ahead = behind = width / 2 (the launcher checks)
+    const float* p = tile + 25 * min(q, RUNS - 1) + offset;
+    const float* pa = p + h;
+    const float* pb = p - h;
+    float top = 0.f;
+    const float m = brv_fold<MM>([&](int k) { return __fsub_rn(pa[k], pb[k]); }, &top);
+    if (in) l2[wl * RUNS + q] = m;
+    brv_top(top, smax, wl, lane);
   }
 }
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(smem_addr(dst)), "l"(src)
-               : "memory");
+// Five neighbours' median.
+template <bool MM>
+__device__ __forceinline__ float brv_next(const float* c) {
+  float none = 0.f;
+  return brv_med5<MM>(c[0], c[1], c[2], c[3], c[4], &none);
 }
+
+// Level 3 of one group for every width slot, from l2 to l3 [nwb][brv_l3(M)]
+// (level 2 itself where that is the last).
+__host__ __device__ constexpr int brv_l3(int m) { return m > 2 ? pow5c(m - 3) : 1; }
+template <bool MM, int M>
+__device__ __forceinline__ void brv_level3(const float* l2, float* l3, int nwb) {
+  constexpr int N3 = brv_l3(M);
+  for (int k = threadIdx.x; k < nwb * N3; k += blockDim.x)
+    l3[k] = M > 2 ? brv_next<MM>(l2 + 5 * k) : l2[k];
+}
+
+// Levels 4..M of `ngroups` groups from their l3 rows, and the group maxima:
+// rows of work [ngroups][nwb][5] in between.
+template <bool MM, int M>
+__device__ __forceinline__ void brv_finish(const WidthCtx& ctx, int nwb, const float* l3, float* work,
+                                           const unsigned* smax, float* __restrict__ out,
+                                           size_t out_pitch, size_t ser, int g_begin, int ngroups,
+                                           bool rec) {
+  if constexpr (M == 5) {
+    for (int k = threadIdx.x; k < ngroups * nwb * 5; k += blockDim.x)
+      work[k] = brv_next<MM>(l3 + 5 * k);
+    __syncthreads();
+  }
+  for (int k = threadIdx.x; k < ngroups * nwb; k += blockDim.x) {
+    const int j = k / nwb, wl = k - j * nwb;
+    const size_t slot = ser * nwb + wl, g = (size_t)(g_begin + j);
+    out[slot * out_pitch + g] = M == 5   ? brv_next<MM>(work + 5 * k)
+                                : M == 4 ? brv_next<MM>(l3 + 5 * k)
+                                         : l3[k];
+    if (rec) ctx.gmax[slot * ctx.ngroups + g] = __uint_as_float(smax[j * BRV_MAXW + wl]);
+  }
+}
+
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_addr(dst)), "l"(src)
                : "memory");
@@ -1065,38 +1067,35 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Block (x, y): groups [x * gpb, (x + 1) * gpb) of series y.  The next
 // group's window is copied into the other half of a double buffer (cp.async)
-// while the current group's medians are computed.
+// while the current group's medians are computed.  Of 8424 series x 28000
+// samples x 10 widths: 1.03 ms with runs of 20 samples as float4 loads, whose
+// level-1 medians went through shared memory (bound by its bandwidth, 84 %, and
+// 12400 instructions a group), 0.71 ms so (issue 78 %, min/max pipe 68 %).
 template <int M>
-__global__ void __launch_bounds__(BRV_THREADS) k_block_rms_pass1_vec(WidthCtx ctx, int w0,
-                                                                     int nwb, int win,
-                                                                     float* __restrict__ out,
-                                                                     size_t out_pitch,
-                                                                     int ngroups, int gpb) {
+__global__ void __launch_bounds__(BRV_THREADS, 2) k_block_rms_pass1_vec(
+    WidthCtx ctx, int nwb, int win, float* __restrict__ out, size_t out_pitch, int ngroups,
+    int gpb) {
   extern __shared__ __align__(16) float dyn[];
-  const int win4 = (win + 3) & ~3;
-  float* tiles = dyn;                    // [2][win4]
-  constexpr int n1 = pow5c(M - 1);       // level-1 medians per width
-  const int n1p = (n1 + 3) & ~3;         // row pitch: 16-byte aligned rows
-  float* la = dyn + 2 * win4;            // [nwb][n1p]
-  float* lb = la + nwb * n1p;            // [nwb][n1 / 5 + 1]
-  float* srun = lb + nwb * (n1 / 5 + 1); // [nwb][n1 / 4 + 4] (group maxima)
+  constexpr int RUNS = brv_runs(M);
+  constexpr size_t gsz = pow5c(M);
+  __shared__ unsigned smax[BRV_GPB * BRV_MAXW];  // group maxima, as bits
+  float* tiles = dyn;                            // [2][win]
+  float* l2 = dyn + 2 * win;                     // [nwb][RUNS]; at the end [gpb][nwb][5]
+  float* l3 = l2 + nwb * (RUNS > 5 * BRV_GPB ? RUNS : 5 * BRV_GPB);  // [gpb][nwb][brv_l3(M)]
   const size_t ser = blockIdx.y;
   const int g_begin = blockIdx.x * gpb;
   const int g_end = min(g_begin + gpb, ngroups);
-  const WidthInfo& w_first = ctx.winfo[w0];
   const float* sc = ctx.scan + ser * ctx.scan_pitch;
-  const float delta = (float)(ctx.stride - w_first.bn);
-  constexpr size_t gsz = pow5c(M);
   const int offset = ctx.offset;
-  // the launcher guarantees contiguous groups (one beam) whose window fits
-  auto first_of = [&](int g) {
-    const size_t q0 = (size_t)g * gsz;
-    return reblock_index((unsigned)q0 / w_first.bn, delta, (unsigned)q0);
-  };
-  const size_t span = gsz - 1 + 2 * (size_t)offset + 2;
+  // one beam: group g is the samples from g * 5^M; its window is copied from
+  // the 16 bytes that hold its first sample to the row's end at most (inside
+  // the row's pitch)
+  const size_t row_end = (ctx.scan_len + 3) & ~(size_t)3;
   auto prefetch = [&](int g, float* tile) {
-    const float* src = sc + first_of(g);
-    for (size_t k = threadIdx.x; k < span; k += blockDim.x) cp_async4(tile + k, src + k);
+    const size_t at = (size_t)g * gsz & ~(size_t)3;
+    const unsigned n = (unsigned)min((size_t)win, row_end > at ? row_end - at : 0);
+    for (unsigned k = 4 * threadIdx.x; k < n; k += 4 * blockDim.x)
+      cp_async16(tile + k, sc + at + k);
     cp_async_commit();
   };
   // A prefix sum that is finite at its end is finite everywhere (a non-finite
@@ -1104,25 +1103,26 @@ __global__ void __launch_bounds__(BRV_THREADS) k_block_rms_pass1_vec(WidthCtx ct
   // min/max median network selects the same values as the reference's.
   const float last = sc[ctx.scan_len - 1];
   const bool finite = fabsf(last) <= 3.402823466e38f;
-  if (g_begin >= g_end || span > (size_t)win) return;
+  if (g_begin >= g_end) return;
   const bool rec = ctx.gmax != nullptr && ctx.ngroups > 0;
+  for (int k = threadIdx.x; k < BRV_GPB * BRV_MAXW; k += blockDim.x) smax[k] = 0;
   prefetch(g_begin, tiles);
   for (int g = g_begin; g < g_end; g++) {
-    float* tile = tiles + (size_t)((g - g_begin) & 1) * win4;
-    // the previous group's levels (and final reads of la/lb) are finished
+    const int j = g - g_begin;
+    const float* tile = tiles + (size_t)(j & 1) * win + (((size_t)g * gsz) & 3);
+    cp_async_wait<0>();
+    // the group's window is complete; the previous group's level 3 is finished
     __syncthreads();
-    if (g + 1 < g_end) {
-      prefetch(g + 1, tiles + (size_t)((g + 1 - g_begin) & 1) * win4);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    if (g + 1 < g_end) prefetch(g + 1, tiles + (size_t)((j + 1) & 1) * win);
+    if (finite) brv_level12<true, M>(tile, offset, nwb, l2, smax + j * BRV_MAXW);
+    else brv_level12<false, M>(tile, offset, nwb, l2, smax + j * BRV_MAXW);
     __syncthreads();
-    if (finite)
-      brv_levels<true, M>(ctx, tile, offset, w0, nwb, la, lb, out, out_pitch, ser, g, srun, rec);
-    else
-      brv_levels<false, M>(ctx, tile, offset, w0, nwb, la, lb, out, out_pitch, ser, g, srun, rec);
+    if (finite) brv_level3<true, M>(l2, l3 + j * nwb * brv_l3(M), nwb);
+    else brv_level3<false, M>(l2, l3 + j * nwb * brv_l3(M), nwb);
   }
+  __syncthreads();
+  if (finite) brv_finish<true, M>(ctx, nwb, l3, l2, smax, out, out_pitch, ser, g_begin, g_end - g_begin, rec);
+  else brv_finish<false, M>(ctx, nwb, l3, l2, smax, out, out_pitch, ser, g_begin, g_end - g_begin, rec);
 }
 
 __global__ void k_block_rms_final(WidthCtx ctx, int w0, int nwb, const float* __restrict__ lev,
@@ -1181,18 +1181,19 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
   }
   // a group of samples is contiguous unless it straddles a beam gap
   // (nbeams > 1); single-beam series always take the vector kernel
+  vec = vec && w_begin == 0 && nwb <= BRV_MAXW && m1 >= 2 && ctx.scan_pitch % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(ctx.scan) & 15) == 0;
   if (vec && ctx.nbeams == 1) {
-    const size_t win = pow5(m1) + 2 * (size_t)ctx.offset + 2;
-    const size_t n1 = pow5(m1 - 1);
-    const size_t smem = (2 * ((win + 3) & ~(size_t)3) + nwb * ((n1 + 3) & ~(size_t)3) +
-                         nwb * (n1 / 5 + 1) + nwb * (n1 / 4 + 4)) *
-                        sizeof(float);
+    const size_t runs = (size_t)brv_runs(m1);
+    // a window begins up to 3 samples before its group
+    const size_t win = (pow5(m1) + 2 * (size_t)ctx.offset + 6) & ~(size_t)3;
+    const size_t smem = (2 * win + nwb * (std::max<size_t>(runs, 5 * BRV_GPB) +
+                                          BRV_GPB * (size_t)brv_l3(m1))) * sizeof(float);
     if (smem <= 200 * 1024) {
       auto kern = m1 == 5 ? k_block_rms_pass1_vec<5>
                   : m1 == 4 ? k_block_rms_pass1_vec<4>
                   : m1 == 3 ? k_block_rms_pass1_vec<3>
-                  : m1 == 2 ? k_block_rms_pass1_vec<2>
-                            : k_block_rms_pass1_vec<1>;
+                            : k_block_rms_pass1_vec<2>;
       if ((e = raise_smem_limit(kern, smem)) != cudaSuccess) return e;
       // the group maxima of the widths [0, nwb) for count_hits
       if (ctx.gmax && w_begin == 0 && nwb <= VH_MAXW && nseg * ng1 <= ctx.gmax_cap) {
@@ -1202,11 +1203,11 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
       }
       // about 8 consecutive groups per block, spread evenly; fewer where that
       // leaves the SMs without two blocks each
-      const size_t nblk_x = std::max((ng1 + 7) / 8, std::min<size_t>(ng1, 296 / ctx.nser + 1));
+      const size_t nblk_x = std::max((ng1 + BRV_GPB - 1) / BRV_GPB, std::min<size_t>(ng1, 296 / ctx.nser + 1));
       const size_t gpb = (ng1 + nblk_x - 1) / nblk_x;
       const unsigned nthreads = 32u * (unsigned)std::min(nwb, BRV_THREADS / 32);
       kern<<<dim3((unsigned)((ng1 + gpb - 1) / gpb), ctx.nser), nthreads, smem, s>>>(
-          ctx, w_begin, nwb, (int)win, ws.a, ng1, (int)ng1, (int)gpb); note_launch();
+          ctx, nwb, (int)win, ws.a, ng1, (int)ng1, (int)gpb); note_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       float* fin;
       size_t fin_pitch, fin_count;
