@@ -220,6 +220,12 @@ struct WidthInfo {
 };
 
 constexpr int TS_GMAX = 4;  // time-scrunched widths whose group maxima are kept
+constexpr unsigned GMAX_STEP = 800;  // 32 lanes of 25 samples
+// floats that hold the maxima of nser series of n samples and nw widths
+inline size_t gmax_floats(size_t nser, size_t nw, size_t n) {
+  return nser * nw * (n / 3125 * 4 + 9);
+}
+
 struct WidthCtx {
   const float* scan;
   size_t scan_pitch;
@@ -236,15 +242,16 @@ struct WidthCtx {
   int dm_offset;                // DM index of each unit's first series
   float* norm;        // [nser][nw]  1 / block_rms
   float thresh;
-  // Largest |boxcar value| of each block-RMS group (gsize consecutive
-  // filtered samples, ngroups complete groups per series) for the
-  // unscrunched widths [0, gmax_nw): [nser][gmax_nw][ngroups].  block_rms
-  // records it when gmax is set and the group geometry fits gmax_cap floats
-  // (else ngroups = 0); count_hits skips the tiles whose covering groups
-  // stay below every width's threshold.
+  // Largest |boxcar value| of each stretch of GMAX_STEP filtered
+  // samples, counted anew from the start of each block-RMS group of gsize (at
+  // most gsteps stretches each), for the unscrunched widths [0, gmax_nw):
+  // [nser][gmax_nw][ngmax], over all samples (the last, incomplete group's
+  // too).  block_rms records it when gmax is set and the maxima fit gmax_cap
+  // floats (else ngmax = 0); count_hits skips the tiles whose stretches stay
+  // below every width's threshold.
   float* gmax;
   size_t gmax_cap;
-  unsigned gsize, ngroups;
+  unsigned gsize, gsteps, ngmax;
   int gmax_nw;
   // the same of the k-th width after those (time-scrunched; one beam): group
   // maxima [nser][ts_ngroups[k]] from gmax + ts_gmax[k] on (0 groups: none)
@@ -266,6 +273,28 @@ struct HitBuffers {
   unsigned* tile_list;  // capacity nser * ntiles
   unsigned* tile_list_n;
   bool list_valid;
+  // what the group maxima leave to be counted, listed by count_hits
+  // (sel_valid): tiles (ser * ntiles + tile) and the set of unscrunched widths
+  // to count in each, ((ser * nw + width) * ntiles + tile) of the
+  // time-scrunched ones, and each width's smallest boxcar value that is a hit
+  unsigned *sel, *sel_widths, *sel_n;  // capacity nser * ntiles
+  unsigned *sel_ts, *sel_ts_n;         // capacity nser * (nw - unscrunched) * ntiles
+  float* bound;                        // [nser][nw], -1: none
+  bool sel_valid;
+  // the lists and bounds in hit_list_words(nser, nw, ntiles) words of p
+  static size_t hit_list_words(size_t nser, size_t nw, size_t ntiles) {
+    return 4 + nser * nw + nser * ntiles * (nw + 3);
+  }
+  void set_lists(unsigned* p, size_t nser, size_t nw, size_t ntiles) {
+    tile_list_n = p;
+    sel_n = p + 1;
+    sel_ts_n = p + 2;
+    bound = reinterpret_cast<float*>(p + 4);
+    tile_list = p + 4 + nser * nw;
+    sel = tile_list + nser * ntiles;
+    sel_widths = sel + nser * ntiles;
+    sel_ts = sel_widths + nser * ntiles;
+  }
   unsigned* tile_cnt;   // [nser][nw][ntiles]
   unsigned* sw_cnt;     // [nser*nw + 1]
   unsigned* sw_off;     // [nser*nw + 1]

@@ -902,8 +902,14 @@ __global__ void k_block_rms_pass1_multi(WidthCtx ctx, int w0, int nwb, int m, in
 // the staged window at a lane stride of 25 words, which no two lanes' banks
 // share, and no level-1 medians in shared memory.  Widths 1, 2, 4 and 8 share
 // one 33-value window.
+constexpr int HIT_TILE = 2048;  // samples of a threshold tile
+constexpr int HIT_THREADS = 256;
+constexpr int HIT_PER_THREAD = HIT_TILE / HIT_THREADS;
+// whether the thresholds first look which tiles can have hits
+static bool select_pays(int nser, size_t ntiles) { return (size_t)nser * ntiles > 148 * 8; }
+
 constexpr int BRV_THREADS = 512;  // at most 16 warps: one per boxcar width
-constexpr int BRV_MAXW = 32;  // width slots with a group maximum
+constexpr int BRV_MAXW = 32;  // width slots of the vector kernel
 constexpr int BRV_GPB = 8;    // groups of a block at most
 constexpr int VH_MAXW = 16;  // unscrunched widths the vector kernels handle at once
 
@@ -938,8 +944,9 @@ __host__ __device__ constexpr int brv_runs(int m) { return pow5c(m - 2); }
 __host__ __device__ constexpr int brv_steps(int m) { return (brv_runs(m) + 31) / 32; }
 constexpr int BRV_SMALL = 4;  // widths 1, 2, 4, 8: one window, one warp
 
-// Median of the five medians of 25 boxcar magnitudes val(0..24); *top is raised
-// to the largest.
+// Median of the five medians of 25 boxcar magnitudes |val(0..24)|; *top is raised
+// to the largest magnitude (shared with the medians; the largest value itself
+// would take 5 % longer and skips 1 % more tiles).
 template <bool MM, class F>
 __device__ __forceinline__ float brv_fold(F val, float* top) {
   float m[5], none = 0.f;
@@ -953,22 +960,23 @@ __device__ __forceinline__ float brv_fold(F val, float* top) {
   return brv_med5<MM>(m[0], m[1], m[2], m[3], m[4], &none);
 }
 
-// The largest value of a width slot's step to smax[wl].  Values are
-// non-negative or NaN, so their bit patterns order as unsigned; fmaxf drops a
-// NaN unless all its operands are NaN, and no sample is then left out of a
-// maximum that decides a skip: a NaN boxcar never passes the test.
-__device__ __forceinline__ void brv_top(float top, unsigned* smax, int wl, int lane) {
+// The largest magnitude of a width slot's step to *gmax.  Bit patterns
+// of values >= +0 order as unsigned; the maxima drop a NaN unless all their
+// operands are NaN, and no sample is then left out of a maximum that decides a
+// skip: a NaN boxcar never passes the test.
+__device__ __forceinline__ void brv_top(float top, float* gmax, int lane) {
   const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
-  if (lane == 0) atomicMax(&smax[wl], m);
+  if (lane == 0) *gmax = __uint_as_float(m);
 }
 
 // Levels 1 and 2 of one group, whose first sample is at `tile`, for every width
 // slot, to l2 [nwb][brv_runs(M)].  The work is cut into steps of 32 runs of one width, the four small
 // widths' step counting as four, and dealt out so that the warps (one per slot)
-// get equal shares.
+// get equal shares.  A step's maximum goes to gmax[width slot * gpitch + step]
+// (gmax may be null).
 template <bool MM, int M>
 __device__ __forceinline__ void brv_level12(const float* tile, int offset, int nwb, float* l2,
-                                            unsigned* smax) {
+                                            float* gmax, size_t gpitch) {
   constexpr int RUNS = brv_runs(M), STEPS = brv_steps(M);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
 #pragma unroll 1
@@ -984,7 +992,7 @@ __device__ __forceinline__ void brv_level12(const float* tile, int offset, int n
       float top = 0.f;
       const float m = brv_fold<MM>(val, &top);
       if (in) l2[wl * RUNS + q] = m;
-      brv_top(top, smax, wl, lane);
+      if (gmax) brv_top(top, gmax + wl * gpitch + c, lane);
     };
     slot(0, [&](int r) { return __fsub_rn(w[r + 5], w[r + 4]); });
     slot(1, [&](int r) { return __fsub_rn(w[r + 5], w[r + 3]); });
@@ -1010,7 +1018,32 @@ __device__ __forceinline__ void brv_level12(const float* tile, int offset, int n
     float top = 0.f;
     const float m = brv_fold<MM>([&](int k) { return __fsub_rn(pa[k], pb[k]); }, &top);
     if (in) l2[wl * RUNS + q] = m;
-    brv_top(top, smax, wl, lane);
+    if (gmax) brv_top(top, gmax + wl * gpitch + u % STEPS, lane);
+  }
+}
+
+// The maxima of the n < 5^M samples after the last group, step by step.
+__device__ __forceinline__ void brv_rest(const WidthInfo* winfo, const float* tile, int offset,
+                                         int nwb, unsigned n, float* gmax, size_t gpitch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int steps = (int)((n + GMAX_STEP - 1) / GMAX_STEP);
+  for (int u = warp; u < nwb * steps; u += nwarps) {
+    const int wl = u / steps, c = u % steps;
+    const float* a = tile + offset + winfo[wl].ahead;
+    const float* b = tile + offset - winfo[wl].behind;
+    const unsigned i0 = c * GMAX_STEP + lane;
+    float top = 0.f;
+    if ((c + 1) * GMAX_STEP <= n) {
+#pragma unroll
+      for (unsigned k = 0; k < GMAX_STEP; k += 64)
+        top = k + 32 < GMAX_STEP
+                  ? max3(top, fabsf(__fsub_rn(a[i0 + k], b[i0 + k])),
+                         fabsf(__fsub_rn(a[i0 + k + 32], b[i0 + k + 32])))
+                  : fmaxf(top, fabsf(__fsub_rn(a[i0 + k], b[i0 + k])));
+    } else {
+      for (unsigned i = i0; i < n; i += 32) top = fmaxf(top, fabsf(__fsub_rn(a[i], b[i])));
+    }
+    brv_top(top, gmax + wl * gpitch + c, lane);
   }
 }
 
@@ -1031,13 +1064,12 @@ __device__ __forceinline__ void brv_level3(const float* l2, float* l3, int nwb) 
     l3[k] = M > 2 ? brv_next<MM>(l2 + 5 * k) : l2[k];
 }
 
-// Levels 4..M of `ngroups` groups from their l3 rows, and the group maxima:
-// rows of work [ngroups][nwb][5] in between.
+// Levels 4..M of `ngroups` groups from their l3 rows; rows of work
+// [ngroups][nwb][5] in between.
 template <bool MM, int M>
-__device__ __forceinline__ void brv_finish(const WidthCtx& ctx, int nwb, const float* l3, float* work,
-                                           const unsigned* smax, float* __restrict__ out,
-                                           size_t out_pitch, size_t ser, int g_begin, int ngroups,
-                                           bool rec) {
+__device__ __forceinline__ void brv_finish(int nwb, const float* l3, float* work,
+                                           float* __restrict__ out, size_t out_pitch, size_t ser,
+                                           int g_begin, int ngroups) {
   if constexpr (M == 5) {
     for (int k = threadIdx.x; k < ngroups * nwb * 5; k += blockDim.x)
       work[k] = brv_next<MM>(l3 + 5 * k);
@@ -1049,7 +1081,6 @@ __device__ __forceinline__ void brv_finish(const WidthCtx& ctx, int nwb, const f
     out[slot * out_pitch + g] = M == 5   ? brv_next<MM>(work + 5 * k)
                                 : M == 4 ? brv_next<MM>(l3 + 5 * k)
                                          : l3[k];
-    if (rec) ctx.gmax[slot * ctx.ngroups + g] = __uint_as_float(smax[j * BRV_MAXW + wl]);
   }
 }
 
@@ -1074,17 +1105,16 @@ __device__ __forceinline__ void cp_async_wait() {
 template <int M>
 __global__ void __launch_bounds__(BRV_THREADS, 2) k_block_rms_pass1_vec(
     WidthCtx ctx, int nwb, int win, float* __restrict__ out, size_t out_pitch, int ngroups,
-    int gpb) {
+    unsigned rest, int gpb) {
   extern __shared__ __align__(16) float dyn[];
   constexpr int RUNS = brv_runs(M);
   constexpr size_t gsz = pow5c(M);
-  __shared__ unsigned smax[BRV_GPB * BRV_MAXW];  // group maxima, as bits
   float* tiles = dyn;                            // [2][win]
   float* l2 = dyn + 2 * win;                     // [nwb][RUNS]; at the end [gpb][nwb][5]
   float* l3 = l2 + nwb * (RUNS > 5 * BRV_GPB ? RUNS : 5 * BRV_GPB);  // [gpb][nwb][brv_l3(M)]
   const size_t ser = blockIdx.y;
   const int g_begin = blockIdx.x * gpb;
-  const int g_end = min(g_begin + gpb, ngroups);
+  const int g_end = min(g_begin + gpb, ngroups + (rest ? 1 : 0));
   const float* sc = ctx.scan + ser * ctx.scan_pitch;
   const int offset = ctx.offset;
   // one beam: group g is the samples from g * 5^M; its window is copied from
@@ -1104,25 +1134,32 @@ __global__ void __launch_bounds__(BRV_THREADS, 2) k_block_rms_pass1_vec(
   const float last = sc[ctx.scan_len - 1];
   const bool finite = fabsf(last) <= 3.402823466e38f;
   if (g_begin >= g_end) return;
-  const bool rec = ctx.gmax != nullptr && ctx.ngroups > 0;
-  for (int k = threadIdx.x; k < BRV_GPB * BRV_MAXW; k += blockDim.x) smax[k] = 0;
+  // (group ngroups is the rest: only its maxima are wanted)
+  const bool rec = ctx.gmax != nullptr && ctx.ngmax > 0;
+  const size_t gpitch = ctx.ngmax;
   prefetch(g_begin, tiles);
   for (int g = g_begin; g < g_end; g++) {
     const int j = g - g_begin;
     const float* tile = tiles + (size_t)(j & 1) * win + (((size_t)g * gsz) & 3);
+    float* gmax = rec ? ctx.gmax + ser * nwb * gpitch + (size_t)g * brv_steps(M) : nullptr;
     cp_async_wait<0>();
     // the group's window is complete; the previous group's level 3 is finished
     __syncthreads();
     if (g + 1 < g_end) prefetch(g + 1, tiles + (size_t)((j + 1) & 1) * win);
-    if (finite) brv_level12<true, M>(tile, offset, nwb, l2, smax + j * BRV_MAXW);
-    else brv_level12<false, M>(tile, offset, nwb, l2, smax + j * BRV_MAXW);
+    if (g == ngroups) {
+      brv_rest(ctx.winfo, tile, offset, nwb, rest, gmax, gpitch);
+      break;
+    }
+    if (finite) brv_level12<true, M>(tile, offset, nwb, l2, gmax, gpitch);
+    else brv_level12<false, M>(tile, offset, nwb, l2, gmax, gpitch);
     __syncthreads();
     if (finite) brv_level3<true, M>(l2, l3 + j * nwb * brv_l3(M), nwb);
     else brv_level3<false, M>(l2, l3 + j * nwb * brv_l3(M), nwb);
   }
   __syncthreads();
-  if (finite) brv_finish<true, M>(ctx, nwb, l3, l2, smax, out, out_pitch, ser, g_begin, g_end - g_begin, rec);
-  else brv_finish<false, M>(ctx, nwb, l3, l2, smax, out, out_pitch, ser, g_begin, g_end - g_begin, rec);
+  const int n = min(g_end, ngroups) - g_begin;
+  if (finite) brv_finish<true, M>(nwb, l3, l2, out, out_pitch, ser, g_begin, n);
+  else brv_finish<false, M>(nwb, l3, l2, out, out_pitch, ser, g_begin, n);
 }
 
 __global__ void k_block_rms_final(WidthCtx ctx, int w0, int nwb, const float* __restrict__ lev,
@@ -1151,8 +1188,8 @@ __global__ void k_block_rms_final(WidthCtx ctx, int w0, int nwb, const float* __
 
 cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end,
                       TreeScratch& ws, cudaStream_t s) {
-  if (w_begin == 0) {  // no group maxima unless recorded below
-    ctx.ngroups = 0;
+  if (w_begin == 0) {  // no maxima unless recorded below
+    ctx.ngmax = 0;
     for (unsigned& n : ctx.ts_ngroups) n = 0;
   }
   const int nwb = w_end - w_begin;
@@ -1195,19 +1232,29 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
                   : m1 == 3 ? k_block_rms_pass1_vec<3>
                             : k_block_rms_pass1_vec<2>;
       if ((e = raise_smem_limit(kern, smem)) != cudaSuccess) return e;
-      // the group maxima of the widths [0, nwb) for count_hits
-      if (ctx.gmax && w_begin == 0 && nwb <= VH_MAXW && nseg * ng1 <= ctx.gmax_cap) {
+      // the maxima of the widths [0, nwb) for count_hits, whose samples are
+      // those below bn and n, the same for all of them
+      const size_t ngs = (size_t)brv_steps(m1);
+      const size_t all = std::min<size_t>(hw[0].bn, hw[0].n);
+      unsigned rest = 0;
+      if (ctx.gmax && select_pays(ctx.nser, (hw[0].n + HIT_TILE - 1) / HIT_TILE) &&
+          nwb <= VH_MAXW && hw[0].n <= ctx.stride && all >= ng1 * pow5(m1) &&
+          nseg * (ng1 + 1) * ngs <= ctx.gmax_cap) {
+        rest = (unsigned)(all - ng1 * pow5(m1));
         ctx.gsize = (unsigned)pow5(m1);
-        ctx.ngroups = (unsigned)ng1;
+        ctx.gsteps = (unsigned)ngs;
+        ctx.ngmax = (unsigned)(ng1 * ngs) + (rest + GMAX_STEP - 1) / GMAX_STEP;
         ctx.gmax_nw = nwb;
       }
       // about 8 consecutive groups per block, spread evenly; fewer where that
       // leaves the SMs without two blocks each
-      const size_t nblk_x = std::max((ng1 + BRV_GPB - 1) / BRV_GPB, std::min<size_t>(ng1, 296 / ctx.nser + 1));
-      const size_t gpb = (ng1 + nblk_x - 1) / nblk_x;
+      const size_t ngr = ng1 + (rest ? 1 : 0);
+      const size_t nblk_x =
+          std::max((ngr + BRV_GPB - 1) / BRV_GPB, std::min<size_t>(ngr, 296 / ctx.nser + 1));
+      const size_t gpb = (ngr + nblk_x - 1) / nblk_x;
       const unsigned nthreads = 32u * (unsigned)std::min(nwb, BRV_THREADS / 32);
-      kern<<<dim3((unsigned)((ng1 + gpb - 1) / gpb), ctx.nser), nthreads, smem, s>>>(
-          ctx, nwb, (int)win, ws.a, ng1, (int)ng1, (int)gpb); note_launch();
+      kern<<<dim3((unsigned)((ngr + gpb - 1) / gpb), ctx.nser), nthreads, smem, s>>>(
+          ctx, nwb, (int)win, ws.a, ng1, (int)ng1, rest, (int)gpb); note_launch();
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       float* fin;
       size_t fin_pitch, fin_count;
@@ -1229,8 +1276,8 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
     // the group maxima of a time-scrunched width, after the unscrunched ones
     float* gm = nullptr;
     const int k = w_begin - ctx.gmax_nw;
-    if (ctx.gmax && ctx.ngroups > 0 && ctx.nbeams == 1 && nwb == 1 && k >= 0 && k < TS_GMAX) {
-      size_t at = (size_t)ctx.nser * ctx.gmax_nw * ctx.ngroups;
+    if (ctx.gmax && ctx.ngmax > 0 && ctx.nbeams == 1 && nwb == 1 && k >= 0 && k < TS_GMAX) {
+      size_t at = (size_t)ctx.nser * ctx.gmax_nw * ctx.ngmax;
       for (int j = 0; j < k; j++) at += (size_t)ctx.nser * ctx.ts_ngroups[j];
       if (at + (size_t)ctx.nser * ng1 <= ctx.gmax_cap) {
         gm = ctx.gmax + at;
@@ -1256,9 +1303,6 @@ cudaError_t block_rms(WidthCtx& ctx, const WidthInfo* hw, int w_begin, int w_end
 // Thresholding (find_giants.cu:47-60,137-183): hits are filtered indices i
 // with (i % beam_stride) < bn and normalised value > thresh.
 // ===========================================================================
-constexpr int HIT_TILE = 2048;
-constexpr int HIT_THREADS = 256;
-constexpr int HIT_PER_THREAD = HIT_TILE / HIT_THREADS;
 
 __device__ __forceinline__ bool hit_at(const WidthCtx& ctx, const float* sc, float norm,
                                        const WidthInfo& w, size_t i, float* val) {
@@ -1269,63 +1313,63 @@ __device__ __forceinline__ bool hit_at(const WidthCtx& ctx, const float* sc, flo
   return v > ctx.thresh;
 }
 
+// Entry of the time-scrunched widths' tile list.
+__device__ __forceinline__ void sel_item(unsigned e, unsigned ntiles, unsigned nw, unsigned* ser,
+                                         unsigned* wi, unsigned* tile) {
+  const unsigned sw = e / ntiles;
+  *tile = e - sw * ntiles;
+  *ser = sw / nw;
+  *wi = sw - *ser * nw;
+}
+
 // Counts of one tile; consecutive threads take consecutive samples (the order
 // does not matter to a count), and each thread finds its sample's place in the
-// beam once and steps it.  A tile whose block-RMS groups' maxima stay below the
-// threshold counts nothing and reads nothing (the survey gulp's time-scrunched
-// width: 180 us; 370 without the maxima, 687 with a 64-bit remainder per
-// sample and 8 strided samples per thread too).
+// beam once and steps it.  The tiles are those that k_select_tiles lists, strided
+// over the blocks, or block (x, y, z): tile x of width w_base + y of series z.
+// The survey gulp's time-scrunched width: 687 us with a 64-bit remainder per
+// sample and 8 strided samples per thread, 370 without, 180 with each block
+// asking the group maxima first, 53 us with the list.
 __global__ void __launch_bounds__(HIT_THREADS) k_count_hits(WidthCtx ctx, HitBuffers hb,
                                                             int w_base) {
-  const int wi = w_base + blockIdx.y;
-  const size_t ser = blockIdx.z;
-  const unsigned tile = blockIdx.x;
-  const WidthInfo w = ctx.winfo[wi];
-  const float norm = ctx.norm[ser * ctx.nw + wi];
-  const unsigned ts = (unsigned)w.ts, stride = (unsigned)ctx.stride;
-  const unsigned i0 = tile * HIT_TILE + threadIdx.x;
-  const float* lo = ctx.scan + ser * ctx.scan_pitch + (ctx.offset - w.behind) + (size_t)i0 * ts;
-  const float* hi = lo + w.behind + w.ahead;
-  unsigned c = 0;
-  bool need = tile * HIT_TILE < w.n;
-  const int tk = wi - ctx.gmax_nw;
-  if (need && tk >= 0 && tk < TS_GMAX && ctx.ts_ngroups[tk] > 0) {
-    // the groups' window indices are the filtered indices (one beam)
-    const unsigned ng = ctx.ts_ngroups[tk], gs = ctx.ts_gsize[tk];
-    const unsigned g0 = tile * HIT_TILE / gs, g1 = (tile * HIT_TILE + HIT_TILE - 1) / gs;
-    if (g1 < ng) {
-      const float* gm = ctx.gmax + ctx.ts_gmax[tk] + ser * ng;
-      float mx = 0.f;
-      for (unsigned g = g0; g <= g1; g++) mx = fmaxf(mx, gm[g]);
-      // RN(d * norm) is monotone in d for a positive norm
-      need = !(norm > 0.f && __fmul_rn(mx, norm) <= ctx.thresh);
-    }
-  }
-  if (need) {
-    unsigned at = i0 % stride;  // sample within its beam
-    const unsigned step = HIT_THREADS % stride;
-#pragma unroll
-    for (int k = 0; k < HIT_PER_THREAD; k++) {
-      const unsigned i = i0 + k * HIT_THREADS;
-      if (i < w.n && at < w.bn) {
-        const size_t p = (size_t)(k * HIT_THREADS) * ts;
-        c += __fmul_rn(__fsub_rn(hi[p], lo[p]), norm) > ctx.thresh;
-      }
-      at += step;
-      if (at >= stride) at -= stride;
-    }
-  }
   __shared__ unsigned red[HIT_THREADS / 32];
+  const unsigned nlist = hb.sel_valid ? *hb.sel_ts_n : 1u;
+  for (unsigned idx = hb.sel_valid ? blockIdx.x : 0; idx < nlist; idx += gridDim.x) {
+    unsigned ser = blockIdx.z, wi = w_base + blockIdx.y, tile = blockIdx.x;
+    if (hb.sel_valid) sel_item(hb.sel_ts[idx], hb.ntiles, (unsigned)ctx.nw, &ser, &wi, &tile);
+    const size_t sw = (size_t)ser * ctx.nw + wi;
+    const WidthInfo w = ctx.winfo[wi];
+    const float norm = ctx.norm[sw];
+    const unsigned ts = (unsigned)w.ts, stride = (unsigned)ctx.stride;
+    const unsigned i0 = tile * HIT_TILE + threadIdx.x;
+    const float* lo =
+        ctx.scan + (size_t)ser * ctx.scan_pitch + (ctx.offset - w.behind) + (size_t)i0 * ts;
+    const float* hi = lo + w.behind + w.ahead;
+    unsigned c = 0;
+    if (tile * HIT_TILE < w.n) {
+      unsigned at = i0 % stride;  // sample within its beam
+      const unsigned step = HIT_THREADS % stride;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned t = 0;
-    for (int k = 0; k < HIT_THREADS / 32; k++) t += red[k];
-    size_t sw = ser * ctx.nw + wi;
-    hb.tile_cnt[sw * hb.ntiles + tile] = t;
-    if (t) atomicAdd(&hb.sw_cnt[sw], t);
+      for (int k = 0; k < HIT_PER_THREAD; k++) {
+        const unsigned i = i0 + k * HIT_THREADS;
+        if (i < w.n && at < w.bn) {
+          const size_t p = (size_t)(k * HIT_THREADS) * ts;
+          c += __fmul_rn(__fsub_rn(hi[p], lo[p]), norm) > ctx.thresh;
+        }
+        at += step;
+        if (at >= stride) at -= stride;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned t = 0;
+      for (int k = 0; k < HIT_THREADS / 32; k++) t += red[k];
+      hb.tile_cnt[sw * hb.ntiles + tile] = t;
+      if (t) atomicAdd(&hb.sw_cnt[sw], t);
+    }
+    __syncthreads();  // the partial counts are read
   }
 }
 
@@ -1351,13 +1395,11 @@ __global__ void k_scan_tiles(const unsigned* __restrict__ cnt, unsigned* __restr
   }
 }
 
-__global__ void __launch_bounds__(HIT_THREADS) k_write_hits(WidthCtx ctx, HitBuffers hb,
-                                                            int w_base) {
-  const int wi = w_base + blockIdx.y;
-  const size_t ser = blockIdx.z;
-  const unsigned tile = blockIdx.x;
+__device__ __forceinline__ void write_hits_tile(const WidthCtx& ctx, const HitBuffers& hb,
+                                                size_t ser, unsigned wi, unsigned tile,
+                                                unsigned* wsum) {
   const size_t sw = ser * ctx.nw + wi;
-  if (hb.tile_cnt[sw * hb.ntiles + tile] == 0) return;
+  if (hb.tile_cnt[sw * hb.ntiles + tile] == 0) return;  // uniform across the block
   const WidthInfo& w = ctx.winfo[wi];
   const float* sc = ctx.scan + ser * ctx.scan_pitch;
   const float norm = ctx.norm[sw];
@@ -1371,7 +1413,6 @@ __global__ void __launch_bounds__(HIT_THREADS) k_write_hits(WidthCtx ctx, HitBuf
   }
   unsigned c = __popc(flags);
   // block exclusive scan of c
-  __shared__ unsigned wsum[HIT_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned x = c;
 #pragma unroll
@@ -1394,6 +1435,24 @@ __global__ void __launch_bounds__(HIT_THREADS) k_write_hits(WidthCtx ctx, HitBuf
       }
       pos++;
     }
+  }
+}
+
+// The tiles that k_select_tiles lists, strided over the blocks, or block (x, y,
+// z): tile x of width w_base + y of series z.
+__global__ void __launch_bounds__(HIT_THREADS) k_write_hits(WidthCtx ctx, HitBuffers hb,
+                                                            int w_base) {
+  __shared__ unsigned wsum[HIT_THREADS / 32];
+  if (!hb.sel_valid) {
+    write_hits_tile(ctx, hb, blockIdx.z, w_base + blockIdx.y, blockIdx.x, wsum);
+    return;
+  }
+  const unsigned n = *hb.sel_ts_n;
+  for (unsigned idx = blockIdx.x; idx < n; idx += gridDim.x) {
+    unsigned ser, wi, tile;
+    sel_item(hb.sel_ts[idx], hb.ntiles, (unsigned)ctx.nw, &ser, &wi, &tile);
+    write_hits_tile(ctx, hb, ser, wi, tile, wsum);
+    __syncthreads();  // the warp sums are reused by the next item
   }
 }
 
@@ -1669,9 +1728,11 @@ __device__ bool hit_bound(float nrm, float thresh, float* dmin) {
   return true;
 }
 
-template <bool ALLV, bool MUL>
+// Hits of the widths in `widths` (SEL; else of all) among this thread's samples
+// of a tile.
+template <bool SEL, bool ALLV, bool MUL>
 __device__ __forceinline__ void count_vec_body(const float* tile, int offset, int nw1,
-                                               unsigned valid, const int* s_ahead,
+                                               unsigned widths, unsigned valid, const int* s_ahead,
                                                const int* s_behind, const float* s_norm,
                                                const float* s_dmin, float thresh,
                                                unsigned* cnt) {
@@ -1679,11 +1740,12 @@ __device__ __forceinline__ void count_vec_body(const float* tile, int offset, in
   for (int g = 0; g < 2; g++) {
     const int j0 = 1024 * g + 4 * threadIdx.x;
     float win[12];
-    vec_window(tile, j0, offset, win);
+    if (!SEL || (widths & 7u)) vec_window(tile, j0, offset, win);
     const unsigned vg = (valid >> (4 * g)) & 0xFu;
 #pragma unroll
     for (int wi = 0; wi < VH_MAXW; wi++) {
       if (wi >= nw1) break;
+      if (SEL && !((widths >> wi) & 1u)) continue;  // uniform across the block
       float d[4];
       vec_boxcar(tile, j0, offset, wi, s_ahead[wi], s_behind[wi], win, d);
       unsigned c = 0;
@@ -1702,106 +1764,166 @@ __device__ __forceinline__ void count_vec_body(const float* tile, int offset, in
   }
 }
 
-// Block (x, y): tiles [x * tpb, (x + 1) * tpb) of series y (tpb <= 8); the
-// next tile's window is copied (cp.async, double buffer) while the current one
-// is counted.  With group maxima (ctx.gmax, recorded by the block-RMS pass) a
-// tile whose covering groups all lie below a width's bound dmin cannot hold a
-// hit of that width (|d| <= group max < dmin for each of its samples, and
-// the test is d >= dmin); a tile that no width can hit gets zero counts
-// without being read.  Tiles with hits are appended to hb.tile_list.
+// The tiles and widths whose maxima (ctx.gmax, recorded by the block-RMS pass)
+// leave room for a hit.  A tile whose stretches' maxima all lie below a width's
+// bound dmin cannot hold a hit of that width (d <= |d| <= maximum < dmin for
+// each of its samples, and the test is d >= dmin).  Tiles that no
+// unscrunched width can hit, and those of a time-scrunched width that it
+// cannot, get zero counts; the others are listed for the count and write
+// passes.  A warp per series, its lanes tiles.  With the test at the head of
+// the count's blocks, for tiles only, selection and count took 309 us for
+// 8424 series x 16 tiles x 10 widths and 320 us for 1482 x 103 x 13; 70 and
+// 119 us so.
+__global__ void __launch_bounds__(128) k_select_tiles(WidthCtx ctx, HitBuffers hb, int nw1) {
+  const unsigned ser = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (ser >= (unsigned)ctx.nser) return;
+  const unsigned nt = hb.ntiles;
+  // lane w: the bound of width w; -1: never skipped (maxima are >= 0)
+  float skip = -1.f;
+  if (lane < ctx.nw) {
+    float dm = 0.f;
+    if (hit_bound(ctx.norm[(size_t)ser * ctx.nw + lane], ctx.thresh, &dm)) skip = dm;
+    hb.bound[(size_t)ser * ctx.nw + lane] = skip;
+  }
+  const unsigned n1 = ctx.winfo[0].n;  // of the unscrunched widths
+  // some maximum of gm[k0..k1] reaches the bound, or one is missing; bit
+  // patterns of non-negative floats order as unsigned.  The first five (a tile
+  // has no more where the groups are 3125 samples) are loaded together.
+  auto reaches = [&](const float* gm, unsigned n, unsigned k0, unsigned k1, float bound) {
+    if (k1 >= n) return true;
+    unsigned mk = 0;
+#pragma unroll
+    for (unsigned j = 0; j < 5; j++) mk = max(mk, __float_as_uint(gm[min(k0 + j, k1)]));
+    for (unsigned k = k0 + 5; k <= k1; k++) mk = max(mk, __float_as_uint(gm[k]));
+    return !(__uint_as_float(mk) < bound);
+  };
+  auto stretch = [&](unsigned i) {
+    return i / ctx.gsize * ctx.gsteps + i % ctx.gsize / GMAX_STEP;
+  };
+  auto append = [&](bool need, unsigned* list, unsigned* n, unsigned entry) {
+    const unsigned b = __ballot_sync(0xffffffffu, need);
+    unsigned at = 0;
+    if (b && lane == 0) at = atomicAdd(n, (unsigned)__popc(b));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(b & ((1u << lane) - 1u));
+    if (need) list[at] = entry;
+    return at;
+  };
+  for (unsigned t0 = 0; t0 < nt; t0 += 32) {
+    const unsigned t = t0 + lane;
+    const bool in = t < nt;
+    const unsigned i0 = t * HIT_TILE, i1 = i0 + HIT_TILE - 1;
+    unsigned widths = 0, k0 = 0, k1 = 0;
+    if (i0 < n1) {
+      k0 = stretch(i0);
+      k1 = stretch(min(i1, n1 - 1));
+    }
+#pragma unroll 4
+    for (int wi = 0; wi < nw1; wi++) {
+      const float bound = __shfl_sync(0xffffffffu, skip, wi);
+      if (in && i0 < n1 &&
+          reaches(ctx.gmax + ((size_t)ser * ctx.gmax_nw + wi) * ctx.ngmax, ctx.ngmax, k0, k1,
+                  bound))
+        widths |= 1u << wi;
+    }
+    if (in && !widths)
+      for (int wi = 0; wi < nw1; wi++)
+        hb.tile_cnt[((size_t)ser * ctx.nw + wi) * nt + t] = 0;
+    const unsigned at = append(widths != 0, hb.sel, hb.sel_n, ser * nt + t);
+    if (widths) hb.sel_widths[at] = widths;
+    for (int wi = nw1; wi < ctx.nw; wi++) {
+      const float bound = __shfl_sync(0xffffffffu, skip, wi);
+      const size_t sw = (size_t)ser * ctx.nw + wi;
+      const int tk = wi - ctx.gmax_nw;
+      bool w_need = in && i0 < ctx.winfo[wi].n;
+      if (w_need && tk >= 0 && tk < TS_GMAX && ctx.ts_ngroups[tk] > 0)
+        w_need = reaches(ctx.gmax + ctx.ts_gmax[tk] + (size_t)ser * ctx.ts_ngroups[tk],
+                         ctx.ts_ngroups[tk], i0 / ctx.ts_gsize[tk], i1 / ctx.ts_gsize[tk], bound);
+      if (in && !w_need) hb.tile_cnt[sw * nt + t] = 0;
+      append(w_need, hb.sel_ts, hb.sel_ts_n, (unsigned)(sw * nt + t));
+    }
+  }
+}
+
+// Counts of the listed tiles (SEL), strided over the blocks, or of all widths of
+// every tile, an equal share of them per block; the next tile's window is copied (cp.async, double buffer) while the
+// current one is counted.  Tiles with hits are appended to hb.tile_list.
+template <bool SEL>
 __global__ void __launch_bounds__(HIT_THREADS) k_count_hits_vec(WidthCtx ctx, HitBuffers hb,
                                                                 int nw1, size_t slen,
-                                                                size_t span4, int tpb) {
+                                                                size_t span4) {
   extern __shared__ __align__(16) float tiles[];  // [2][span4]
   __shared__ int s_ahead[VH_MAXW], s_behind[VH_MAXW];
-  __shared__ float s_norm[VH_MAXW], s_dmin[VH_MAXW], s_skip[VH_MAXW];
+  __shared__ float s_norm[VH_MAXW], s_dmin[VH_MAXW];
   __shared__ int s_mul;
-  __shared__ unsigned s_need;
   __shared__ unsigned red[HIT_THREADS / 32][VH_MAXW / 2];
-  const size_t ser = blockIdx.y;
-  const unsigned t_begin = blockIdx.x * (unsigned)tpb;
-  const unsigned t_end = min(t_begin + (unsigned)tpb, hb.ntiles);
-  const float thresh = ctx.thresh;
-  const float* sc = ctx.scan + ser * ctx.scan_pitch;
-  const bool use_gmax = ctx.gmax != nullptr && ctx.ngroups > 0 && ctx.gmax_nw >= nw1;
-  if (threadIdx.x == 0) {
-    s_mul = 0;
-    s_need = use_gmax ? 0u : 0xFFu;
+  const unsigned step = SEL ? gridDim.x : 1u;
+  unsigned n = SEL ? *hb.sel_n : (unsigned)ctx.nser * hb.ntiles;
+  unsigned idx = blockIdx.x;
+  if (!SEL) {
+    const unsigned share = (n + gridDim.x - 1) / gridDim.x;
+    idx *= share;
+    n = min(n, idx + share);
   }
-  __syncthreads();
+  if (idx >= n) return;
+  const float thresh = ctx.thresh;
+  const int offset = ctx.offset;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < (unsigned)nw1) {
     s_ahead[threadIdx.x] = ctx.winfo[threadIdx.x].ahead;
     s_behind[threadIdx.x] = ctx.winfo[threadIdx.x].behind;
-    const float nrm = ctx.norm[ser * ctx.nw + threadIdx.x];
-    s_norm[threadIdx.x] = nrm;
-    float dm = 0.f;
-    const bool ok = hit_bound(nrm, thresh, &dm);
-    if (!ok) atomicOr(&s_mul, 1);
-    s_dmin[threadIdx.x] = dm;
-    s_skip[threadIdx.x] = ok ? dm : -1.f;  // -1: never skipped (maxima are >= 0)
   }
-  if (t_begin >= t_end) return;  // uniform
-  const unsigned ntb = t_end - t_begin;
-  if (use_gmax) {
-    __syncthreads();
-    for (unsigned idx = threadIdx.x; idx < ntb * (unsigned)nw1; idx += blockDim.x) {
-      const unsigned ti = idx / (unsigned)nw1, wi = idx - ti * (unsigned)nw1;
-      const size_t i0 = (size_t)(t_begin + ti) * HIT_TILE;
-      const size_t g_lo = i0 / ctx.gsize, g_hi = (i0 + HIT_TILE - 1) / ctx.gsize;
-      bool need = true;
-      if (g_hi < ctx.ngroups) {
-        // bit patterns of non-negative floats (or NaN, which wins and keeps
-        // the tile) order as unsigned
-        const float* gm = ctx.gmax + (ser * (size_t)ctx.gmax_nw + wi) * ctx.ngroups;
-        unsigned mk = 0;
-        for (size_t g = g_lo; g <= g_hi; g++) mk = max(mk, __float_as_uint(gm[g]));
-        need = !(__uint_as_float(mk) < s_skip[wi]);
-      }
-      if (need) atomicOr(&s_need, 1u << ti);
-    }
-    __syncthreads();
-    // skipped tiles: zero counts (read by the scans and the write pass)
-    for (unsigned idx = threadIdx.x; idx < ntb * (unsigned)nw1; idx += blockDim.x) {
-      const unsigned ti = idx / (unsigned)nw1, wi = idx - ti * (unsigned)nw1;
-      if (!((s_need >> ti) & 1u))
-        hb.tile_cnt[(ser * ctx.nw + wi) * hb.ntiles + t_begin + ti] = 0;
-    }
-  }
-  unsigned rest = s_need & ((1u << ntb) - 1u);
-  if (!rest) return;  // uniform
-  const int offset = ctx.offset;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned t = t_begin + (unsigned)(__ffs(rest) - 1);
-  rest &= rest - 1u;
-  int bi = 0;
-  vec_prefetch(sc, (size_t)t * HIT_TILE, tiles, span4, slen);
-  for (;;) {
-    float* tile = tiles + (size_t)bi * span4;
+  auto prefetch = [&](unsigned e, float* tile) {
+    vec_prefetch(ctx.scan + (size_t)(e / hb.ntiles) * ctx.scan_pitch,
+                 (size_t)(e % hb.ntiles) * HIT_TILE, tile, span4, slen);
+  };
+  auto item = [&](unsigned k) { return SEL ? hb.sel[k] : k; };
+  auto item_widths = [&](unsigned k) { return SEL ? hb.sel_widths[k] : ~0u; };
+  unsigned e = item(idx), widths = item_widths(idx);
+  prefetch(e, tiles);
+  size_t known = ~(size_t)0;  // warp 0: the series whose bounds are in place
+  for (int bi = 0;; bi ^= 1) {
+    const float* tile = tiles + (size_t)bi * span4;
+    const size_t ser = e / hb.ntiles;
+    const unsigned t = e % hb.ntiles;
     // the previous tile is counted and its reduction slots are read
     __syncthreads();
-    const bool more = rest != 0u;
-    unsigned tn = 0;
-    if (more) {
-      tn = t_begin + (unsigned)(__ffs(rest) - 1);
-      rest &= rest - 1u;
-      vec_prefetch(sc, (size_t)tn * HIT_TILE, tiles + (size_t)(bi ^ 1) * span4, span4, slen);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+    idx += step;
+    const bool more = idx < n;
+    const unsigned next = more ? item(idx) : 0u, next_widths = more ? item_widths(idx) : 0u;
+    if (more) prefetch(next, tiles + (size_t)(bi ^ 1) * span4);
+    if (warp == 0 && ser != known) {
+      bool ok = true;
+      if (lane < nw1) {
+        const float nrm = ctx.norm[ser * ctx.nw + lane];
+        float dm = 0.f;
+        if (SEL) {
+          dm = hb.bound[ser * ctx.nw + lane];
+          ok = dm != -1.f;
+        } else {
+          ok = hit_bound(nrm, thresh, &dm);
+        }
+        s_norm[lane] = nrm;
+        s_dmin[lane] = dm;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (lane == 0) s_mul = !ok;
+      known = ser;
     }
+    if (more) cp_async_wait<1>();
+    else cp_async_wait<0>();
     __syncthreads();
-    const size_t i0 = (size_t)t * HIT_TILE;
     bool allv;
-    const unsigned valid = vec_valid(ctx, i0, &allv);
+    const unsigned valid = vec_valid(ctx, (size_t)t * HIT_TILE, &allv);
     unsigned cnt[VH_MAXW / 2];
 #pragma unroll
     for (int p = 0; p < VH_MAXW / 2; p++) cnt[p] = 0;
     if (s_mul) {
-      if (allv) count_vec_body<true, true>(tile, offset, nw1, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
-      else count_vec_body<false, true>(tile, offset, nw1, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
+      if (allv) count_vec_body<SEL, true, true>(tile, offset, nw1, widths, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
+      else count_vec_body<SEL, false, true>(tile, offset, nw1, widths, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
     } else {
-      if (allv) count_vec_body<true, false>(tile, offset, nw1, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
-      else count_vec_body<false, false>(tile, offset, nw1, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
+      if (allv) count_vec_body<SEL, true, false>(tile, offset, nw1, widths, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
+      else count_vec_body<SEL, false, false>(tile, offset, nw1, widths, valid, s_ahead, s_behind, s_norm, s_dmin, thresh, cnt);
     }
 #pragma unroll
     for (int p = 0; p < VH_MAXW / 2; p++) {
@@ -1821,10 +1943,10 @@ __global__ void __launch_bounds__(HIT_THREADS) k_count_hits_vec(WidthCtx ctx, Hi
       if (tot) atomicAdd(&hb.sw_cnt[sw], tot);
     }
     if (__syncthreads_or(tot != 0u) && threadIdx.x == 0 && hb.tile_list)
-      hb.tile_list[atomicAdd(hb.tile_list_n, 1u)] = (unsigned)(ser * hb.ntiles + t);
+      hb.tile_list[atomicAdd(hb.tile_list_n, 1u)] = e;
     if (!more) break;
-    t = tn;
-    bi ^= 1;
+    e = next;
+    widths = next_widths;
   }
 }
 
@@ -1940,7 +2062,7 @@ static bool vec_hits_ok(const WidthCtx& ctx, int nw1) {
 
 cudaError_t count_hits(const WidthCtx& ctx, HitBuffers& hb, unsigned ntiles, cudaStream_t s) {
   hb.ntiles = ntiles;
-  hb.list_valid = false;
+  hb.list_valid = hb.sel_valid = false;
   cudaError_t e = cudaMemsetAsync(hb.sw_cnt, 0, ((size_t)ctx.nser * ctx.nw + 1) * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   // unscrunched widths share one staged window per tile
@@ -1949,20 +2071,22 @@ cudaError_t count_hits(const WidthCtx& ctx, HitBuffers& hb, unsigned ntiles, cud
   const size_t smem = (HIT_TILE + 2 * (size_t)ctx.offset + 2) * sizeof(float);
   const size_t span4 = (HIT_TILE + 2 * (size_t)ctx.offset + 2 + 3) & ~(size_t)3;
   const size_t slen = ctx.scan_len;
-  if (vec_hits_ok(ctx, nw1) && 2 * span4 * sizeof(float) <= 200 * 1024) {
-    if ((e = raise_smem_limit(k_count_hits_vec, 2 * span4 * sizeof(float))) != cudaSuccess)
-      return e;
-    if (hb.tile_list) {
-      if ((e = cudaMemsetAsync(hb.tile_list_n, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
-      hb.list_valid = true;
+  if (vec_hits_ok(ctx, nw1) && 2 * span4 * sizeof(float) <= 200 * 1024 && ctx.nw <= 32 &&
+      (size_t)ctx.nser * ctx.nw * ntiles < 0xFFFFFFFFull) {
+    // the three lists' lengths
+    if ((e = cudaMemsetAsync(hb.tile_list_n, 0, 3 * sizeof(unsigned), s)) != cudaSuccess) return e;
+    hb.list_valid = true;
+    const size_t all = (size_t)ctx.nser * ntiles;
+    // (with no more tiles than blocks at once, counting them all is the
+    // quicker: 11 us for 55 series of 4 tiles, 19 with the selection)
+    hb.sel_valid = ctx.gmax && ctx.ngmax > 0 && ctx.gmax_nw >= nw1 && select_pays(ctx.nser, ntiles);
+    if (hb.sel_valid) {
+      k_select_tiles<<<(unsigned)((ctx.nser + 3) / 4), 128, 0, s>>>(ctx, hb, nw1); note_launch();
     }
-    // about 8 consecutive tiles per block (at most 8), spread evenly; fewer
-    // where that leaves the SMs without two blocks each (55 series of 4 tiles:
-    // 11 us with a tile per block against 19 with four)
-    const unsigned nbx = std::max((ntiles + 7) / 8, std::min(ntiles, 296u / (unsigned)ctx.nser + 1));
-    const unsigned tpb = (ntiles + nbx - 1) / nbx;
-    k_count_hits_vec<<<dim3((ntiles + tpb - 1) / tpb, ctx.nser), HIT_THREADS,
-                       2 * span4 * sizeof(float), s>>>(ctx, hb, nw1, slen, span4, (int)tpb); note_launch();
+    auto kern = hb.sel_valid ? k_count_hits_vec<true> : k_count_hits_vec<false>;
+    if ((e = raise_smem_limit(kern, 2 * span4 * sizeof(float))) != cudaSuccess) return e;
+    kern<<<(unsigned)std::min<size_t>(all, 148 * 8), HIT_THREADS, 2 * span4 * sizeof(float), s>>>(
+        ctx, hb, nw1, slen, span4); note_launch();
   } else if (nw1 > 0 && smem <= 200 * 1024) {
     if ((e = raise_smem_limit(k_count_hits_multi, smem)) != cudaSuccess) return e;
     k_count_hits_multi<<<dim3(ntiles, ctx.nser), HIT_THREADS, smem, s>>>(ctx, hb, nw1, slen); note_launch();
@@ -1970,7 +2094,10 @@ cudaError_t count_hits(const WidthCtx& ctx, HitBuffers& hb, unsigned ntiles, cud
     nw1 = 0;
   }
   if (nw1 < ctx.nw) {
-    k_count_hits<<<dim3(ntiles, ctx.nw - nw1, ctx.nser), HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
+    const dim3 grid = hb.sel_valid
+                          ? dim3((unsigned)std::min<size_t>((size_t)ctx.nser * ntiles, 148 * 8))
+                          : dim3(ntiles, ctx.nw - nw1, ctx.nser);
+    k_count_hits<<<grid, HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
   }
   return cudaGetLastError();
 }
@@ -2007,8 +2134,11 @@ cudaError_t write_hits(const WidthCtx& ctx, HitBuffers& hb, cudaStream_t s) {
   if (nw1 < ctx.nw) {
     unsigned n = 1;  // tiles past every such width's samples hold nothing
     for (int w = nw1; w < ctx.nw; w++) n = std::max(n, ctx.host_winfo[w].n);
-    k_write_hits<<<dim3(std::min(hb.ntiles, (n + HIT_TILE - 1) / HIT_TILE), ctx.nw - nw1,
-                        ctx.nser), HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
+    const unsigned nt = std::min(hb.ntiles, (n + HIT_TILE - 1) / HIT_TILE);
+    const dim3 grid = hb.sel_valid
+                          ? dim3((unsigned)std::min<size_t>((size_t)ctx.nser * nt, 148 * 8))
+                          : dim3(nt, ctx.nw - nw1, ctx.nser);
+    k_write_hits<<<grid, HIT_THREADS, 0, s>>>(ctx, hb, nw1); note_launch();
   }
   return cudaGetLastError();
 }

@@ -676,8 +676,7 @@ static hd_error enqueue_gulp(hd_pipeline pl, const GulpGeom& g,
   for (int w = n_ts1; w < nw; w++) HD_TRY(hdb::block_rms(wctx, wi.data(), w, w + 1, ws, s));
 
   hdb::HitBuffers hb{};
-  hb.tile_list = pl->tile_list.as<unsigned>();
-  hb.tile_list_n = hb.tile_list + g.NS * g.ntiles;
+  hb.set_lists(pl->tile_list.as<unsigned>(), g.NS, nw, g.ntiles);
   hb.tile_cnt = pl->tile_cnt.as<unsigned>();
   hb.tile_off = pl->tile_off.as<unsigned>();
   hb.sw_cnt = pl->sw_cnt.as<unsigned>();
@@ -780,7 +779,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   const size_t nw = wi.size();
   g.ntiles = (unsigned)((wi[0].n + 2047) / 2048);
   g.nsw = g.NS * nw;
-  g.gcap_groups = g.NS * nw * (nbeams * g.stride / 3125 + 5);
+  g.gcap_groups = hdb::gmax_floats(g.NS, nw, nbeams * g.stride);
 
   // every buffer at the size the host-sized path gives this shape, with the
   // hit and giant lists at the capacities
@@ -808,7 +807,8 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   need(pl->tile_off, g.nsw * g.ntiles * sizeof(unsigned));
   need(pl->sw_cnt, (g.nsw + 1) * sizeof(unsigned));
   need(pl->sw_off, (g.nsw + 1) * sizeof(unsigned));
-  need(pl->tile_list, (g.NS * g.ntiles + 1) * sizeof(unsigned));
+  need(pl->tile_list,
+       hdb::HitBuffers::hit_list_words(g.NS, nw, g.ntiles) * sizeof(unsigned));
   const size_t H = (size_t)hcap + 1, G = (size_t)gcap + 1;
   need(pl->hit_ind, H * sizeof(unsigned));
   need(pl->hit_val, H * sizeof(float));
@@ -1316,9 +1316,8 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
     wctx.dm_offset = (int)G.d0;
     wctx.norm = pl->norm.as<float>();
     wctx.thresh = P.detect_thresh;
-    // largest |boxcar| per block-RMS group (at most nbeams * stride / 5^5 + 4
-    // groups per series), read by the count pass to skip quiet tiles
-    const size_t gcap = NSg * (size_t)nw * (nbeams * stride_s / 3125 + 5);
+    // the boxcars' maxima, read by the count pass to skip quiet tiles
+    const size_t gcap = hdb::gmax_floats(NSg, nw, nbeams * stride_s);
     HD_TRY(pl->gmax.ensure(gcap * sizeof(float)));
     wctx.gmax = pl->gmax.as<float>();
     wctx.gmax_cap = gcap;
@@ -1334,9 +1333,9 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
     HD_TRY(pl->tile_off.ensure(nsw * ntiles * sizeof(unsigned)));
     HD_TRY(pl->sw_cnt.ensure((nsw + 1) * sizeof(unsigned)));
     HD_TRY(pl->sw_off.ensure((nsw + 1) * sizeof(unsigned)));
-    HD_TRY(pl->tile_list.ensure((NSg * ntiles + 1) * sizeof(unsigned)));
-    hb.tile_list = pl->tile_list.as<unsigned>();
-    hb.tile_list_n = hb.tile_list + NSg * ntiles;
+    HD_TRY(pl->tile_list.ensure(hdb::HitBuffers::hit_list_words(NSg, nw, ntiles) *
+                                sizeof(unsigned)));
+    hb.set_lists(pl->tile_list.as<unsigned>(), NSg, nw, ntiles);
     hb.tile_cnt = pl->tile_cnt.as<unsigned>();
     hb.tile_off = pl->tile_off.as<unsigned>();
     hb.sw_cnt = pl->sw_cnt.as<unsigned>();
