@@ -50,6 +50,36 @@ cudaError_t raise_smem_limit(const void* func, size_t bytes) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int tp_col(int t, int w) { return w ^ (((t >> 2) ^ (t & 3)) & 31); }
 
+// The staged tile's channel rows from sample t0 on.  Warp: channel words warp,
+// warp + 8, ...; lane: samples 4l .. 4l+3.
+__device__ __forceinline__ void transpose_store(const uint32_t* tile, size_t t0, size_t nsamps,
+                                                int c0, int nchans, uint8_t* __restrict__ out,
+                                                size_t pitch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t t = t0 + 4 * lane;
+  for (int ws = warp; ws < 32; ws += 8) {
+    if (4 * ws + c0 >= nchans) break;
+    uint32_t a[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int r = 4 * lane + j;
+      a[j] = tile[r * 32 + tp_col(r, ws)];
+    }
+    // 4 x 4 byte transpose: o[b] = byte b of a[0..3]
+    const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), lo23 = __byte_perm(a[2], a[3], 0x5140);
+    const uint32_t hi01 = __byte_perm(a[0], a[1], 0x7362), hi23 = __byte_perm(a[2], a[3], 0x7362);
+    const uint32_t o[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                           __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
+    if (t < nsamps) {
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const int c = c0 + 4 * ws + b;
+        if (c < nchans) reinterpret_cast<uint32_t*>(out + (size_t)c * pitch + t)[0] = o[b];
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) k_transpose_tf_ft(const uint8_t* __restrict__ in,
                                                          size_t nsamps, int nchans,
                                                          uint8_t* __restrict__ out,
@@ -99,30 +129,7 @@ __global__ void __launch_bounds__(256) k_transpose_tf_ft(const uint8_t* __restri
     }
   }
   __syncthreads();
-  // warp: channel words wsel = warp, warp + 8, ...; lane: samples 4l .. 4l+3
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t t = t0 + 4 * lane;
-  for (int ws = warp; ws < 32; ws += 8) {
-    if (4 * ws + c0 >= nchans) break;
-    uint32_t a[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int r = 4 * lane + j;
-      a[j] = tile[r * 32 + tp_col(r, ws)];
-    }
-    // 4 x 4 byte transpose: o[b] = byte b of a[0..3]
-    const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), lo23 = __byte_perm(a[2], a[3], 0x5140);
-    const uint32_t hi01 = __byte_perm(a[0], a[1], 0x7362), hi23 = __byte_perm(a[2], a[3], 0x7362);
-    const uint32_t o[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
-                           __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
-    if (t < nsamps) {
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const int c = c0 + 4 * ws + b;
-        if (c < nchans) reinterpret_cast<uint32_t*>(out + (size_t)c * pitch + t)[0] = o[b];
-      }
-    }
-  }
+  transpose_store(tile, t0, nsamps, c0, nchans, out, pitch);
 }
 
 // ---------------------------------------------------------------------------
@@ -256,48 +263,78 @@ __device__ uint32_t zap_word(const uint32_t* __restrict__ win, const int* __rest
 }
 
 // Zap masked spectra and write the result channel-major (FT), and optionally
-// time-major (TF) for callers that want the cleaned filterbank back.
+// time-major (TF) for callers that want the cleaned filterbank back.  Bound by
+// its reads and writes: the transpose's tile and word order, rows of whole
+// 16-byte words loaded 16 bytes at a time, and the masked rows filled in by a
+// warp each, a word per lane (their draws are long and few).  1024 channels x
+// 262144 samples: 330 us with a word per lane in every row and bytes gathered
+// one by one, 165 us so.
 __global__ void __launch_bounds__(256) k_zap_to_ft(const uint8_t* __restrict__ in, size_t nsamps,
                                                    int nchans, const int* __restrict__ mask,
                                                    unsigned max_resample_dist,
                                                    uint8_t* __restrict__ out_ft, size_t pitch,
                                                    uint8_t* __restrict__ out_tf) {
-  __shared__ uint32_t tile[128][33];
+  __shared__ uint32_t tile[128 * 32];
   const size_t t0 = (size_t)blockIdx.x * 128;
   const int c0 = blockIdx.y * 128;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned stride = (unsigned)(nchans >> 2);
+  const unsigned w0 = (unsigned)(c0 >> 2);
   const uint32_t* win = reinterpret_cast<const uint32_t*>(in);
-  for (int r = warp; r < 128; r += 8) {
-    size_t t = t0 + r;
-    unsigned w = (unsigned)(c0 >> 2) + lane;
-    uint32_t v = 0;
-    if (t < nsamps && w < stride) {
-      if (mask[t]) {
-        unsigned i = (unsigned)t * stride + w;
-        v = zap_word(win, mask, i, (unsigned)t, w, stride, (unsigned)nsamps, max_resample_dist);
-      } else {
-        v = win[t * stride + w];
-      }
-      if (out_tf) reinterpret_cast<uint32_t*>(out_tf)[t * stride + w] = v;
+  // ---- the rows that stay as they are ----
+  if ((nchans & 15) == 0 &&
+      ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out_tf)) & 15) == 0) {
+    // thread: 16-byte chunk q of rows r0, r0 + 32, r0 + 64, r0 + 96
+    const int q = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const unsigned w = w0 + 4 * q;
+    uint4 v[4];
+    bool masked[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const size_t t = t0 + r0 + 32 * k;
+      const bool in_data = t < nsamps && w < stride;
+      v[k] = make_uint4(0u, 0u, 0u, 0u);
+      masked[k] = t < nsamps && mask[t] != 0;
+      if (in_data) v[k] = *reinterpret_cast<const uint4*>(win + t * stride + w);
     }
-    tile[r][lane] = v;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (masked[k]) continue;
+      const int r = r0 + 32 * k;
+      tile[r * 32 + tp_col(r, 4 * q)] = v[k].x;
+      tile[r * 32 + tp_col(r, 4 * q + 1)] = v[k].y;
+      tile[r * 32 + tp_col(r, 4 * q + 2)] = v[k].z;
+      tile[r * 32 + tp_col(r, 4 * q + 3)] = v[k].w;
+      if (out_tf && t0 + r < nsamps && w < stride)
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint32_t*>(out_tf) + (t0 + r) * stride + w) =
+            v[k];
+    }
+  } else {
+    for (int r = warp; r < 128; r += 8) {
+      const size_t t = t0 + r;
+      if (t < nsamps && mask[t]) continue;
+      const bool in_data = t < nsamps && w0 + lane < stride;
+      const uint32_t v = in_data ? win[t * stride + w0 + lane] : 0u;
+      tile[r * 32 + tp_col(r, lane)] = v;
+      if (out_tf && in_data) reinterpret_cast<uint32_t*>(out_tf)[t * stride + w0 + lane] = v;
+    }
+  }
+  // ---- the masked rows: warp w those of rows w, w + 8, ... ----
+  const size_t tl = t0 + warp + 8 * lane;
+  unsigned todo = __ballot_sync(0xffffffffu, lane < 16 && tl < nsamps && mask[tl] != 0);
+  for (; todo; todo &= todo - 1) {
+    const int r = warp + 8 * (__ffs(todo) - 1);
+    const unsigned t = (unsigned)(t0 + r), w = w0 + lane;
+    uint32_t v = 0u;
+    if (w < stride) {
+      v = zap_word(win, mask, t * stride + w, t, w, stride, (unsigned)nsamps, max_resample_dist);
+      if (out_tf) reinterpret_cast<uint32_t*>(out_tf)[(size_t)t * stride + w] = v;
+    }
+    tile[r * 32 + tp_col(r, lane)] = v;
   }
   if (!out_ft) return;
   __syncthreads();
-  for (int cr = warp; cr < 128; cr += 8) {
-    int c = c0 + cr;
-    if (c >= nchans) break;
-    int wsel = cr >> 2, bsel = cr & 3;
-    uint32_t o = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      uint32_t v = tile[4 * lane + j][wsel];
-      o |= ((v >> (8 * bsel)) & 0xFFu) << (8 * j);
-    }
-    size_t t = t0 + 4 * lane;
-    if (t < nsamps) reinterpret_cast<uint32_t*>(out_ft + (size_t)c * pitch + t)[0] = o;
-  }
+  transpose_store(tile, t0, nsamps, c0, nchans, out_ft, pitch);
 }
 
 // ---------------------------------------------------------------------------

@@ -1101,7 +1101,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // while the current group's medians are computed.  Of 8424 series x 28000
 // samples x 10 widths: 1.03 ms with runs of 20 samples as float4 loads, whose
 // level-1 medians went through shared memory (bound by its bandwidth, 84 %, and
-// 12400 instructions a group), 0.71 ms so (issue 78 %, min/max pipe 68 %).
+// 12400 instructions a group), 0.71 ms so, 0.81 with the maxima per 800 samples
+// and of the rest
+// (issue 78 %, min/max pipe 65 %).
 template <int M>
 __global__ void __launch_bounds__(BRV_THREADS, 2) k_block_rms_pass1_vec(
     WidthCtx ctx, int nwb, int win, float* __restrict__ out, size_t out_pitch, int ngroups,
