@@ -74,10 +74,6 @@ struct DedispArgs {
   // test of the error path: the producer issues no copy for the last stage,
   // so the consumers' wait on it runs out (HDB_TEST_WITHHOLD_STAGE=1)
   int withhold_last;
-  // always 1: the multiplier of the kernel's multiply-add accumulations.  A
-  // runtime value keeps them multiply-adds, which issue to the FMA pipe and
-  // leave the ALU pipe (byte permutes, adds) to the rest of the work
-  unsigned one;
 };
 
 // Dedispersion tile: DMs and output samples per CTA (a quarter of them words

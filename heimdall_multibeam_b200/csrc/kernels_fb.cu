@@ -529,8 +529,8 @@ __global__ void k_nb_zap(uint32_t* __restrict__ data, size_t nsamps, int units, 
 // and stores the float.  The sums are exact integers in any order.
 //
 // What bounds it: one shared load per word, DM and channel (128 sample terms a
-// wavefront), so the shared-memory pipe (75 % busy in ncu) and instruction
-// issue (70 %).  Measured sample-channel adds per second, the tile from the
+// wavefront), so the shared-memory pipe (84 % busy in ncu) and instruction
+// issue (76 %).  Measured sample-channel adds per second, the tile from the
 // autotuner, against the byte-row kernel before it (8 x 1280 samples, funnel
 // shifts to realign): 4096 channels, DM 0-500: 28.2 T/s (19.2); 1024 channels,
 // DM 0-2000: 26.7 (16.8); 256 channels, DM 0-1000: 20.4 (15.0); 36 x 320

@@ -444,7 +444,6 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   a.out_unit = out_unit;
   a.wait_limit = kDedispWaitLimit;
   a.withhold_last = 0;
-  a.one = 1;
   // error-path test (read per call so a test can clear it between gulps):
   // the last channel stage is withheld and the waits give up quickly
   if (const char* e = std::getenv("HDB_TEST_WITHHOLD_STAGE"))
