@@ -476,9 +476,16 @@ __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
   return __fdiv_rn(a, b);
 }
 
+// Whether blocks of `ser` series keep their RMS values and reciprocals in shared
+// memory: decided from the launch's series per block, for its last block too,
+// which may hold fewer series but gets no more shared memory than the others.
+__host__ __device__ constexpr bool sc_rms_in_smem(int ser, int nbeams) {
+  return (long long)ser * nbeams <= SC_MAXRMS;
+}
+
 size_t scan_smem_bytes(int ser, int nbeams, int ch) {
   size_t b = 128 + (size_t)sc_nb(ch) * ser * (ch + 4) * sizeof(float);
-  if ((size_t)ser * nbeams <= SC_MAXRMS) b += 2 * (size_t)ser * nbeams * sizeof(float);
+  if (sc_rms_in_smem(ser, nbeams)) b += 2 * (size_t)ser * nbeams * sizeof(float);
   return b;
 }
 
@@ -505,7 +512,7 @@ __global__ void __launch_bounds__(CH >= 512 ? 160 : 256, CH >= 512 ? 3 : 4) k_no
   const int nb = min(S, nser - s0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int np = (int)(blockDim.x >> 5) - 1;
-  const bool rms_smem = nb * nbeams <= SC_MAXRMS;
+  const bool rms_smem = sc_rms_in_smem(S, nbeams);
   const unsigned nstage = len / CH + 1;     // outputs 0..len
   const unsigned len4 = (len + 3u) & ~3u;   // copies round up to 16 bytes (inside the row pitch)
 
