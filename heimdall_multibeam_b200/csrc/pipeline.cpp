@@ -140,9 +140,25 @@ struct hd_pipeline_t {
   // host-sized path and fixes the shape's hit and giant capacities and its
   // number of clustering sweep pairs; later gulps of the shape replay one
   // graph per set of device buffers.
+  //
+  // When to capture: a capture costs 2 ms (a gulp of 64 channels x 8192 spectra,
+  // 256 x 65536) to 5 ms (36 x 320 x 32768) and a replay saves 0.08 to 0.12 ms
+  // of the host-sized path (0.41 -> 0.33 ms of the smallest), so a graph pays
+  // after 25 to 50 replays.  A pipeline of a few shapes is taken for a steady
+  // stream and captures a shape at its first return.  With more shapes (gulp
+  // lengths that vary) a shape must first come back kReturns times without a
+  // graph, and again whenever its graph is lost to other shapes or to buffers
+  // that have moved: what captures cost stays below about what the host-sized
+  // gulps before them took over replays, in any order of lengths.
+  static constexpr size_t kFewShapes = 3;      // shapes of a pipeline that captures at once
+  static constexpr unsigned kReturns = 32;     // returns before a capture with more of them
+  static constexpr size_t kMaxShapes = 64, kMaxGraphs = 32;
+  static constexpr size_t kShapeGraphs = 3;    // sets of buffers: the input rotates over three
   struct GraphShape {
     std::vector<size_t> key;
     unsigned hcap = 0, gcap = 0, pairs = 0;
+    unsigned returns = 0;  // gulps without a graph to replay since one was last lost
+    unsigned long long used = 0;
     bool broken = false;  // capture failed: this shape stays on the host-sized path
   };
   struct GraphGulp {
@@ -162,16 +178,49 @@ struct hd_pipeline_t {
   DevBuf geo, gflags;
   // what the last host-sized gulp saw (sizes a new shape's capacities)
   unsigned obs_hits = 0, obs_giants = 0, obs_pairs = 0;
+  static bool of_shape(const GraphGulp& g, const std::vector<size_t>& shape) {
+    return g.key.size() >= shape.size() &&
+           std::equal(shape.begin(), shape.end(), g.key.begin());
+  }
   void drop_graphs(const std::vector<size_t>& shape) {
     for (size_t i = 0; i < graphs.size();) {
-      const auto& k = graphs[i].key;
-      if (k.size() >= shape.size() && std::equal(shape.begin(), shape.end(), k.begin())) {
+      if (of_shape(graphs[i], shape)) {
         if (graphs[i].exec) cudaGraphExecDestroy(graphs[i].exec);
         graphs.erase(graphs.begin() + i);
       } else {
         i++;
       }
     }
+  }
+  size_t graphs_of(const GraphShape& gs) const {
+    size_t n = 0;
+    for (const GraphGulp& g : graphs) n += of_shape(g, gs.key);
+    return n;
+  }
+  // Whether a gulp of the shape that found no graph to replay is to capture
+  // one (the rule above); if so there is room for it.
+  bool may_capture(GraphShape& gs) {
+    const bool many = graph_shapes.size() > kFewShapes;
+    const bool full = graphs_of(gs) >= kShapeGraphs;
+    if (full && many) {  // their buffers have moved
+      drop_graphs(gs.key);
+      gs.returns = 0;
+    }
+    if (++gs.returns < (many ? kReturns : 1)) return false;
+    if ((full && !many) || graphs.size() >= kMaxGraphs) {
+      // the least recently used one goes (of this shape's, where it has its
+      // share), and its shape waits again
+      size_t old = graphs.size();
+      for (size_t i = 0; i < graphs.size(); i++)
+        if ((!full || of_shape(graphs[i], gs.key)) &&
+            (old == graphs.size() || graphs[i].used < graphs[old].used))
+          old = i;
+      for (GraphShape& x : graph_shapes)
+        if (of_shape(graphs[old], x.key)) x.returns = 0;
+      cudaGraphExecDestroy(graphs[old].exec);
+      graphs.erase(graphs.begin() + old);
+    }
+    return true;
   }
 
   unsigned* h_small = nullptr;  // pinned host words
@@ -760,7 +809,10 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
     pl->pending_shape = shape;
     return false;
   }
+  gs->used = ++pl->graph_clock;
   if (gs->broken) return false;
+  bool capture = false;  // asked before the lists are grown where there is nothing to replay
+  if (pl->graphs_of(*gs) == 0 && !(capture = pl->may_capture(*gs))) return false;
   const unsigned hcap = gs->hcap, gcap = gs->gcap, pairs = gs->pairs;
 
   g.dm_tol = std::min<size_t>(P.cand_sep_dm, g.D);
@@ -866,6 +918,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   hd_pipeline_t::GraphGulp* gg = nullptr;
   for (auto& x : pl->graphs)
     if (x.key == key) gg = &x;
+  if (!gg && !capture && !pl->may_capture(*gs)) return false;
   if (!gg) {
     hd_pipeline_t::GraphGulp ng;
     ng.key = key;
@@ -894,15 +947,6 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
       cudaGetLastError();
       gs->broken = true;
       return false;
-    }
-    // a few graphs per pipeline (the prefetched form rotates three input
-    // buffers); the least recently used goes
-    if (pl->graphs.size() >= 6) {
-      size_t old = 0;
-      for (size_t i = 1; i < pl->graphs.size(); i++)
-        if (pl->graphs[i].used < pl->graphs[old].used) old = i;
-      cudaGraphExecDestroy(pl->graphs[old].exec);
-      pl->graphs.erase(pl->graphs.begin() + old);
     }
     pl->graphs.push_back(ng);
     gg = &pl->graphs.back();
@@ -1562,9 +1606,16 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
   pl->timing[6] = el(6, 7);
   if (!pl->pending_shape.empty()) {
     // a new shape for the graph form: capacities from what this gulp saw
-    if (pl->graph_shapes.size() >= 64) pl->graph_shapes.erase(pl->graph_shapes.begin());
+    if (pl->graph_shapes.size() >= hd_pipeline_t::kMaxShapes) {
+      size_t old = 0;
+      for (size_t i = 1; i < pl->graph_shapes.size(); i++)
+        if (pl->graph_shapes[i].used < pl->graph_shapes[old].used) old = i;
+      pl->drop_graphs(pl->graph_shapes[old].key);
+      pl->graph_shapes.erase(pl->graph_shapes.begin() + old);
+    }
     hd_pipeline_t::GraphShape gsh;
     gsh.key = pl->pending_shape;
+    gsh.used = ++pl->graph_clock;
     gsh.hcap = graph_capacity(pl->obs_hits, 1u << 16);
     gsh.gcap = graph_capacity(pl->obs_giants, 1u << 14);
     gsh.pairs = std::min(std::max(pl->obs_pairs + 1, 2u), 16u);

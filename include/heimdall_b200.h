@@ -425,7 +425,10 @@ unsigned long long hd_get_launch_count(void);
  * capacities and its number of clustering sweeps; later gulps of the shape
  * copy their input into the pipeline's buffer, wherever it comes from, and
  * launch one captured graph with every total kept on the device, and the host
- * reads the results once.  A gulp whose totals exceed the capacities, or whose
+ * reads the results once.  A pipeline that has seen more than three shapes (gulp
+ * lengths that vary) captures a shape only once it has come back 32 times without
+ * a graph, which is about what a capture costs; until then such gulps stay on the
+ * host-sized path.  A gulp whose totals exceed the capacities, or whose
  * clustering needs more sweeps, is searched again on the host-sized path and
  * the shape's capacities grow: results never depend on the form.  Adaptive dt,
  * narrow-band zapping and 16-bit input stay on the host-sized path, and so do
