@@ -57,7 +57,9 @@ struct DedispArgs {
   size_t in_pitch;        // words
   int split;              // word t holds samples t + q*split, q = 0..3
   const int* delays;      // [dm_count][nchans] delay in samples
-  const int2* blk_range;  // [n_dm_blocks][nchans] least and largest delay of the block's DMs
+  // [n_dm_blocks][nchans] least and largest delay of the block's DMs (not read
+  // by tiles of one trial)
+  const int2* blk_range;
   const int* chans;       // active (not killed) channel indices
   int nact;
   int nchans;
@@ -97,6 +99,11 @@ constexpr int kDedispRows = 32;  // channel rows per stage at most
 int dedisp_stage_bytes(int dm_block, int time_block, int mean_row, int longest_row);
 size_t dedisp_smem_bytes(int dm_block, int time_block, int cap);
 cudaError_t launch_dedisp(const DedispArgs& a, const DedispTile& t, cudaStream_t s);
+// Least and largest delay of each block of `db` trials and channel of the delays
+// [ntrials][nchans]; the largest span and the spans' sum into span[0], span[1]
+// (zero before).
+cudaError_t launch_block_ranges(const int* delays, size_t ntrials, size_t nchans, int db,
+                                int2* range, unsigned long long* span, cudaStream_t s);
 // Four-sample words of the channel-major byte rows of `units` inputs: word t
 // (t < nwords) of a row = samples t + q*split, q = 0..3.  Pitches and units in
 // bytes (in, multiples of 16) and words (out, multiples of 16 and 4).

@@ -602,7 +602,12 @@ __global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT,
     auto channel = [&](int k0) {
       const bool have = lane < CH && k0 + lane < a.nact;
       c = have ? a.chans[k0 + lane] : 0;
-      r = have ? brange[c] : make_int2(0, 0);
+      if constexpr (DB == 1) {
+        const int dl = have ? a.delays[(size_t)d_lo * a.nchans + c] : 0;
+        r = make_int2(dl, dl);
+      } else {
+        r = have ? brange[c] : make_int2(0, 0);
+      }
     };
     channel(0);
     int st = 0;
@@ -778,6 +783,35 @@ __global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT,
     if (lane == 0) mbar_arrive(&empty[buf]);
   }
   flush(first, true);
+}
+
+// Least and largest delay of each block of `db` trials, per channel, and over all
+// of them the largest span and the sum of the spans (span[0], span[1], from 0).
+// Thread: one channel of blocks blockIdx.y, + gridDim.y, ...
+__global__ void __launch_bounds__(256) k_block_ranges(const int* __restrict__ delays, int ntrials,
+                                                      int nchans, int db, int2* __restrict__ range,
+                                                      unsigned long long* __restrict__ span) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  unsigned most = 0;
+  unsigned long long sum = 0;
+  for (int b = blockIdx.y; (long long)b * db < ntrials && c < nchans; b += gridDim.y) {
+    int lo = 0x7FFFFFFF, hi = 0;  // (delays are not negative)
+    for (int d = b * db; d < min(ntrials, (b + 1) * db); d++) {
+      const int v = delays[(size_t)d * nchans + c];
+      lo = min(lo, v);
+      hi = max(hi, v);
+    }
+    range[(size_t)b * nchans + c] = make_int2(lo, hi);
+    most = max(most, (unsigned)(hi - lo));
+    sum += (unsigned)(hi - lo);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(span, (unsigned long long)most);
+    atomicAdd(span + 1, sum);
+  }
 }
 
 // Channel-major byte rows -> four-sample words: word t of channel c holds
@@ -1101,6 +1135,17 @@ cudaError_t launch_dedisp(const DedispArgs& a0, const DedispTile& t, cudaStream_
   HDB_DD_TILE(1, 1, 4, 1, 16)
 #undef HDB_DD_TILE
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_block_ranges(const int* delays, size_t ntrials, size_t nchans, int db,
+                                int2* range, unsigned long long* span, cudaStream_t s) {
+  if (ntrials < 1 || ntrials > 0x3FFFFFFFull || nchans < 1 || nchans > 0x3FFFFFFFull)
+    return cudaErrorInvalidValue;
+  const size_t nblk = (ntrials + db - 1) / db;
+  dim3 grid((unsigned)((nchans + 255) / 256), (unsigned)std::min<size_t>(nblk, 65535));
+  k_block_ranges<<<grid, 256, 0, s>>>(delays, (int)ntrials, (int)nchans, db, range, span);
+  note_launch();
+  return cudaGetLastError();
 }
 
 cudaError_t launch_split_words(const uint8_t* in, size_t in_pitch, size_t in_unit, int nchans,

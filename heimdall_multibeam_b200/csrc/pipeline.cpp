@@ -908,8 +908,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   }
   for (const void* q : {(const void*)plan->d_delays, (const void*)plan->d_blk_range[0],
                         (const void*)plan->d_blk_range[1], (const void*)plan->d_blk_range[2],
-                        (const void*)plan->d_blk_range[3], (const void*)plan->d_blk_range[4],
-                        (const void*)plan->d_words,
+                        (const void*)plan->d_blk_range[3], (const void*)plan->d_words,
                         (const void*)plan->d_active, (const void*)plan->d_dm_list,
                         (const void*)plan->d_err})
     key.push_back((size_t)q);

@@ -93,50 +93,94 @@ static void free_dev(void* p) {
   if (p) cudaFree(p);
 }
 
+static void free_ranges(int2** d_range) {
+  free_dev(d_range[0]);
+  free_dev(d_range[kDedispDmBlockSizes - 1]);
+  for (int k = 0; k < kDedispDmBlockSizes; k++) d_range[k] = nullptr;
+}
+
 static void free_groups(dedisp_plan p) {
   for (auto& g : p->groups) {
     free_dev(g.d_delays);
-    for (int2* b : g.d_blk_range) free_dev(b);
+    free_ranges(g.d_blk_range);
   }
   p->groups.clear();
 }
 
-// Per DM-block size: the least and the largest delay of every (block, channel),
-// and over those the largest and the mean span.
-static void block_ranges(const std::vector<int>& delays, size_t D, size_t C,
-                         std::vector<int2>* range, size_t* max_span, size_t* mean_span) {
-  for (int k = 0; k < kDedispDmBlockSizes; k++) {
-    const size_t DB = (size_t)kDedispDmBlocks[k];
-    const size_t nblk = (D + DB - 1) / DB;
-    range[k].resize(nblk * C);
-    max_span[k] = 0;
-    size_t sum = 0;
-    for (size_t b = 0; b < nblk; b++) {
-      int2* r = range[k].data() + b * C;
-      const size_t d1 = std::min(D, (b + 1) * DB);
-      for (size_t d = b * DB; d < d1; d++) {
-        const int* dl = delays.data() + d * C;
-        for (size_t c = 0; c < C; c++)
-          r[c] = d == b * DB ? int2{dl[c], dl[c]}
-                             : int2{std::min(r[c].x, dl[c]), std::max(r[c].y, dl[c])};
-      }
-      for (size_t c = 0; c < C; c++) {
-        max_span[k] = std::max(max_span[k], (size_t)(r[c].y - r[c].x));
-        sum += (size_t)(r[c].y - r[c].x);
-      }
-    }
-    mean_span[k] = range[k].empty() ? 0 : sum / range[k].size();
-  }
+// Bytes of a tile's staged row whose DM block spans `span` samples of delay:
+// the span and the tile's words, from a 16-byte boundary on (2^18, more than
+// fits, from 2^16 words on).
+static int row_bytes(size_t span, int time_block) {
+  const size_t words = span + 3 + (size_t)time_block / 4;
+  return words >= (size_t)1 << 16 ? 1 << 18 : (int)((4 * words + 15) & ~(size_t)15);
 }
 
-static dedisp_error upload_ranges(const std::vector<int2>* range, int2** d_range) {
-  for (int k = 0; k < kDedispDmBlockSizes; k++) {
-    const size_t bytes = range[k].size() * sizeof(int2);
-    if (dev_malloc(&d_range[k], bytes) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
-    if (cudaMemcpy(d_range[k], range[k].data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+static int dm_block_index(int dm_block) {
+  for (int k = 0; k < kDedispDmBlockSizes; k++)
+    if (kDedispDmBlocks[k] == dm_block) return k;
+  return -1;
+}
+
+// The delay span of a tile's DM blocks (one trial has none).
+static size_t span_of(const size_t* span, int dm_block) {
+  const int k = dm_block_index(dm_block);
+  return k < 0 ? 0 : span[k];
+}
+
+// Bytes of a tile's stage buffers (0: a row does not fit shared memory).
+static int stage_of(const size_t* max_span, const size_t* mean_span, const int* tile) {
+  return dedisp_stage_bytes(tile[0], tile[1], row_bytes(span_of(mean_span, tile[0]), tile[1]),
+                            row_bytes(span_of(max_span, tile[0]), tile[1]));
+}
+
+// Per DM-block size: the least and the largest delay of every (block, channel) of
+// the D x C delays on the device, and over those the largest and the mean span.
+// Made there: the tables are 7/16 of the delays' bytes and take no pass over them
+// on the host (the first gulp of a fresh pipeline of 1482 trials x 1024 channels:
+// 37 ms; 48 ms with five tables made there and uploaded, of blocks of one and two
+// trials among them).  The blocks of two trials come last, where no tile of the
+// other sizes fits.
+static dedisp_error build_ranges(const int* d_delays, size_t D, size_t C, int2** d_range,
+                                 size_t* max_span, size_t* mean_span) {
+  struct Spans {
+    unsigned long long largest, sum;
+  };
+  constexpr int kMain = kDedispDmBlockSizes - 1;
+  auto blocks = [&](int k) { return (D + kDedispDmBlocks[k] - 1) / kDedispDmBlocks[k]; };
+  // sizes [k0, k1) in one allocation, the spans behind them
+  auto build = [&](int k0, int k1) {
+    size_t n = 0;
+    for (int k = k0; k < k1; k++) n += blocks(k) * C;
+    const size_t spans_at = n * sizeof(int2), spans_bytes = (size_t)(k1 - k0) * sizeof(Spans);
+    uint8_t* mem = nullptr;
+    if (dev_malloc(&mem, spans_at + spans_bytes) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
+    if (cudaMemset(mem + spans_at, 0, spans_bytes) != cudaSuccess) {
+      free_dev(mem);
+      return DEDISP_INTERNAL_GPU_ERROR;
+    }
+    int2* at = reinterpret_cast<int2*>(mem);
+    for (int k = k0; k < k1; k++) {
+      d_range[k] = at;
+      if (launch_block_ranges(d_delays, D, C, kDedispDmBlocks[k], at,
+                              reinterpret_cast<unsigned long long*>(mem + spans_at) + 2 * (k - k0),
+                              0) != cudaSuccess)
+        return DEDISP_INTERNAL_GPU_ERROR;
+      at += blocks(k) * C;
+    }
+    Spans spans[kDedispDmBlockSizes];
+    if (cudaMemcpy(spans, mem + spans_at, spans_bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
       return DEDISP_MEM_COPY_FAILED;
-  }
-  return DEDISP_NO_ERROR;
+    for (int k = k0; k < k1; k++) {
+      max_span[k] = (size_t)spans[k - k0].largest;
+      mean_span[k] = (size_t)spans[k - k0].sum / (blocks(k) * C);
+    }
+    return DEDISP_NO_ERROR;
+  };
+  const dedisp_error e = build(0, kMain);
+  if (e != DEDISP_NO_ERROR) return e;
+  for (const auto& t : kDedispTiles)
+    if (stage_of(max_span, mean_span, t)) return DEDISP_NO_ERROR;
+  return build(kMain, kDedispDmBlockSizes);
 }
 
 // Trials of one scrunch factor: delays at that factor, per DM-block ranges
@@ -160,7 +204,6 @@ static dedisp_error build_groups(dedisp_plan p) {
         g.delays[i * C + c] = v;
         g.max_delay = std::max(g.max_delay, (size_t)v);
       }
-    block_ranges(g.delays, Dg, C, g.blk_range, g.max_span, g.mean_span);
     p->groups.push_back(std::move(g));
     dedisp_plan_struct::Group& G = p->groups.back();
     if (dev_malloc(&G.d_delays, G.delays.size() * sizeof(int)) != cudaSuccess)
@@ -168,7 +211,7 @@ static dedisp_error build_groups(dedisp_plan p) {
     if (cudaMemcpy(G.d_delays, G.delays.data(), G.delays.size() * sizeof(int),
                    cudaMemcpyHostToDevice) != cudaSuccess)
       return DEDISP_MEM_COPY_FAILED;
-    const dedisp_error e = upload_ranges(G.blk_range, G.d_blk_range);
+    const dedisp_error e = build_ranges(G.d_delays, Dg, C, G.d_blk_range, G.max_span, G.mean_span);
     if (e != DEDISP_NO_ERROR) return e;
   }
   return DEDISP_NO_ERROR;
@@ -187,7 +230,6 @@ dedisp_error plan_prepare(dedisp_plan p) {
       p->delays[d * C + c] = (int)v;
       p->max_delay = std::max(p->max_delay, v);
     }
-  block_ranges(p->delays, D, C, p->blk_range, p->max_span, p->mean_span);
   p->active.clear();
   for (size_t c = 0; c < C; c++)
     if (p->killmask[c]) p->active.push_back((int)c);
@@ -196,10 +238,7 @@ dedisp_error plan_prepare(dedisp_plan p) {
   cudaGetDevice(&dev);
   free_dev(p->d_delays); free_dev(p->d_active); free_dev(p->d_dm_list);
   p->d_delays = nullptr; p->d_active = nullptr; p->d_dm_list = nullptr;
-  for (auto& b : p->d_blk_range) {
-    free_dev(b);
-    b = nullptr;
-  }
+  free_ranges(p->d_blk_range);
   if (hdb::dev_malloc(&p->d_delays, p->delays.size() * sizeof(int)) != cudaSuccess ||
       hdb::dev_malloc(&p->d_active, (p->active.size() + 1) * sizeof(int)) != cudaSuccess ||
       hdb::dev_malloc(&p->d_dm_list, D * sizeof(float)) != cudaSuccess)
@@ -215,28 +254,17 @@ dedisp_error plan_prepare(dedisp_plan p) {
       cudaMemcpy(p->d_dm_list, p->dm_list.data(), D * sizeof(float), cudaMemcpyHostToDevice) !=
           cudaSuccess)
     return DEDISP_MEM_COPY_FAILED;
-  const dedisp_error re = upload_ranges(p->blk_range, p->d_blk_range);
-  if (re != DEDISP_NO_ERROR) return re;
+  if (!p->adaptive) {
+    const dedisp_error re =
+        build_ranges(p->d_delays, D, C, p->d_blk_range, p->max_span, p->mean_span);
+    if (re != DEDISP_NO_ERROR) return re;
+  }
   dedisp_error ge = build_groups(p);
   if (ge != DEDISP_NO_ERROR) return ge;
   p->device = dev;
   p->dirty = false;
   p->gen++;
   return DEDISP_NO_ERROR;
-}
-
-static int dm_block_index(int dm_block) {
-  for (int k = 0; k < kDedispDmBlockSizes; k++)
-    if (kDedispDmBlocks[k] == dm_block) return k;
-  return -1;
-}
-
-// Bytes of a tile's staged row whose DM block spans `span` samples of delay:
-// the span and the tile's words, from a 16-byte boundary on (2^18, more than
-// fits, from 2^16 words on).
-static int row_bytes(size_t span, int time_block) {
-  const size_t words = span + 3 + (size_t)time_block / 4;
-  return words >= (size_t)1 << 16 ? 1 << 18 : (int)((4 * words + 15) & ~(size_t)15);
 }
 
 // Delay spans that dedispersion takes: one staged row of a DM block's span as
@@ -390,14 +418,9 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   // candidate tiles {dm_block, time_block, mean rows per stage} whose staged
   // rows fit shared memory
   std::vector<std::array<int, 3>> cand;
-  auto stage_of = [&](int dm_block, int time_block) {
-    const int k = dm_block_index(dm_block);
-    return dedisp_stage_bytes(dm_block, time_block, row_bytes(mean_span[k], time_block),
-                              row_bytes(max_span[k], time_block));
-  };
   auto offer = [&](const int* t) {
-    const int stage = stage_of(t[0], t[1]);
-    const int mean = row_bytes(mean_span[dm_block_index(t[0])], t[1]);
+    const int stage = stage_of(max_span, mean_span, t);
+    const int mean = row_bytes(span_of(mean_span, t[0]), t[1]);
     if (stage) cand.push_back({t[0], t[1], std::max(1, std::min(kDedispRows, stage / mean))});
   };
   for (const auto& t : kDedispTiles) offer(t);
@@ -452,8 +475,9 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
       a.wait_limit = 1u << 12;
     }
   auto with_tile = [&](const std::array<int, 3>& t) {
-    a.blk_range = d_blk_range[dm_block_index(t[0])];
-    return DedispTile{t[0], t[1], stage_of(t[0], t[1])};
+    const int k = dm_block_index(t[0]);
+    a.blk_range = k < 0 ? nullptr : d_blk_range[k];
+    return DedispTile{t[0], t[1], stage_of(max_span, mean_span, t.data())};
   };
   const std::array<size_t, 3> key = {nsamps, units, tune_key};
   auto it = p->tiles.find(key);
@@ -574,7 +598,7 @@ dedisp_error plan_dedisperse_group(dedisp_plan p, size_t gi, const uint8_t* d_ft
 
 dedisp_plan_struct::~dedisp_plan_struct() {
   hdb::free_dev(d_delays);
-  for (int2* b : d_blk_range) hdb::free_dev(b);
+  hdb::free_ranges(d_blk_range);
   hdb::free_dev(d_active);
   hdb::free_dev(d_dm_list);
   hdb::free_dev(d_err);

@@ -14,10 +14,11 @@
 
 #include "dedisp.h"
 
-// Trials per block of the dedispersion tiles (the tables below hold one entry
-// per size)
-constexpr int kDedispDmBlockSizes = 5;
-constexpr int kDedispDmBlocks[kDedispDmBlockSizes] = {8, 16, 32, 2, 1};
+// Trials per block of the dedispersion tiles that have a table of the blocks'
+// delay ranges: the last size only where no tile of the others fits.  (Tiles of
+// one trial read its delays themselves.)
+constexpr int kDedispDmBlockSizes = 4;
+constexpr int kDedispDmBlocks[kDedispDmBlockSizes] = {8, 16, 32, 2};
 
 struct dedisp_plan_struct {
   dedisp_size nchans = 0;
@@ -33,14 +34,14 @@ struct dedisp_plan_struct {
   bool dirty = true;
   unsigned long long gen = 0;      // counts the rebuilds of the device tables
   std::vector<int> delays;         // [dm][chan]
-  // per DM-block size (kDedispDmBlocks): [dm block][chan] least and largest
-  // delay
-  std::vector<int2> blk_range[kDedispDmBlockSizes];
   std::vector<int> active;         // channels with killmask != 0
   size_t max_delay = 0;
   // over blocks and channels: the largest and the mean of (max - min) delay
   size_t max_span[kDedispDmBlockSizes] = {}, mean_span[kDedispDmBlockSizes] = {};
   int* d_delays = nullptr;
+  // per DM-block size (kDedispDmBlocks): [dm block][chan] least and largest
+  // delay; the first entry begins the allocation of all but the last size (none
+  // with adaptive dt, whose groups have their own)
   int2* d_blk_range[kDedispDmBlockSizes] = {};
   // dedispersion tile {dm_block, time_block, mean rows per stage, source} per (nsamps,
   // units, scrunch group): the fastest of the candidates, timed on first use
@@ -66,7 +67,6 @@ struct dedisp_plan_struct {
     size_t max_delay = 0;            // largest scrunched delay of the group
     size_t max_span[kDedispDmBlockSizes] = {}, mean_span[kDedispDmBlockSizes] = {};
     std::vector<int> delays;         // [d1 - d0][chan]
-    std::vector<int2> blk_range[kDedispDmBlockSizes];
     int* d_delays = nullptr;
     int2* d_blk_range[kDedispDmBlockSizes] = {};
   };
@@ -103,7 +103,7 @@ size_t delay_of(float dm, float table_c);
 std::vector<float> generate_dm_list(float dm_start, float dm_end, double dt, double ti,
                                     double f0, double df, size_t nchans, double tol);
 
-// Recomputes delays, block minima, active channels and uploads them.
+// Recomputes delays, blocks' delay ranges, active channels and uploads them.
 dedisp_error plan_prepare(dedisp_plan p);
 
 // Pitch (bytes) of the channel-major working copy for nsamps samples.
