@@ -818,31 +818,35 @@ __global__ void __launch_bounds__(256) k_block_ranges(const int* __restrict__ de
 // samples t, t + S, t + 2S, t + 3S of the row, for t < nwords (bytes past the
 // row's pitch read as 0; they reach no output).  Thread: 16 words, four
 // 16-byte loads and four 16-byte stores (S, the pitches and the bases are
-// multiples of 16).
+// multiples of 16), of channels blockIdx.y, + gridDim.y, ... (a grid has 65535
+// rows at most).
 __global__ void __launch_bounds__(256) k_split_words(const uint8_t* __restrict__ in,
-                                                     size_t in_pitch, size_t in_unit, int split,
-                                                     int nwords, uint32_t* __restrict__ out,
-                                                     size_t out_pitch, size_t out_unit) {
+                                                     size_t in_pitch, size_t in_unit, int nchans,
+                                                     int split, int nwords,
+                                                     uint32_t* __restrict__ out, size_t out_pitch,
+                                                     size_t out_unit) {
   const int t = 16 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= nwords) return;
-  const uint8_t* row = in + (size_t)blockIdx.z * in_unit + (size_t)blockIdx.y * in_pitch;
-  uint4 v[4];
+  for (int c = blockIdx.y; c < nchans; c += gridDim.y) {
+    const uint8_t* row = in + (size_t)blockIdx.z * in_unit + (size_t)c * in_pitch;
+    uint4 v[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const size_t at = (size_t)t + (size_t)q * split;
-    v[q] = at + 16 <= in_pitch ? __ldg(reinterpret_cast<const uint4*>(row + at))
-                               : make_uint4(0u, 0u, 0u, 0u);
-  }
-  uint4* o = reinterpret_cast<uint4*>(out + (size_t)blockIdx.z * out_unit +
-                                      (size_t)blockIdx.y * out_pitch + t);
-  const uint32_t* x = reinterpret_cast<const uint32_t*>(v);
+    for (int q = 0; q < 4; q++) {
+      const size_t at = (size_t)t + (size_t)q * split;
+      v[q] = at + 16 <= in_pitch ? __ldg(reinterpret_cast<const uint4*>(row + at))
+                                 : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint4* o = reinterpret_cast<uint4*>(out + (size_t)blockIdx.z * out_unit +
+                                        (size_t)c * out_pitch + t);
+    const uint32_t* x = reinterpret_cast<const uint32_t*>(v);
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const uint32_t a0 = x[j], a1 = x[4 + j], a2 = x[8 + j], a3 = x[12 + j];
-    const uint32_t lo01 = __byte_perm(a0, a1, 0x5140), lo23 = __byte_perm(a2, a3, 0x5140);
-    const uint32_t hi01 = __byte_perm(a0, a1, 0x7362), hi23 = __byte_perm(a2, a3, 0x7362);
-    o[j] = make_uint4(__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
-                      __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632));
+    for (int j = 0; j < 4; j++) {
+      const uint32_t a0 = x[j], a1 = x[4 + j], a2 = x[8 + j], a3 = x[12 + j];
+      const uint32_t lo01 = __byte_perm(a0, a1, 0x5140), lo23 = __byte_perm(a2, a3, 0x5140);
+      const uint32_t hi01 = __byte_perm(a0, a1, 0x7362), hi23 = __byte_perm(a2, a3, 0x7362);
+      o[j] = make_uint4(__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                        __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632));
+    }
   }
 }
 
@@ -1151,14 +1155,14 @@ cudaError_t launch_block_ranges(const int* delays, size_t ntrials, size_t nchans
 cudaError_t launch_split_words(const uint8_t* in, size_t in_pitch, size_t in_unit, int nchans,
                                size_t units, int split, size_t nwords, uint32_t* out,
                                size_t out_pitch, size_t out_unit, cudaStream_t s) {
-  if (units < 1 || units > 65535 || nchans < 1 || nchans > 65535 || in_pitch % 16 ||
+  if (units < 1 || units > 65535 || nchans < 1 || in_pitch % 16 ||
       in_unit % 16 || split % 16 || out_pitch % 16 || out_unit % 4 || nwords > out_pitch ||
       nwords > 0x7FFFFFF0ull)
     return cudaErrorInvalidValue;
   const unsigned nthr = (unsigned)((nwords + 15) / 16);
-  dim3 grid((nthr + 255) / 256, (unsigned)nchans, (unsigned)units);
-  k_split_words<<<grid, 256, 0, s>>>(in, in_pitch, in_unit, split, (int)nwords, out, out_pitch,
-                                     out_unit);
+  dim3 grid((nthr + 255) / 256, (unsigned)std::min(nchans, 65535), (unsigned)units);
+  k_split_words<<<grid, 256, 0, s>>>(in, in_pitch, in_unit, nchans, split, (int)nwords, out,
+                                     out_pitch, out_unit);
   note_launch();
   return cudaGetLastError();
 }
