@@ -392,6 +392,18 @@ void tile_cache_put(uint64_t key, const std::array<int, 3>& t) {
 }
 }  // namespace
 
+// One of the plan's buffers at `count` elements at least; on failure it is empty.
+template <class T>
+static dedisp_error grow(T** buf, size_t* cap, size_t count) {
+  if (*cap >= count) return DEDISP_NO_ERROR;
+  free_dev(*buf);
+  *buf = nullptr;
+  *cap = 0;
+  if (dev_malloc(buf, count * sizeof(T)) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
+  *cap = count;
+  return DEDISP_NO_ERROR;
+}
+
 // One launch set over trials whose delays are d_delays (dm_count rows; host
 // copy h_delays) on a channel-major input of nsamps samples, nout output
 // samples per trial; the tile is tuned per (nsamps, units, tune_key) and kept
@@ -579,13 +591,8 @@ dedisp_error plan_dedisperse_group(dedisp_plan p, size_t gi, const uint8_t* d_ft
   const size_t ns = nsamps / g.s;
   const size_t pitch_s = ft_pitch(p, ns);
   const size_t need = units * pitch_s * C;
-  if (p->d_scr_cap < need) {
-    free_dev(p->d_scr);
-    p->d_scr = nullptr;
-    p->d_scr_cap = 0;
-    if (dev_malloc(&p->d_scr, need) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
-    p->d_scr_cap = need;
-  }
+  const dedisp_error ge = grow(&p->d_scr, &p->d_scr_cap, need);
+  if (ge != DEDISP_NO_ERROR) return ge;
   if (launch_scrunch_ft(d_ft, pitch, nsamps, (int)C, (int)g.s, p->d_scr, pitch_s, units,
                         in_unit, pitch_s * C, s) != cudaSuccess)
     return DEDISP_INTERNAL_GPU_ERROR;
@@ -775,12 +782,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   const uint8_t* d_tf = in;
   if (!dev_ptrs) {
     size_t need = nsamps * in_stride;
-    if (p->d_in_tf_cap < need) {
-      hdb::free_dev(p->d_in_tf);
-      p->d_in_tf = nullptr;
-      if (hdb::dev_malloc(&p->d_in_tf, need) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
-      p->d_in_tf_cap = need;
-    }
+    if ((de = hdb::grow(&p->d_in_tf, &p->d_in_tf_cap, need)) != DEDISP_NO_ERROR) return de;
     if (cudaMemcpyAsync(p->d_in_tf, in, need, cudaMemcpyHostToDevice, s) != cudaSuccess)
       return DEDISP_MEM_COPY_FAILED;
     d_tf = p->d_in_tf;
@@ -788,11 +790,8 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   const size_t plane = pitch * p->nchans;
   size_t need_ft = plane * (in_nbits == 16 ? 2 : 1);
   if (p->d_in_ft_cap < need_ft) {
-    hdb::free_dev(p->d_in_ft);
-    p->d_in_ft = nullptr;
-    if (hdb::dev_malloc(&p->d_in_ft, need_ft) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
+    if ((de = hdb::grow(&p->d_in_ft, &p->d_in_ft_cap, need_ft)) != DEDISP_NO_ERROR) return de;
     cudaMemsetAsync(p->d_in_ft, 0, need_ft, s);
-    p->d_in_ft_cap = need_ft;
   }
   if (cudaMemsetAsync(p->d_err, 0, sizeof(unsigned), s) != cudaSuccess ||
       hdb::input_to_ft(d_tf, nsamps, (int)p->nchans, (int)in_nbits, p->d_in_ft, pitch, s, 1,
@@ -803,13 +802,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   if (!dev_ptrs) {
     opitch = (nout + 3) & ~(size_t)3;
     size_t need = opitch * D;
-    if (p->d_out_cap < need) {
-      hdb::free_dev(p->d_out);
-      p->d_out = nullptr;
-      if (hdb::dev_malloc(&p->d_out, need * sizeof(float)) != cudaSuccess)
-        return DEDISP_MEM_ALLOC_FAILED;
-      p->d_out_cap = need;
-    }
+    if ((de = hdb::grow(&p->d_out, &p->d_out_cap, need)) != DEDISP_NO_ERROR) return de;
     d_o = p->d_out;
   } else if (opitch % 4) {
     return DEDISP_INVALID_STRIDE;
@@ -817,13 +810,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   if (in_nbits == 16) {
     // high-byte plane, low-byte plane, then lo + 256 hi
     const size_t need = opitch * D;
-    if (p->d_out_hi_cap < need) {
-      hdb::free_dev(p->d_out_hi);
-      p->d_out_hi = nullptr;
-      if (hdb::dev_malloc(&p->d_out_hi, need * sizeof(float)) != cudaSuccess)
-        return DEDISP_MEM_ALLOC_FAILED;
-      p->d_out_hi_cap = need;
-    }
+    if ((de = hdb::grow(&p->d_out_hi, &p->d_out_hi_cap, need)) != DEDISP_NO_ERROR) return de;
     de = hdb::plan_dedisperse_ft(p, p->d_in_ft + plane, pitch, nsamps, p->d_out_hi, opitch, s);
     if (de != DEDISP_NO_ERROR) return de;
   }
