@@ -62,7 +62,11 @@ struct DedispArgs {
   const int2* blk_range;
   const int* chans;       // active (not killed) channel indices
   int nact;
-  int nchans;
+  int nchans;             // channels of the delay tables
+  int chan0;              // the channel whose words begin `in`
+  // `out` holds 32-bit integer sums of other channels, to be added to, and the
+  // sums are left as integers for a later launch's channels
+  bool sums_before, sums_after;
   int dm_count;
   int nout;               // output samples per DM
   float* out;

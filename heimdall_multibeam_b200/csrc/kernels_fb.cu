@@ -526,7 +526,9 @@ __global__ void k_nb_zap(uint32_t* __restrict__ data, size_t nsamps, int units, 
 // 256 channels the sums of a word go to the output row: a single run is
 // converted and stored; with more channels the row holds 32-bit integer
 // partial sums (stored, then added to in L2) until the last run adds its own
-// and stores the float.  The sums are exact integers in any order.
+// and stores the float.  The sums are exact integers in any order.  The runs may
+// be those of several launches over a part of the channels each (sums_before,
+// sums_after).
 //
 // What bounds it: one shared load per word, DM and channel (128 sample terms a
 // wavefront), so the shared-memory pipe (84 % busy in ncu) and instruction
@@ -662,7 +664,8 @@ __global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT,
       if (lane == 0) mbar_expect_tx(&full[buf], (uint32_t)total);
       __syncwarp();
       if (lane < nk)
-        bulk_g2s(smem + at, in + (size_t)c_now * a.in_pitch + lo, (uint32_t)bytes, &full[buf]);
+        bulk_g2s(smem + at, in + (size_t)(c_now - a.chan0) * a.in_pitch + lo, (uint32_t)bytes,
+                 &full[buf]);
       k0 += nk;
     }
     const int issued = st;
@@ -731,7 +734,7 @@ __global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT,
   };
 
   int nsum = 0;
-  bool first = true;
+  bool first = !a.sums_before;
   for (int st = 0, k0 = 0; k0 < a.nact; st++) {
     const int buf = st % DD_NST;
     if (!mbar_wait(&full[buf], (uint32_t)((st / DD_NST) & 1), a.wait_limit)) {
@@ -782,7 +785,7 @@ __global__ void __launch_bounds__((NWD * NWT + 1) * 32, dd_min_blocks(NWD * NWT,
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[buf]);
   }
-  flush(first, true);
+  flush(first, !a.sums_after);
 }
 
 // Least and largest delay of each block of `db` trials, per channel, and over all

@@ -38,11 +38,14 @@ struct DevBuf {
   ~DevBuf() { if (p) cudaFree(p); }
   template <class T>
   T* as() { return reinterpret_cast<T*>(p); }
-  cudaError_t ensure(size_t bytes) {
-    if (bytes <= cap) return cudaSuccess;
+  void release() {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
+  }
+  cudaError_t ensure(size_t bytes) {
+    if (bytes <= cap) return cudaSuccess;
+    release();
     size_t b = std::max<size_t>(bytes, 256);
     cudaError_t e = hdb::dev_malloc(&p, b);
     if (e == cudaSuccess) cap = b;
@@ -886,7 +889,20 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   need(pl->rows, G * sizeof(hdb::GroupRow));
   need(pl->unit_off, (U + 1) * sizeof(unsigned));
   need(pl->geo, 4 * sizeof(int));
-  if (ae != cudaSuccess) return false;  // the host-sized path reports it
+  // the plan's share, so that the capture allocates nothing
+  if (ae == cudaSuccess && hdb::plan_reserve(plan, nsamps, U) != DEDISP_NO_ERROR)
+    ae = cudaErrorMemoryAllocation;
+  if (ae != cudaSuccess) {
+    // no room for the lists at their capacities: this shape stays on the
+    // host-sized path, which takes them at the totals' size
+    gs->broken = true;
+    for (DevBuf* b : {&pl->hit_ind, &pl->hit_val, &pl->hit_sw, &pl->head, &pl->gid, &m.key,
+                      &m.peak, &m.ind, &m.begin, &m.end, &m.filter, &m.dm, &m.label,
+                      &pl->cl_pack, &pl->cl_first, &pl->root_flag, &pl->root_off, &pl->mkey,
+                      &pl->rows, &pl->scan_tmp})
+      b->release();
+    return false;
+  }
   const size_t spec = std::min<size_t>(gcap, kSpecRows);
   if (pl->ensure_rows_host(std::max<size_t>(spec, 1)) != cudaSuccess) return false;
 
@@ -909,6 +925,7 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   for (const void* q : {(const void*)plan->d_delays, (const void*)plan->d_blk_range[0],
                         (const void*)plan->d_blk_range[1], (const void*)plan->d_blk_range[2],
                         (const void*)plan->d_blk_range[3], (const void*)plan->d_words,
+                        (const void*)plan->d_words_cap,
                         (const void*)plan->d_active, (const void*)plan->d_dm_list,
                         (const void*)plan->d_err})
     key.push_back((size_t)q);
@@ -1050,11 +1067,10 @@ static bool graph_gulp(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool
   return true;
 }
 
-static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool on_device,
-                              hd_size nsamps, hd_size nbits, hd_size first_idx, hd_size nbeams,
-                              const hd_size* beams, hd_error* statuses,
-                              hd_size* nsamps_processed, bool graph = false) {
-  if (!pl) return HD_INVALID_PIPELINE;
+static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool on_device,
+                             hd_size nsamps, hd_size nbits, hd_size first_idx, hd_size nbeams,
+                             const hd_size* beams, hd_error* statuses,
+                             hd_size* nsamps_processed, bool graph) {
   const bool resident = pl->fb_resident;
   pl->fb_resident = false;
   if (!fbs || !nsamps_processed || U == 0) return HD_INVALID_POINTER;
@@ -1632,6 +1648,22 @@ static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t 
     pl->pending_shape.clear();
   }
   return any_too_many ? HD_TOO_MANY_EVENTS : HD_NO_ERROR;
+}
+
+// A gulp for which the device has no room is searched again with the
+// dedispersion's scratch in smaller parts, as long as that gives memory back.
+static hd_error execute_units(hd_pipeline pl, const hd_byte* const* fbs, size_t U, bool on_device,
+                              hd_size nsamps, hd_size nbits, hd_size first_idx, hd_size nbeams,
+                              const hd_size* beams, hd_error* statuses,
+                              hd_size* nsamps_processed, bool graph = false) {
+  if (!pl) return HD_INVALID_PIPELINE;
+  const bool resident = pl->fb_resident;
+  for (;;) {
+    pl->fb_resident = resident;
+    const hd_error e = execute_once(pl, fbs, U, on_device, nsamps, nbits, first_idx, nbeams, beams,
+                                    statuses, nsamps_processed, graph);
+    if (e != HD_MEM_ALLOC_FAILED || !hdb::plan_give_back(pl->plan)) return e;
+  }
 }
 
 hd_error hd_execute(hd_pipeline pl, const hd_byte* h_filterbank, hd_size nsamps, hd_size nbits,

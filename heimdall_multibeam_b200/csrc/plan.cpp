@@ -261,6 +261,7 @@ dedisp_error plan_prepare(dedisp_plan p) {
   }
   dedisp_error ge = build_groups(p);
   if (ge != DEDISP_NO_ERROR) return ge;
+  p->words_limit = p->words_most;
   p->device = dev;
   p->dirty = false;
   p->gen++;
@@ -392,22 +393,103 @@ void tile_cache_put(uint64_t key, const std::array<int, 3>& t) {
 }
 }  // namespace
 
+// Candidate tiles {dm_block, time_block, mean rows per stage}: those whose
+// staged rows fit shared memory.
+static std::vector<std::array<int, 3>> tiles_for(const size_t* max_span,
+                                                 const size_t* mean_span) {
+  std::vector<std::array<int, 3>> cand;
+  auto offer = [&](const int* t) {
+    const int stage = stage_of(max_span, mean_span, t);
+    const int mean = row_bytes(span_of(mean_span, t[0]), t[1]);
+    if (stage) cand.push_back({t[0], t[1], std::max(1, std::min(kDedispRows, stage / mean))});
+  };
+  for (const auto& t : kDedispTiles) offer(t);
+  if (cand.empty())
+    for (const auto& t : kDedispLongTiles) offer(t);
+  return cand;
+}
+
+// The four-sample words of one channel for nout outputs: words q * split apart in
+// the samples, those that some delay reaches, and the row pitch, which holds the
+// last tile's rows of every candidate.
+struct WordRows {
+  size_t split, nwords, pitch;
+};
+static WordRows word_rows(const std::vector<std::array<int, 3>>& cand, size_t nout,
+                          size_t max_delay) {
+  WordRows w;
+  w.split = ((nout + 3) / 4 + 15) & ~(size_t)15;
+  w.nwords = (w.split + max_delay + 15) & ~(size_t)15;
+  w.pitch = w.nwords;
+  for (const auto& t : cand) {
+    const size_t tbw = (size_t)t[1] / 4, ntb = (w.split + tbw - 1) / tbw;
+    w.pitch = std::max(w.pitch, ntb * tbw + max_delay + 8);
+  }
+  w.pitch = (w.pitch + 15) & ~(size_t)15;
+  return w;
+}
+
+// The word buffer for `rows` channel rows of `pitch` words: of all of them, or of
+// fewer (half, a quarter, ..., one row at least) where the device has no room for
+// more.  The size that was had is kept as the limit until the plan is rebuilt, so
+// that later calls do not try the larger ones again.
+static dedisp_error ensure_words(dedisp_plan p, size_t rows, size_t pitch) {
+  const size_t all = rows * pitch;
+  const size_t least = std::max(pitch, std::min(all, p->words_limit));
+  if (p->d_words_cap >= least) return DEDISP_NO_ERROR;
+  free_dev(p->d_words);
+  p->d_words = nullptr;
+  p->d_words_cap = 0;
+  for (size_t want = least;; want = std::max(pitch, want / 2)) {
+    if (dev_malloc(&p->d_words, want * sizeof(uint32_t)) == cudaSuccess) {
+      p->d_words_cap = want;
+      if (want < least) p->words_limit = want;
+      return DEDISP_NO_ERROR;
+    }
+    if (want == pitch) return DEDISP_MEM_ALLOC_FAILED;
+  }
+}
+
+dedisp_error plan_reserve(dedisp_plan p, size_t nsamps, size_t units) {
+  if (nsamps <= p->max_delay || units == 0 || p->active.empty()) return DEDISP_NO_ERROR;
+  const WordRows w = word_rows(tiles_for(p->max_span, p->mean_span), nsamps - p->max_delay,
+                               p->max_delay);
+  return ensure_words(p, units * p->nchans, w.pitch);
+}
+
+bool plan_give_back(dedisp_plan p) {
+  constexpr size_t kKeep = (size_t)4 << 20;  // words: 16 MiB
+  if (p->d_words_cap <= kKeep) return false;
+  p->words_limit = std::max(kKeep, p->d_words_cap / 4);
+  free_dev(p->d_words);
+  p->d_words = nullptr;
+  p->d_words_cap = 0;
+  return true;
+}
+
 // One of the plan's buffers at `count` elements at least; on failure it is empty.
+// The word buffer, which can be had in parts, makes room.
 template <class T>
-static dedisp_error grow(T** buf, size_t* cap, size_t count) {
+static dedisp_error grow(dedisp_plan p, T** buf, size_t* cap, size_t count) {
   if (*cap >= count) return DEDISP_NO_ERROR;
   free_dev(*buf);
   *buf = nullptr;
   *cap = 0;
-  if (dev_malloc(buf, count * sizeof(T)) != cudaSuccess) return DEDISP_MEM_ALLOC_FAILED;
-  *cap = count;
-  return DEDISP_NO_ERROR;
+  do {
+    if (dev_malloc(buf, count * sizeof(T)) == cudaSuccess) {
+      *cap = count;
+      return DEDISP_NO_ERROR;
+    }
+  } while (plan_give_back(p));
+  return DEDISP_MEM_ALLOC_FAILED;
 }
 
 // One launch set over trials whose delays are d_delays (dm_count rows; host
 // copy h_delays) on a channel-major input of nsamps samples, nout output
 // samples per trial; the tile is tuned per (nsamps, units, tune_key) and kept
-// in the persistent tile cache.
+// in the persistent tile cache.  Where the word buffer holds no more, a few
+// filterbanks or (of one filterbank) a few channels go through it at a time; the
+// channels' sums meet in the output rows.
 static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_delays,
                                       const int* d_delays, int2* const* d_blk_range,
                                       const size_t* max_span, const size_t* mean_span,
@@ -427,55 +509,27 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   if (units > 65535) return DEDISP_INVALID_STRIDE;
   // one channel row of the widest block's delay span must fit shared memory
   if (!spans_supported(max_span)) return DEDISP_NCHANS_EXCEEDS_LIMIT;
-  // candidate tiles {dm_block, time_block, mean rows per stage} whose staged
-  // rows fit shared memory
-  std::vector<std::array<int, 3>> cand;
-  auto offer = [&](const int* t) {
-    const int stage = stage_of(max_span, mean_span, t);
-    const int mean = row_bytes(span_of(mean_span, t[0]), t[1]);
-    if (stage) cand.push_back({t[0], t[1], std::max(1, std::min(kDedispRows, stage / mean))});
-  };
-  for (const auto& t : kDedispTiles) offer(t);
-  if (cand.empty())
-    for (const auto& t : kDedispLongTiles) offer(t);
-  // ---- the four-sample words of the input ----
-  const size_t split = ((nout + 3) / 4 + 15) & ~(size_t)15;
-  const size_t nwords = (split + max_delay + 15) & ~(size_t)15;
-  size_t wpitch = nwords;
-  for (const auto& t : cand) {
-    const size_t tbw = (size_t)t[1] / 4, ntb = (split + tbw - 1) / tbw;
-    wpitch = std::max(wpitch, ntb * tbw + max_delay + 8);  // past the last tile's rows
-  }
-  wpitch = (wpitch + 15) & ~(size_t)15;
-  const size_t wunit = wpitch * p->nchans;
-  if (p->d_words_cap < units * wunit) {
-    free_dev(p->d_words);
-    p->d_words = nullptr;
-    p->d_words_cap = 0;
-    if (dev_malloc(&p->d_words, units * wunit * sizeof(uint32_t)) != cudaSuccess)
-      return DEDISP_MEM_ALLOC_FAILED;
-    p->d_words_cap = units * wunit;
-  }
-  if (nout > 0x7FFFFFFFull - 4096 ||
-      launch_split_words(d_ft, pitch, in_unit, (int)p->nchans, units, (int)split, nwords,
-                         p->d_words, wpitch, wunit, s) != cudaSuccess)
-    return DEDISP_INTERNAL_GPU_ERROR;
+  if (nout > 0x7FFFFFFFull - 4096) return DEDISP_INTERNAL_GPU_ERROR;
+  const std::vector<std::array<int, 3>> cand = tiles_for(max_span, mean_span);
+  const WordRows w = word_rows(cand, nout, max_delay);
+  const size_t C = p->nchans;
+  const dedisp_error we = ensure_words(p, units * C, w.pitch);
+  if (we != DEDISP_NO_ERROR) return we;
+  const size_t rows = p->d_words_cap / w.pitch;  // of the buffer
+  const size_t part_units = std::min(units, std::max<size_t>(1, rows / C));
+  const size_t part_chans = std::min(C, rows);
   DedispArgs a{};
   a.in = p->d_words;
-  a.in_pitch = wpitch;
-  a.split = (int)split;
+  a.in_pitch = w.pitch;
+  a.split = (int)w.split;
   a.delays = d_delays;
-  a.chans = p->d_active;
-  a.nact = (int)p->active.size();
-  a.nchans = (int)p->nchans;
+  a.nchans = (int)C;
   a.dm_count = dm_count;
   a.nout = (int)nout;
-  a.out = d_out;
   a.out_pitch = out_pitch;
   a.cap = 0;
   a.err = p->d_err;
-  a.units = (int)units;
-  a.in_unit = wunit;
+  a.in_unit = w.pitch * part_chans;
   a.out_unit = out_unit;
   a.wait_limit = kDedispWaitLimit;
   a.withhold_last = 0;
@@ -490,6 +544,23 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
     const int k = dm_block_index(t[0]);
     a.blk_range = k < 0 ? nullptr : d_blk_range[k];
     return DedispTile{t[0], t[1], stage_of(max_span, mean_span, t.data())};
+  };
+  // the words of filterbanks [u0, u0 + n) and channels [c0, c1), and the launch's
+  // share of the sums
+  auto part = [&](size_t u0, size_t n, size_t c0, size_t c1) {
+    const auto k0 = std::lower_bound(p->active.begin(), p->active.end(), (int)c0);
+    const auto k1 = std::lower_bound(k0, p->active.end(), (int)c1);
+    a.chans = p->d_active + (k0 - p->active.begin());
+    a.nact = (int)(k1 - k0);
+    a.chan0 = (int)c0;
+    a.sums_before = k0 != p->active.begin();
+    a.sums_after = k1 != p->active.end();
+    a.out = d_out + u0 * out_unit;
+    a.units = (int)n;
+    return a.nact == 0 ||
+           launch_split_words(d_ft + u0 * in_unit + c0 * pitch, pitch, in_unit, (int)(c1 - c0), n,
+                              (int)w.split, w.nwords, p->d_words, w.pitch, a.in_unit,
+                              s) == cudaSuccess;
   };
   const std::array<size_t, 3> key = {nsamps, units, tune_key};
   auto it = p->tiles.find(key);
@@ -518,8 +589,13 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
       }
     }
     if (p->tune && !forced && !cached && cand.size() > 1) {
-      // autotuner: each candidate once to warm up and once timed; all give the
-      // same sums, so the output of the last run stands
+      // autotuner: each candidate once to warm up and once timed, on the first
+      // part that has channels (no sums are added to)
+      for (size_t c0 = 0; c0 < C; c0 += part_chans) {
+        if (!part(0, part_units, c0, std::min(C, c0 + part_chans)))
+          return DEDISP_INTERNAL_GPU_ERROR;
+        if (a.nact) break;
+      }
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       if (cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess) {
         float best_ms = 0.f;
@@ -550,7 +626,13 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   }
   p->last_tile = {it->second[0], it->second[1], it->second[2]};
   p->last_tile_source = it->second[3];
-  if (launch_dedisp(a, with_tile(p->last_tile), s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
+  const DedispTile tile = with_tile(p->last_tile);
+  for (size_t u0 = 0; u0 < units; u0 += part_units)
+    for (size_t c0 = 0; c0 < C; c0 += part_chans) {
+      if (!part(u0, std::min(part_units, units - u0), c0, std::min(C, c0 + part_chans)))
+        return DEDISP_INTERNAL_GPU_ERROR;
+      if (a.nact && launch_dedisp(a, tile, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
+    }
   return DEDISP_NO_ERROR;
 }
 
@@ -591,7 +673,7 @@ dedisp_error plan_dedisperse_group(dedisp_plan p, size_t gi, const uint8_t* d_ft
   const size_t ns = nsamps / g.s;
   const size_t pitch_s = ft_pitch(p, ns);
   const size_t need = units * pitch_s * C;
-  const dedisp_error ge = grow(&p->d_scr, &p->d_scr_cap, need);
+  const dedisp_error ge = grow(p, &p->d_scr, &p->d_scr_cap, need);
   if (ge != DEDISP_NO_ERROR) return ge;
   if (launch_scrunch_ft(d_ft, pitch, nsamps, (int)C, (int)g.s, p->d_scr, pitch_s, units,
                         in_unit, pitch_s * C, s) != cudaSuccess)
@@ -649,6 +731,11 @@ dedisp_error dedisp_create_plan(dedisp_plan* plan, dedisp_size nchans, dedisp_fl
       p->forced_dm_block = db;
       p->forced_time_block = tb;
     }
+  }
+  // HDB_DEDISP_WORDS bounds the word buffer (in words)
+  if (const char* e = std::getenv("HDB_DEDISP_WORDS")) {
+    unsigned long long n = 0;
+    if (std::sscanf(e, "%llu", &n) == 1 && n) p->words_most = (size_t)n;
   }
   *plan = p;
   return DEDISP_NO_ERROR;
@@ -782,7 +869,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   const uint8_t* d_tf = in;
   if (!dev_ptrs) {
     size_t need = nsamps * in_stride;
-    if ((de = hdb::grow(&p->d_in_tf, &p->d_in_tf_cap, need)) != DEDISP_NO_ERROR) return de;
+    if ((de = hdb::grow(p, &p->d_in_tf, &p->d_in_tf_cap, need)) != DEDISP_NO_ERROR) return de;
     if (cudaMemcpyAsync(p->d_in_tf, in, need, cudaMemcpyHostToDevice, s) != cudaSuccess)
       return DEDISP_MEM_COPY_FAILED;
     d_tf = p->d_in_tf;
@@ -790,7 +877,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   const size_t plane = pitch * p->nchans;
   size_t need_ft = plane * (in_nbits == 16 ? 2 : 1);
   if (p->d_in_ft_cap < need_ft) {
-    if ((de = hdb::grow(&p->d_in_ft, &p->d_in_ft_cap, need_ft)) != DEDISP_NO_ERROR) return de;
+    if ((de = hdb::grow(p, &p->d_in_ft, &p->d_in_ft_cap, need_ft)) != DEDISP_NO_ERROR) return de;
     cudaMemsetAsync(p->d_in_ft, 0, need_ft, s);
   }
   if (cudaMemsetAsync(p->d_err, 0, sizeof(unsigned), s) != cudaSuccess ||
@@ -802,7 +889,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   if (!dev_ptrs) {
     opitch = (nout + 3) & ~(size_t)3;
     size_t need = opitch * D;
-    if ((de = hdb::grow(&p->d_out, &p->d_out_cap, need)) != DEDISP_NO_ERROR) return de;
+    if ((de = hdb::grow(p, &p->d_out, &p->d_out_cap, need)) != DEDISP_NO_ERROR) return de;
     d_o = p->d_out;
   } else if (opitch % 4) {
     return DEDISP_INVALID_STRIDE;
@@ -810,7 +897,7 @@ dedisp_error dedisp_execute_adv(const dedisp_plan p, dedisp_size nsamps, const d
   if (in_nbits == 16) {
     // high-byte plane, low-byte plane, then lo + 256 hi
     const size_t need = opitch * D;
-    if ((de = hdb::grow(&p->d_out_hi, &p->d_out_hi_cap, need)) != DEDISP_NO_ERROR) return de;
+    if ((de = hdb::grow(p, &p->d_out_hi, &p->d_out_hi_cap, need)) != DEDISP_NO_ERROR) return de;
     de = hdb::plan_dedisperse_ft(p, p->d_in_ft + plane, pitch, nsamps, p->d_out_hi, opitch, s);
     if (de != DEDISP_NO_ERROR) return de;
   }

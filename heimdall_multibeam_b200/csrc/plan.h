@@ -73,8 +73,13 @@ struct dedisp_plan_struct {
   std::vector<Group> groups;          // built only with adaptive dt
   uint8_t* d_scr = nullptr;           // scrunched channel-major input
   size_t d_scr_cap = 0;
-  uint32_t* d_words = nullptr;        // four-sample words of the input being dedispersed
+  // four-sample words of the input being dedispersed, of all its filterbanks and
+  // channels where memory allows, else of a part of them at a time
+  uint32_t* d_words = nullptr;
   size_t d_words_cap = 0;             // words
+  // the buffer grows no further than words_limit: what was to be had, at most
+  // words_most (HDB_DEDISP_WORDS)
+  size_t words_most = (size_t)-1, words_limit = (size_t)-1;
 
   // scratch for dedisp_execute* with host pointers
   uint8_t* d_in_tf = nullptr;
@@ -108,6 +113,14 @@ dedisp_error plan_prepare(dedisp_plan p);
 
 // Pitch (bytes) of the channel-major working copy for nsamps samples.
 size_t ft_pitch(const dedisp_plan p, size_t nsamps);
+
+// Allocates what dedispersing `units` filterbanks of nsamps samples needs beside
+// the caller's buffers (a plan without adaptive dt; the calls below do it too).
+dedisp_error plan_reserve(dedisp_plan p, size_t nsamps, size_t units);
+
+// After a caller's allocation failed: whether the plan gave memory back (its next
+// inputs are taken in smaller parts), so that trying again may help.
+bool plan_give_back(dedisp_plan p);
 
 // Dedisperses the FT copy already on the device into out (device floats).
 // With units > 1, one launch dedisperses `units` filterbanks that lie

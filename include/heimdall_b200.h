@@ -405,7 +405,9 @@ hd_error hd_bf16_gemm_tc(int m, int n, int k, const void* d_a, long long sam, lo
  * cache file, keyed by the device, the gulp shape and the delay table:
  * HDB_TUNE_CACHE=path, else $XDG_CACHE_HOME/heimdall_b200/dedisp_tiles.txt,
  * else $HOME/.cache/heimdall_b200/dedisp_tiles.txt; HDB_TUNE_CACHE=0 turns it
- * off. */
+ * off.  HDB_DEDISP_WORDS=n bounds the dedispersion's scratch to n 32-bit words
+ * (a channel's at least); without it the scratch takes what the gulp would have
+ * and gives way, in parts, where the device has no room for it. */
 hd_error hd_get_dedisp_tile(hd_pipeline pipeline, int* dm_block, int* time_block, int* rows);
 
 /* Where the last gulp's dedispersion tile came from: 0 the default tile,
