@@ -616,7 +616,9 @@ hd_error hd_get_giants(hd_pipeline pipeline, hd_float* peaks, hd_size* inds, hd_
  * When hd_execute_beams copies host filterbanks in pieces overlapped with
  * their transpose and dedispersion (cleaning off), [7] ends when the last
  * piece has landed, [1] then covers the last piece's transpose and [2] its
- * dedispersion. */
+ * dedispersion.  With adaptive dt [3] to [5] are the sums over the scrunch
+ * groups, of which [3] is the time that the search waits for a group's series:
+ * they are made while other groups are dedispersed ([2]) and searched. */
 hd_error hd_get_timing(hd_pipeline pipeline, float* ms, int n);
 
 #ifdef __cplusplus
