@@ -188,6 +188,7 @@ SYMBOLS = {
     "hd_get_beam_set_candidates": (C.c_int, [_P, _SZ, _P, _SZP]),
     "hd_destroy_beam_set": (None, [_P]),
     "hd_get_launch_count": (C.c_ulonglong, []),
+    "hd_release_workspaces": (None, []),
     "hd_set_graphs": (C.c_int, [_P, C.c_int]),
     "hd_get_graph_replays": (C.c_ulonglong, [_P]),
     "hd_measure_int_add_rate": (C.c_int, [C.c_int, C.POINTER(C.c_double)]),
@@ -923,6 +924,12 @@ class Classifier:
             if err != HD_NO_ERROR:
                 raise HdError(err, "hd_classifier_score_device")
         return out
+
+
+def release_workspaces() -> None:
+    """hd_release_workspaces: the device memory that profile_candidates keeps
+    between calls goes back to the devices."""
+    lib().hd_release_workspaces()
 
 
 def profile_candidates(filterbank, tsamp: float, fch1: float, foff: float, dm_list,

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(32 * FT_BINS) k_prof_ft(const uint8_t* __restr
 // of a 1.2 ms call, so a finished call leaves them for the next one: each call
 // takes one for itself (threads never share one), at most two per device stay,
 // of 256 MiB at most, and trim_pools() gives them back (dev_malloc calls it
-// when the device is out of memory).
+// when the device is out of memory, a program hd_release_workspaces()).
 struct Workspace {
   int dev = 0;
   cudaStream_t stream = nullptr;
@@ -412,6 +412,8 @@ void trim_pools() {
 }
 
 }  // namespace hdb
+
+extern "C" void hd_release_workspaces(void) { hdb::trim_pools(); }
 
 extern "C" hd_error hd_profile_candidates(
     const hd_byte* filterbank, hd_size nsamps, hd_size nchans, int on_device, double tsamp,

@@ -29,7 +29,8 @@
  * hd_search_sigproc_file, hd_search_sigproc_files); the coincidencer (hd_coincide,
  * hd_write_coincident_candidates); the candidate classifier
  * (hd_extract_patches, hd_score_candidates, hd_classifier_*); the candidate
- * profiler (hd_profile_candidates, Applications/candidate_profiler.C).
+ * profiler (hd_profile_candidates, Applications/candidate_profiler.C;
+ * hd_release_workspaces).
  *
  * Ownership and threading: the caller owns every host buffer it passes; the
  * pipeline owns all device memory, its CUDA stream and events.  A pipeline
@@ -315,6 +316,10 @@ hd_error hd_profile_candidates(const hd_byte* filterbank, hd_size nsamps, hd_siz
                                const hd_profile_request* cands, hd_size ncands,
                                hd_size out_nsamps, hd_size out_dm_count, hd_size fscrunch,
                                int do_filter, hd_profile* out);
+/* Gives the device memory that finished hd_profile_candidates calls keep for
+ * later ones (at most two buffers of 256 MiB on each device) back to the
+ * devices.  Calls that are running keep theirs; the next one allocates anew. */
+void     hd_release_workspaces(void);
 
 /* ---- Learned candidate classifier (no counterpart in the reference) ----
  *
