@@ -62,24 +62,23 @@ struct DedispArgs {
   const int2* blk_range;
   const int* chans;       // active (not killed) channel indices
   int nact;
-  int nchans;             // channels of the delay tables
-  int chan0;              // the channel whose words begin `in`
-  // `out` holds 32-bit integer sums of other channels, to be added to, and the
-  // sums are left as integers for a later launch's channels
-  bool sums_before, sums_after;
+  int nchans;
   int dm_count;
   int nout;               // output samples per DM
   float* out;
   size_t out_pitch;       // floats between DM rows
   int cap;                // bytes of a stage buffer (multiple of 16)
   unsigned* err;          // device error word (bit 0: staging wait timed out)
-  int units;              // independent filterbanks dedispersed by one launch
+  int chan0;              // the channel whose words begin `in`
   size_t in_unit;         // words between units' inputs
   size_t out_unit;        // floats between units' outputs
   unsigned wait_limit;    // polls of each bounded mbarrier wait
   // test of the error path: the producer issues no copy for the last stage,
   // so the consumers' wait on it runs out (HDB_TEST_WITHHOLD_STAGE=1)
-  int withhold_last;
+  // launches over a part of the channels: `out` holds 32-bit integer sums of
+  // other channels, to be added to; the sums are left as integers for a later
+  // launch's channels
+  bool withhold_last, sums_before, sums_after;
 };
 
 // Dedispersion tile: DMs and output samples per CTA (a quarter of them words
@@ -102,7 +101,8 @@ constexpr int kDedispRows = 32;  // channel rows per stage at most
 // bytes of a stage buffer for rows of these lengths (0: a row does not fit)
 int dedisp_stage_bytes(int dm_block, int time_block, int mean_row, int longest_row);
 size_t dedisp_smem_bytes(int dm_block, int time_block, int cap);
-cudaError_t launch_dedisp(const DedispArgs& a, const DedispTile& t, cudaStream_t s);
+// (one launch for `units` independent filterbanks)
+cudaError_t launch_dedisp(const DedispArgs& a, int units, const DedispTile& t, cudaStream_t s);
 // Least and largest delay of each block of `db` trials and channel of the delays
 // [ntrials][nchans]; the largest span and the spans' sum into span[0], span[1]
 // (zero before).

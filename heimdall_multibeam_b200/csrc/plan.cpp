@@ -532,12 +532,12 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   a.in_unit = w.pitch * part_chans;
   a.out_unit = out_unit;
   a.wait_limit = kDedispWaitLimit;
-  a.withhold_last = 0;
+  a.withhold_last = false;
   // error-path test (read per call so a test can clear it between gulps):
   // the last channel stage is withheld and the waits give up quickly
   if (const char* e = std::getenv("HDB_TEST_WITHHOLD_STAGE"))
     if (e[0] == '1') {
-      a.withhold_last = 1;
+      a.withhold_last = true;
       a.wait_limit = 1u << 12;
     }
   auto with_tile = [&](const std::array<int, 3>& t) {
@@ -547,6 +547,7 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
   };
   // the words of filterbanks [u0, u0 + n) and channels [c0, c1), and the launch's
   // share of the sums
+  int nunits = 0;
   auto part = [&](size_t u0, size_t n, size_t c0, size_t c1) {
     const auto k0 = std::lower_bound(p->active.begin(), p->active.end(), (int)c0);
     const auto k1 = std::lower_bound(k0, p->active.end(), (int)c1);
@@ -556,7 +557,7 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
     a.sums_before = k0 != p->active.begin();
     a.sums_after = k1 != p->active.end();
     a.out = d_out + u0 * out_unit;
-    a.units = (int)n;
+    nunits = (int)n;
     return a.nact == 0 ||
            launch_split_words(d_ft + u0 * in_unit + c0 * pitch, pitch, in_unit, (int)(c1 - c0), n,
                               (int)w.split, w.nwords, p->d_words, w.pitch, a.in_unit,
@@ -602,9 +603,9 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
         bool have = false;
         for (const auto& t : cand) {
           const DedispTile dt = with_tile(t);
-          if (launch_dedisp(a, dt, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
+          if (launch_dedisp(a, nunits, dt, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
           cudaEventRecord(e0, s);
-          if (launch_dedisp(a, dt, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
+          if (launch_dedisp(a, nunits, dt, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
           cudaEventRecord(e1, s);
           float ms = 0.f;
           if (cudaEventSynchronize(e1) != cudaSuccess ||
@@ -631,7 +632,7 @@ static dedisp_error dedisperse_tables(dedisp_plan p, const std::vector<int>& h_d
     for (size_t c0 = 0; c0 < C; c0 += part_chans) {
       if (!part(u0, std::min(part_units, units - u0), c0, std::min(C, c0 + part_chans)))
         return DEDISP_INTERNAL_GPU_ERROR;
-      if (a.nact && launch_dedisp(a, tile, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
+      if (a.nact && launch_dedisp(a, nunits, tile, s) != cudaSuccess) return DEDISP_INTERNAL_GPU_ERROR;
     }
   return DEDISP_NO_ERROR;
 }
