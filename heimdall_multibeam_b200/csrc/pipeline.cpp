@@ -82,8 +82,6 @@ struct hd_pipeline_t {
   static constexpr int kSide = 3;
   cudaStream_t side[kSide] = {};
   std::vector<cudaEvent_t> side_ev;  // two per group: dedispersed, summed
-  // stage times, three per group: its series are there, hits written, giants made
-  std::vector<cudaEvent_t> group_ev;
   cudaError_t ensure_side(size_t ngroups) {
     for (auto& q : side)
       if (!q)
@@ -92,11 +90,6 @@ struct hd_pipeline_t {
       cudaEvent_t v = nullptr;
       if (cudaError_t e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) return e;
       side_ev.push_back(v);
-    }
-    while (group_ev.size() < 3 * ngroups) {
-      cudaEvent_t v = nullptr;
-      if (cudaError_t e = cudaEventCreate(&v)) return e;
-      group_ev.push_back(v);
     }
     return cudaSuccess;
   }
@@ -300,7 +293,6 @@ struct hd_pipeline_t {
     for (auto& e : chunk_ev) if (e) cudaEventDestroy(e);
     for (auto& q : pf) if (q.done) cudaEventDestroy(q.done);
     for (auto& v : side_ev) cudaEventDestroy(v);
-    for (auto& v : group_ev) cudaEventDestroy(v);
     for (auto& q : side) if (q) cudaStreamDestroy(q);
     if (stream) cudaStreamDestroy(stream);
     if (copy_stream) cudaStreamDestroy(copy_stream);
@@ -1344,12 +1336,6 @@ static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U
     }
   }
   cudaEventRecord(pl->ev[3], s);
-  // stage boundary k (0: series, 1: hits, 2: giants) of the go-th group searched
-  const bool adaptive = !pl->plan->groups.empty();
-  auto stage_end = [&](size_t go, int k) {
-    if (adaptive) cudaEventRecord(pl->group_ev[3 * go + k], s);
-    else if (k < 2) cudaEventRecord(pl->ev[4 + k], s);
-  };
   // the coarsest group's series are ready first
   for (size_t go = 0; go < ngs; go++) {
     const size_t gi = ngs - 1 - go;
@@ -1364,15 +1350,14 @@ static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U
                         pl->ws_a.cap / sizeof(float) - tree_total};
     if (pl->plan->groups.empty()) HD_TRY(series_of(gi, s));
     else HD_TRY(cudaStreamWaitEvent(s, pl->side_ev[2 * gi + 1], 0));
-    stage_end(go, 0);
+    if (go == 0) cudaEventRecord(pl->ev[4], s);
 
     // ---- widths (pipeline.cu:657-776 at this group's factor) ------------------
     wi = widths_for(P, scr, nc_s, stride_s, cur_delay);
     const size_t cur_off = rel_bmax / 2;
     const int nw = (int)wi.size();
     if (nw == 0) {  // the trials' factor exceeds the widest boxcar
-      stage_end(go, 1);
-      stage_end(go, 2);
+      if (go + 1 == ngs) cudaEventRecord(pl->ev[5], s);
       continue;
     }
     HD_TRY(pl->winfo.ensure(nw * sizeof(hdb::WidthInfo)));
@@ -1434,13 +1419,10 @@ static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U
     hb.sw = pl->hit_sw.as<unsigned>();
     hb.cap = gh;
     if (gh) HD_TRY(hdb::write_hits(wctx, hb, s));
-    stage_end(go, 1);
+    if (go + 1 == ngs) cudaEventRecord(pl->ev[5], s);
 
     // ---- giants ------------------------------------------------------------
-    if (!gh) {
-      stage_end(go, 2);
-      continue;
-    }
+    if (!gh) continue;
     HD_TRY(pl->head.ensure((size_t)(gh + 1) * sizeof(unsigned)));
     HD_TRY(pl->gid.ensure((size_t)(gh + 1) * sizeof(unsigned)));
     hdb::GiantBuffers gg{};
@@ -1470,7 +1452,6 @@ static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U
     gs.view(gg);
     gg.cap = gn;
     HD_TRY(hdb::giant_fill(wctx, hb, gh, gn, gg, s));
-    stage_end(go, 2);
   }
   if (search && ngiants) {
     hd_pipeline_t::GiantSet& m = pl->main_giants;
@@ -1626,26 +1607,16 @@ static hd_error execute_once(hd_pipeline pl, const hd_byte* const* fbs, size_t U
                   *nsamps_processed);
 
   // stage timings
-  auto between = [](cudaEvent_t a, cudaEvent_t b) {
+  auto el = [&](int a, int b) {
     float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, a, b) != cudaSuccess) ms = 0.f;
+    if (cudaEventElapsedTime(&ms, pl->ev[a], pl->ev[b]) != cudaSuccess) ms = 0.f;
     return ms;
   };
-  auto el = [&](int a, int b) { return between(pl->ev[a], pl->ev[b]); };
   pl->timing[0] = el(0, 7);
   pl->timing[7] = el(0, 1);
   pl->timing[1] = el(1, 2);
   pl->timing[2] = el(2, 3);
-  if (search && adaptive) {
-    // each stage's share of every group
-    cudaEvent_t last = pl->ev[3];
-    for (size_t go = 0; go < ngs; go++)
-      for (int k = 0; k < 3; k++) {
-        pl->timing[3 + k] += between(last, pl->group_ev[3 * go + k]);
-        last = pl->group_ev[3 * go + k];
-      }
-    pl->timing[5] += between(last, pl->ev[6]);
-  } else if (search) {
+  if (search) {
     pl->timing[3] = el(3, 4);
     pl->timing[4] = el(4, 5);
     pl->timing[5] = el(5, 6);

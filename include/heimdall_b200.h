@@ -621,9 +621,10 @@ hd_error hd_get_giants(hd_pipeline pipeline, hd_float* peaks, hd_size* inds, hd_
  * When hd_execute_beams copies host filterbanks in pieces overlapped with
  * their transpose and dedispersion (cleaning off), [7] ends when the last
  * piece has landed, [1] then covers the last piece's transpose and [2] its
- * dedispersion.  With adaptive dt [3] to [5] are the sums over the scrunch
- * groups, of which [3] is the time that the search waits for a group's series:
- * they are made while other groups are dedispersed ([2]) and searched. */
+ * dedispersion.  With adaptive dt the scrunch groups' series are made while other
+ * groups are dedispersed ([2]) and searched: [3] is the wait for those of the
+ * first group searched, [4] ends with the last group's thresholds (it holds the
+ * other groups' giants), [5] is the last group's giants and the joint list. */
 hd_error hd_get_timing(hd_pipeline pipeline, float* ms, int n);
 
 #ifdef __cplusplus
