@@ -612,8 +612,8 @@ class Pipeline:
         return err, total.value, gulps
 
     def dedisp_tile(self) -> Tuple[int, int, int]:
-        """hd_get_dedisp_tile: (DM block, time block, rows per stage) of the
-        last gulp's dedispersion."""
+        """hd_get_dedisp_tile: (DM block, time block, mean rows per stage) of
+        the last gulp's dedispersion."""
         v = [C.c_int(0) for _ in range(3)]
         lib().hd_get_dedisp_tile(self._p, *(C.byref(x) for x in v))
         return tuple(int(x.value) for x in v)

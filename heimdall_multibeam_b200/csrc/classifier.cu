@@ -7,12 +7,14 @@
 //   each: conv3x3(1->8) ReLU maxpool2, conv3x3(8->16) ReLU maxpool2,
 //         conv3x3(16->32) ReLU maxpool2   -> A: 32x8x8, B: 32x8x32
 //   concat (10240) -> FC 16 ReLU -> FC 2 -> softmax (class 1 = pulse)
-// Convolutions run as implicit GEMMs over an im2col matrix: forward
-// (W x col), backward-data (W^T x dOut, then col2im) and backward-weights
-// (dOut x col^T, split over the pixel dimension).  Every GEMM takes BF16
-// operands (weights rounded from FP32 master copies, activations stored in
-// BF16) and accumulates in FP32 with mma.sync m16n8k16.  Adam updates the
-// FP32 master weights.  Activation layout: [channel][batch][row][col].
+// Training runs the convolutions as GEMMs over an im2col matrix on the tensor
+// cores (umma.cu): forward (W x col) and the weight gradients (dOut x col^T,
+// split over the pixels); the data gradient is a kernel of its own that sums
+// the nine taps' products (k_dgrad3, mma.sync m16n8k16).  Inference is one
+// fused kernel (k_clf_infer).  All products take BF16 operands (weights rounded
+// from FP32 master copies, activations stored in BF16) and accumulate in FP32.
+// Adam updates the FP32 master weights.  Activation layout:
+// [channel][batch][row][col].
 #include <cuda_bf16.h>
 
 #include <algorithm>

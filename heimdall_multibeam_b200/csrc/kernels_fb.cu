@@ -5,8 +5,9 @@
 //   TF  (input, as the reference receives it): spectrum t at in + t*nchans,
 //       one byte per channel (8-bit data).
 //   FT  (device working copy): channel c at ft + c*pitch, one byte per sample,
-//       pitch a multiple of 64 bytes with zero padding past nsamps so the
-//       dedispersion tiles can be fetched with 16-byte-aligned bulk copies.
+//       pitch a multiple of 64 bytes, so that rows are read and written in
+//       16-byte pieces (what lies past nsamps reaches no result).
+//   Four-sample words (what dedispersion reads): k_split_words.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -902,8 +903,8 @@ cudaError_t launch_combine_planes(float* lo, const float* hi, size_t pitch, size
 // power of two; rounded half up) of each channel row, zero past nsamps / s.
 // Bound by its reads.  A thread makes four outputs (one word) from 4 s bytes,
 // read as whole words whose bytes are added four at a time (256 channels x
-// 2^18 samples, s = 2..64: SCR_US us on average; a byte and a thread at a time
-// 78 us).
+// 2^18 samples, s = 2..64: 24 us on average, 39 at s = 2 and 16 to 25 above; a
+// byte and a thread at a time 78 us).
 __global__ void __launch_bounds__(256) k_scrunch_ft(const uint8_t* __restrict__ in,
                                                     size_t in_pitch, unsigned ns, int log2s,
                                                     uint8_t* __restrict__ out, unsigned out_pitch,

@@ -904,15 +904,10 @@ __global__ void k_block_rms_pass1_multi(WidthCtx ctx, int w0, int nwb, int m, in
   }
 }
 
-// Pass 1 for several unscrunched widths.  A lane takes 25 consecutive samples of
-// one width and folds them to a second-level median in registers: 50 loads of
-// the staged window at a lane stride of 25 words, which no two lanes' banks
-// share, and no level-1 medians in shared memory.  Widths 1, 2, 4 and 8 share
-// one 33-value window.
 constexpr int HIT_TILE = 2048;  // samples of a threshold tile
 constexpr int HIT_THREADS = 256;
 constexpr int HIT_PER_THREAD = HIT_TILE / HIT_THREADS;
-// whether the thresholds first look which tiles can have hits
+// whether the thresholds first look which tiles can have hits (count_hits)
 static bool select_pays(int nser, size_t ntiles) { return (size_t)nser * ntiles > 148 * 8; }
 
 constexpr int BRV_THREADS = 512;  // at most 16 warps: one per boxcar width
@@ -1103,6 +1098,11 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory");
 }
 
+// Pass 1 for several unscrunched widths.  A lane takes 25 consecutive samples of
+// one width and folds them to a second-level median in registers: 50 loads of
+// the staged window at a lane stride of 25 words, which no two lanes' banks
+// share, and no level-1 medians in shared memory.  Widths 1, 2, 4 and 8 share
+// one 33-value window.
 // Block (x, y): groups [x * gpb, (x + 1) * gpb) of series y.  The next
 // group's window is copied into the other half of a double buffer (cp.async)
 // while the current group's medians are computed.  Of 8424 series x 28000

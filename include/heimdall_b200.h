@@ -403,7 +403,8 @@ hd_error hd_bf16_gemm_tc(int m, int n, int k, const void* d_a, long long sam, lo
                          long long scm, long long scn, int accumulate, int splits);
 
 /* Dedispersion tile of the last gulp: DM trials and output samples per CTA
- * and channel rows staged per pipeline stage.  The first gulp of each shape
+ * and the mean number of channel rows staged per pipeline stage (a row is as
+ * long as its DM block and channel need).  The first gulp of each shape
  * times every tile that fits shared memory and keeps the fastest (environment:
  * HDB_DEDISP_TUNE=0 keeps 16 x 512, HDB_DEDISP_TILE=DBxTB forces one); all
  * tiles give the same sums.  The choice is kept across processes in a tile
